@@ -105,10 +105,21 @@ struct alignas(16) WideNode {
     float hi1[3]; int n1;
 };
 
-// Four-wide SAH node (128 B): the boxes of up to four children as SoA lanes, then the children:
-// >= 0 an inner Node4 index, < 0 a leaf -1 - (first prim << 3 | count), INT_MIN an empty slot
-// (its box is empty and never hit).  Collapsed from the binary SAH tree: same boxes, same leaves.
-struct alignas(16) Node4 {
+// Four-wide SAH node (64 B, two 256-bit loads): the boxes of up to four children with 8-bit planes,
+// then the children: >= 0 an inner Node4 index, < 0 a leaf -1 - (first prim << 3 | count), INT_MIN
+// an empty slot.  Plane byte q of axis k stands for org[k] + scale[k] * v(q), where v(q) is the float
+// whose bits are 0x3f000000 | q << 16 (0.5 + q / 256 below 128, q / 128 from there on): one byte
+// permutation decodes it.  Byte i of a plane word belongs to child i.  A box's planes are rounded
+// outwards, up to the tolerance that the traversal's slab test allows for (quantise_axis).
+struct alignas(64) Node4 {
+    float org[3], scale[3];
+    uint32_t qlox, qhix, qloy, qhiy, qloz, qhiz;
+    int child[4];
+};
+
+// The same node with exact planes (128 B): the child boxes as SoA lanes (an empty slot's box is
+// inverted), then the children.  Used while the tree is small (SahTree::nodes4x).
+struct alignas(64) Node4x {
     float lox[4], hix[4], loy[4], hiy[4], loz[4], hiz[4];
     int child[4];
     int pad[4];

@@ -324,7 +324,50 @@ void wide_children(const WideNode& w, Slot out[2]) {
         if (!(out[i].mn[0] <= out[i].mx[0])) { out[i].wide = -1; out[i].count = 0; }  // empty box: no child
 }
 
-int emit4(const std::vector<WideNode>& bin, int wide, std::vector<Node4>& out) {
+// Value of plane byte q (see Node4).
+inline double plane_value(int q) { return q < 128 ? 0.5 + q / 256.0 : q / 128.0; }
+// The largest byte whose value is at most about v (v within the byte range).
+inline int plane_byte(double v) {
+    if (!(v > 0.5)) return 0;
+    return std::min(255, (int)(v < 1.0 ? (v - 0.5) * 256.0 : std::min(v, 2.0) * 128.0));
+}
+
+// One axis of a Node4: org, scale and the plane bytes of the used children.  Byte 0 stands for the
+// node's lowest plane and byte 255 for its highest, so the outermost planes (flat walls and floors
+// among them) stay exact to float rounding; planes between are rounded outwards.  `tol` (2^-22 of the
+// coordinates) absorbs the rounding of org and scale; the traversal's margin covers it.  An axis
+// with a non-finite plane gets a NaN org: its slab distances are NaN, which the slab test ignores.
+void quantise_axis(const Slot* c, const int* child, int k, float& org, float& scale, uint32_t& qlo, uint32_t& qhi) {
+    double lo = std::numeric_limits<double>::infinity(), hi = -lo;
+    for (int i = 0; i < 4; i++)
+        if (child[i] != INT_MIN) { lo = std::min(lo, (double)c[i].mn[k]); hi = std::max(hi, (double)c[i].mx[k]); }
+    qlo = qhi = 0;
+    scale = (float)((hi - lo) / (plane_value(255) - 0.5));
+    org = (float)(lo - 0.5 * (double)scale);
+    if (!std::isfinite(scale) || !std::isfinite(org)) {
+        org = std::numeric_limits<float>::quiet_NaN();
+        scale = 0.f;
+        return;
+    }
+    const double tol = std::ldexp(std::max({std::fabs(lo), std::fabs(hi), hi - lo}), -22);
+    auto plane = [&](int q) { return (double)org + (double)scale * plane_value(q); };
+    for (int i = 0; i < 4; i++) {
+        int l = 255, h = 0;  // empty slot: an inverted box
+        if (child[i] != INT_MIN) {
+            const double below = c[i].mn[k] + tol, above = c[i].mx[k] - tol;
+            l = scale > 0.f ? plane_byte((below - org) / scale) : 0;
+            while (l < 255 && plane(l + 1) <= below) l++;
+            while (l > 0 && plane(l) > below) l--;
+            h = scale > 0.f ? plane_byte((above - org) / scale) : 0;
+            while (h < 255 && plane(h) < above) h++;
+            while (h > 0 && plane(h - 1) >= above) h--;
+        }
+        qlo |= (uint32_t)l << (8 * i);
+        qhi |= (uint32_t)h << (8 * i);
+    }
+}
+
+int emit4(const std::vector<WideNode>& bin, int wide, std::vector<Node4>& out, std::vector<Node4x>& outx) {
     Slot c[4];
     int n = 0;
     wide_children(bin[wide], c);
@@ -343,20 +386,27 @@ int emit4(const std::vector<WideNode>& bin, int wide, std::vector<Node4>& out) {
     }
     const int self = (int)out.size();
     out.emplace_back();
+    if (self < (int)kExactNodes) outx.emplace_back();
     int child[4];
     for (int i = 0; i < 4; i++) {
         if (i >= n || (c[i].wide < 0 && c[i].count == 0)) { child[i] = INT_MIN; continue; }
-        child[i] = c[i].wide >= 0 ? emit4(bin, c[i].wide, out) : -1 - ((c[i].first << 3) | c[i].count);
+        child[i] = c[i].wide >= 0 ? emit4(bin, c[i].wide, out, outx) : -1 - ((c[i].first << 3) | c[i].count);
     }
     Node4& d = out[self];
-    const float inf = std::numeric_limits<float>::infinity();
-    for (int i = 0; i < 4; i++) {
-        const bool used = child[i] != INT_MIN;
-        d.lox[i] = used ? c[i].mn[0] : inf; d.hix[i] = used ? c[i].mx[0] : -inf;
-        d.loy[i] = used ? c[i].mn[1] : inf; d.hiy[i] = used ? c[i].mx[1] : -inf;
-        d.loz[i] = used ? c[i].mn[2] : inf; d.hiz[i] = used ? c[i].mx[2] : -inf;
-        d.child[i] = child[i];
-        d.pad[i] = 0;
+    uint32_t* q[3][2] = {{&d.qlox, &d.qhix}, {&d.qloy, &d.qhiy}, {&d.qloz, &d.qhiz}};
+    for (int k = 0; k < 3; k++) quantise_axis(c, child, k, d.org[k], d.scale[k], *q[k][0], *q[k][1]);
+    for (int i = 0; i < 4; i++) d.child[i] = child[i];
+    if (self < (int)kExactNodes) {
+        Node4x& x = outx[self];
+        const float inf = std::numeric_limits<float>::infinity();
+        for (int i = 0; i < 4; i++) {
+            const bool used = child[i] != INT_MIN;
+            x.lox[i] = used ? c[i].mn[0] : inf; x.hix[i] = used ? c[i].mx[0] : -inf;
+            x.loy[i] = used ? c[i].mn[1] : inf; x.hiy[i] = used ? c[i].mx[1] : -inf;
+            x.loz[i] = used ? c[i].mn[2] : inf; x.hiz[i] = used ? c[i].mx[2] : -inf;
+            x.child[i] = child[i];
+            x.pad[i] = 0;
+        }
     }
     return self;
 }
@@ -366,7 +416,9 @@ void collapse_bvh4(SahTree& t) {
     t.nodes4.clear();
     if (t.nodes.empty()) return;
     t.nodes4.reserve(t.nodes.size() / 2 + 1);
-    emit4(t.nodes, 0, t.nodes4);
+    t.nodes4x.clear();
+    emit4(t.nodes, 0, t.nodes4, t.nodes4x);
+    if (t.nodes4.size() > kExactNodes) t.nodes4x.clear();
 }
 
 void make_prims(const HostScene& s, const std::vector<int>& order, std::vector<Prim>& prims) {

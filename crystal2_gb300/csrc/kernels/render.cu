@@ -97,7 +97,7 @@ struct WaveBuffers {
     int* sh_list = nullptr;
     int* mis_list = nullptr;
     int* bucket_list = nullptr;  // kBuckets lists of P slots
-    int* counters = nullptr;  // [0],[1] path queues, [2] shadow, [3] mis, [8..20) material buckets
+    int* counters = nullptr;  // [0],[1] path queues, [2] shadow, [3] mis, [4] shadow and [5] extension rays handed out, [8..20) material buckets, [24] MIS rays handed out
     int* levels = nullptr;    // statistics: paths entering each bounce level (C2G_LEVELS)
     std::vector<void*> owned;
 };
@@ -179,6 +179,7 @@ struct PathRefs {
 // (pass-through), 9 = miss.  k_extend appends each queue slot to its bucket; one specialised
 // k_shade<bucket> per bucket then runs without material divergence.
 constexpr int kCntBucket = 8;  // counters[8 .. 8 + kBuckets): bucket sizes
+constexpr int kCntMisFetch = 24;  // MIS rays handed out (zeroed by k_accumulate)
 
 // Warp-aggregated append into per-key lists (lanes with equal keys share one atomic).
 // Must be called by all 32 lanes; key < 0 appends nothing.
@@ -223,14 +224,15 @@ __global__ void k_raygen(DevScene S, WaveArgs a, PathRefs out, float4* out_L, in
     }
 }
 
-// Minimum resident blocks per SM of the dynamic-fetch traversal kernels (a register budget:
-// 65536 / (128 x blocks) registers per thread).  The traversal waits on dependent node loads, so
-// more resident warps hide more of that latency, until spills to local memory cost more.
+// Minimum resident 256-thread blocks per SM of the persistent traversal kernels: a budget of 64
+// registers per thread.  The traversal waits on dependent node loads, so more resident warps hide more
+// of that latency, until spills to local memory cost more: 1080p many-material step 45.5 ms at four
+// blocks, 49.5 at five (48 registers, spills), 50.4 at three.
 #ifndef C2G_EXTEND_MIN_BLOCKS
-#define C2G_EXTEND_MIN_BLOCKS 1
+#define C2G_EXTEND_MIN_BLOCKS 4
 #endif
 #ifndef C2G_SHADOW_MIN_BLOCKS
-#define C2G_SHADOW_MIN_BLOCKS 1
+#define C2G_SHADOW_MIN_BLOCKS 4
 #endif
 // Minimum resident 128-thread blocks per SM of the shading kernels (their register budget).
 #ifndef C2G_SHADE_MIN_BLOCKS
@@ -274,54 +276,54 @@ __global__ void k_extend(DevScene S, const float4* __restrict__ qo, const float4
     if (COUNT) flush_counts(cnt, C2G_K_EXTEND, rays, tc);
 }
 
-// Four-wide closest-hit extension with dynamic ray fetch (see k_shadow_fetch).  A lane whose ray
-// is finished writes its hit, appends the slot to its material bucket (all lanes join the keyed
-// append of every round; idle lanes with no key) and takes the next ray.
-template <bool COUNT>
-__global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_extend_fetch(DevScene S, const float4* __restrict__ qo, const float4* __restrict__ qd,
-                                                      float4* hit, const int* qcount, int* zero_a, int* zero_b, int* zero_c,
-                                                      int* bucket_cnt, int* bucket_list, int cap, int* fetch,
-                                                      unsigned long long* cnt) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) { *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0; }  // + shadow fetch counter
-    const int n = *qcount;
+// Lane of the four-wide extension (trace_queue): a finished ray writes its hit and joins its
+// material bucket.
+template <bool COUNT, class R>
+struct ExtendLane : QueueTuning<R> {
+    const DevScene& S;
+    const float4 *qo, *qd;
+    float4* hit;
+    int *bucket_cnt, *bucket_list;
+    int cap;
     TraceCounters tc{0, 0};
     unsigned rays = 0;
-    int ray = -1;
-    bool exhausted = false;
-    RayQ r;
-    Hit h{INFINITY, 0.f, 0.f, -1};
+    R r;
+    Hit h;
     Bvh4State st;
-    while (true) {
-        const bool need = ray < 0 && !exhausted;
-        const int idx = warp_fetch(fetch, need, n);
-        if (need) {
-            if (idx >= 0) {
-                const float4 o = qo[idx], d = qd[idx];
-                r = make_rayq(f3(o), f3(d));
-                h = Hit{INFINITY, 0.f, 0.f, -1};
-                ray = idx;
-                bvh4_begin(st);
-                rays++;
-            } else {
-                exhausted = true;
-            }
-        }
-        if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        int key = -1, done_ray = -1;
-        if (ray >= 0 && bvh4_closest_round<COUNT>(S, r, INFINITY, h, st, &tc)) {
+    using Stack = float2;
+    __device__ __forceinline__ void begin(int i) {
+        const float4 o = qo[i], d = qd[i];
+        r = make_ray<R>(S, f3(o), f3(d));
+        h = Hit{INFINITY, 0.f, 0.f, -1};
+        bvh4_begin(st);
+        rays++;
+    }
+    __device__ __forceinline__ void node(Stack* stack) { bvh4_closest_node<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
+    __device__ __forceinline__ void leaf(Stack* stack) { bvh4_closest_leaf<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
+    __device__ __forceinline__ void end(int ray, bool done) {
+        int key = -1;
+        if (done) {
             hit[ray] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
             if (h.obj < 0) key = kBucketMiss;
             else {
                 const int mt = S.objs[h.obj].material;
                 key = mt < 0 ? kBucketNone : S.mats[mt].type;
             }
-            done_ray = ray;
-            ray = -1;
         }
         const int j = warp_append_keyed(bucket_cnt, key);
-        if (key >= 0) bucket_list[key * cap + j] = done_ray;
+        if (key >= 0) bucket_list[key * cap + j] = ray;
     }
-    if (COUNT) flush_counts(cnt, C2G_K_EXTEND, rays, tc);
+};
+
+template <bool COUNT, class R>
+__global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_extend_fetch(DevScene S, const float4* __restrict__ qo, const float4* __restrict__ qd,
+                                                      float4* hit, const int* qcount, int* zero_a, int* zero_b, int* zero_c,
+                                                      int* bucket_cnt, int* bucket_list, int cap, int* fetch,
+                                                      unsigned long long* cnt) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0; }  // + shadow fetch counter
+    ExtendLane<COUNT, R> L{{}, S, qo, qd, hit, bucket_cnt, bucket_list, cap};
+    trace_queue(L, fetch, *qcount);
+    if (COUNT) flush_counts(cnt, C2G_K_EXTEND, L.rays, L.tc);
 }
 
 // ---- shade ---------------------------------------------------------------------------------------
@@ -647,51 +649,70 @@ __global__ void k_shadow(DevScene S, const int* __restrict__ list, const int* co
     if (COUNT) flush_counts(cnt, C2G_K_SHADOW, rays, tc);
 }
 
-// Four-wide any-hit traversal with dynamic ray fetch: a lane whose ray is finished takes the next
-// ray from a global counter at the end of every while-while round, instead of idling until the
-// slowest ray of its warp ends (persistent threads with ray replacement).  Same per-ray traversal
-// as trace_any_bvh4, so the same rays are occluded.
-template <bool COUNT>
+// Lane of the four-wide shadow rays: an occluded ray zeroes its light's contribution.
+template <bool COUNT, class R>
+struct ShadowLane : QueueTuning<R> {
+    const DevScene& S;
+    const int* list;
+    const float4 *so, *sd;
+    float4* sc;
+    TraceCounters tc{0, 0};
+    unsigned rays = 0;
+    R r;
+    float tmax;
+    int ign;
+    bool occluded;
+    Bvh4State st;
+    using Stack = int;
+    __device__ __forceinline__ void begin(int i) {
+        const float4 o = so[i], d = sd[i];
+        r = make_ray<R>(S, f3(o), f3(d));
+        tmax = d.w;
+        ign = __float_as_int(o.w);
+        occluded = false;
+        bvh4_begin(st);
+        rays++;
+    }
+    __device__ __forceinline__ void node(Stack* stack) { bvh4_any_node<COUNT>(S, r, 0.f, tmax, stack, st, &tc); }
+    __device__ __forceinline__ void leaf(Stack* stack) {
+        if (bvh4_any_leaf<COUNT>(S, r, 0.f, tmax, ign, stack, st, &tc)) {
+            occluded = true;
+            st.ref = st.leaf = kNoRef;
+        }
+    }
+    __device__ __forceinline__ void end(int ray, bool done) {
+        if (done && occluded) sc[list[ray]] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+};
+
+template <bool COUNT, class R>
 __global__ void __launch_bounds__(256, C2G_SHADOW_MIN_BLOCKS) k_shadow_fetch(DevScene S, const int* __restrict__ list, const int* count,
                                                       const float4* __restrict__ so, const float4* __restrict__ sd,
                                                       float4* sc, int* fetch, unsigned long long* cnt) {
-    const int n = *count;
-    TraceCounters tc{0, 0};
-    unsigned rays = 0;
-    int ray = -1;
-    bool exhausted = false;
-    RayQ r;
-    float tmax = 0.f;
-    int ign = -1;
-    Bvh4AnyState st;
-    while (true) {
-        const bool need = ray < 0 && !exhausted;
-        const int idx = warp_fetch(fetch, need, n);
-        if (need) {
-            if (idx >= 0) {
-                const float4 o = so[idx], d = sd[idx];
-                r = make_rayq(f3(o), f3(d));
-                tmax = d.w;
-                ign = __float_as_int(o.w);
-                ray = idx;
-                bvh4_begin(st);
-                rays++;
-            } else {
-                exhausted = true;
-            }
-        }
-        if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        if (ray < 0) continue;
-        bool occluded;
-        if (bvh4_any_round<COUNT>(S, r, 0.f, tmax, ign, st, &tc, occluded)) {
-            if (occluded) sc[list[ray]] = make_float4(0.f, 0.f, 0.f, 0.f);
-            ray = -1;
-        }
-    }
-    if (COUNT) flush_counts(cnt, C2G_K_SHADOW, rays, tc);
+    ShadowLane<COUNT, R> L{{}, S, list, so, sd, sc};
+    trace_queue(L, fetch, *count);
+    if (COUNT) flush_counts(cnt, C2G_K_SHADOW, L.rays, L.tc);
 }
 
 // ---- mis: closest hit of the NEE BSDF sample; records the emitter it reaches ---------------------
+// Radiance the ray's hit emits towards it and the light it belongs to (-1: none).  No hit: Light::Le of
+// an area light is zero (Light.h:52).
+__device__ __forceinline__ float4 mis_emitted(const DevScene& S, float3 o, float3 d, const Hit& h) {
+    float3 Le = f3(0.f, 0.f, 0.f);
+    int light = -1;
+    if (h.obj >= 0) {
+        const ObjInfo oi = S.objs[h.obj];
+        if (oi.light >= 0) {
+            Surface s;
+            make_surface(S, o, d, h, s);
+            float3 n_actual = s.front ? s.N : -s.N;
+            Le = area_Le(S.lights[oi.light], n_actual, -d);
+            light = oi.light;
+        }
+    }
+    return make_float4(Le.x, Le.y, Le.z, __int_as_float(light));
+}
+
 template <bool COUNT>
 __global__ void k_mis(DevScene S, const int* __restrict__ list, const int* count, const float4* __restrict__ mo,
                       const float4* __restrict__ md, float4* mis_hit, unsigned long long* cnt) {
@@ -704,28 +725,51 @@ __global__ void k_mis(DevScene S, const int* __restrict__ list, const int* count
         float4 o = mo[i], d = md[i];
         Hit h = trace_closest<COUNT>(S, f3(o), f3(d), &tc);
         rays++;
-        float3 Le = f3(0.f, 0.f, 0.f);
-        int light = -1;
-        if (h.obj >= 0) {
-            const ObjInfo oi = S.objs[h.obj];
-            if (oi.light >= 0) {
-                Surface s;
-                make_surface(S, f3(o), f3(d), h, s);
-                float3 n_actual = s.front ? s.N : -s.N;
-                Le = area_Le(S.lights[oi.light], n_actual, -f3(d));
-                light = oi.light;
-            }
-        }
-        // no hit: Light::Le of an area light is zero (Light.h:52)
-        mis_hit[slot] = make_float4(Le.x, Le.y, Le.z, __int_as_float(light));
+        mis_hit[slot] = mis_emitted(S, f3(o), f3(d), h);
     }
     if (COUNT) flush_counts(cnt, C2G_K_MIS, rays, tc);
+}
+
+// The same on four-wide nodes with ray replacement.
+template <bool COUNT, class R>
+struct MisLane : QueueTuning<R> {
+    const DevScene& S;
+    const int* list;
+    const float4 *mo, *md;
+    float4* mis_hit;
+    TraceCounters tc{0, 0};
+    unsigned rays = 0;
+    R r;
+    Hit h;
+    Bvh4State st;
+    using Stack = float2;
+    __device__ __forceinline__ void begin(int i) {
+        const float4 o = mo[i], d = md[i];
+        r = make_ray<R>(S, f3(o), f3(d));
+        h = Hit{INFINITY, 0.f, 0.f, -1};
+        bvh4_begin(st);
+        rays++;
+    }
+    __device__ __forceinline__ void node(Stack* stack) { bvh4_closest_node<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
+    __device__ __forceinline__ void leaf(Stack* stack) { bvh4_closest_leaf<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
+    __device__ __forceinline__ void end(int ray, bool done) {
+        if (done) mis_hit[list[ray]] = mis_emitted(S, r.o, r.d, h);
+    }
+};
+template <bool COUNT, class R>
+__global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_mis_fetch(DevScene S, const int* __restrict__ list, const int* count,
+                                                                          const float4* __restrict__ mo, const float4* __restrict__ md,
+                                                                          float4* mis_hit, int* fetch, unsigned long long* cnt) {
+    MisLane<COUNT, R> L{{}, S, list, mo, md, mis_hit};
+    trace_queue(L, fetch, *count);
+    if (COUNT) flush_counts(cnt, C2G_K_MIS, L.rays, L.tc);
 }
 
 // ---- accumulate ------------------------------------------------------------------------------------
 __global__ void k_accumulate(WaveArgs a, PathRefs cur, PathRefs nxt, const int2* __restrict__ acc, const float4* __restrict__ sc,
                              const float4* __restrict__ mc, const float4* __restrict__ mis_hit, float4* out_L, const int* qcount,
-                             GuideView gv) {
+                             GuideView gv, int* mis_fetch) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *mis_fetch = 0;  // for the next level
     const int n = *qcount;
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -812,49 +856,72 @@ __global__ void k_trace_rays(DevScene S, int n, const float* o, const float* d, 
     }
 }
 
-// Ray queries on four-wide nodes with dynamic fetch (same results as k_trace_rays).
-__global__ void __launch_bounds__(128) k_trace_rays_fetch(DevScene S, int n, const float* o, const float* d, const float* tmin,
-                                                          const float* tmax, const int* ignore, int any_hit, int* obj,
-                                                          float* t, int* fetch) {
-    int ray = -1;
-    bool exhausted = false;
-    RayQ r;
-    float a = 0.f, b = INFINITY;
-    int ig = -1;
-    Hit h{INFINITY, 0.f, 0.f, -1};
+// Ray queries on four-wide nodes (same results as k_trace_rays).
+template <class R>
+struct ClosestQueryLane : QueueTuning<R> {
+    const DevScene& S;
+    const float *o, *d;
+    int* obj;
+    float* t;
+    R r;
+    Hit h;
     Bvh4State st;
-    Bvh4AnyState sa;
-    while (true) {
-        const bool need = ray < 0 && !exhausted;
-        const int idx = warp_fetch(fetch, need, n);
-        if (need) {
-            if (idx >= 0) {
-                r = make_rayq(f3(o[3 * idx], o[3 * idx + 1], o[3 * idx + 2]), f3(d[3 * idx], d[3 * idx + 1], d[3 * idx + 2]));
-                a = tmin ? tmin[idx] : 0.f;
-                b = tmax ? tmax[idx] : INFINITY;
-                ig = ignore ? ignore[idx] : -1;
-                h = Hit{INFINITY, 0.f, 0.f, -1};
-                ray = idx;
-                if (any_hit) bvh4_begin(sa);
-                else bvh4_begin(st);
-            } else {
-                exhausted = true;
-            }
-        }
-        if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
-        if (ray < 0) continue;
-        if (any_hit) {
-            bool occ;
-            if (bvh4_any_round<false>(S, r, a, b, ig, sa, nullptr, occ)) {
-                obj[ray] = occ ? 1 : 0;
-                ray = -1;
-            }
-        } else if (bvh4_closest_round<false>(S, r, INFINITY, h, st, nullptr)) {
-            obj[ray] = h.obj;
-            if (t) t[ray] = h.obj >= 0 ? h.t : INFINITY;
-            ray = -1;
+    using Stack = float2;
+    __device__ __forceinline__ void begin(int i) {
+        r = make_ray<R>(S, f3(o + 3 * (size_t)i), f3(d + 3 * (size_t)i));
+        h = Hit{INFINITY, 0.f, 0.f, -1};
+        bvh4_begin(st);
+    }
+    __device__ __forceinline__ void node(Stack* stack) { bvh4_closest_node<false>(S, r, INFINITY, h, stack, st, nullptr); }
+    __device__ __forceinline__ void leaf(Stack* stack) { bvh4_closest_leaf<false>(S, r, INFINITY, h, stack, st, nullptr); }
+    __device__ __forceinline__ void end(int ray, bool done) {
+        if (!done) return;
+        obj[ray] = h.obj;
+        if (t) t[ray] = h.obj >= 0 ? h.t : INFINITY;
+    }
+};
+template <class R>
+struct AnyQueryLane : QueueTuning<R> {
+    const DevScene& S;
+    const float *o, *d, *tmin, *tmax;
+    const int* ignore;
+    int* obj;
+    R r;
+    float a, b;
+    int ig;
+    bool occluded;
+    Bvh4State st;
+    using Stack = int;
+    __device__ __forceinline__ void begin(int i) {
+        r = make_ray<R>(S, f3(o + 3 * (size_t)i), f3(d + 3 * (size_t)i));
+        a = tmin ? tmin[i] : 0.f;
+        b = tmax ? tmax[i] : INFINITY;
+        ig = ignore ? ignore[i] : -1;
+        occluded = false;
+        bvh4_begin(st);
+    }
+    __device__ __forceinline__ void node(Stack* stack) { bvh4_any_node<false>(S, r, a, b, stack, st, nullptr); }
+    __device__ __forceinline__ void leaf(Stack* stack) {
+        if (bvh4_any_leaf<false>(S, r, a, b, ig, stack, st, nullptr)) {
+            occluded = true;
+            st.ref = st.leaf = kNoRef;
         }
     }
+    __device__ __forceinline__ void end(int ray, bool done) {
+        if (done) obj[ray] = occluded ? 1 : 0;
+    }
+};
+template <class R>
+__global__ void __launch_bounds__(128, 8) k_closest_rays_fetch(DevScene S, int n, const float* o, const float* d, int* obj, float* t,
+                                                               int* fetch) {
+    ClosestQueryLane<R> L{{}, S, o, d, obj, t};
+    trace_queue(L, fetch, n);
+}
+template <class R>
+__global__ void __launch_bounds__(128, 8) k_any_rays_fetch(DevScene S, int n, const float* o, const float* d, const float* tmin,
+                                                           const float* tmax, const int* ignore, int* obj, int* fetch) {
+    AnyQueryLane<R> L{{}, S, o, d, tmin, tmax, ignore, obj};
+    trace_queue(L, fetch, n);
 }
 
 __global__ void k_halton(DevScene S, HaltonParams hp, int W, int n, const int* px, const int* py, const int* sample, int ndim, float* out) {
@@ -1003,6 +1070,10 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
             S.nodes4 = upload_vec(sah->nodes4, arena, sb_->owned, err, rc);
             if (rc) return rc;
         }
+        if (!sah->nodes4x.empty()) {
+            S.nodes4x = upload_vec(sah->nodes4x, arena, sb_->owned, err, rc);
+            if (rc) return rc;
+        }
         S.sah_width = S.nodes4 ? sah_width_ : 2;
     } else {
         make_prims(s, ref->order, prims);
@@ -1067,6 +1138,7 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
         s.object_box((int)o, b);
         for (int k = 0; k < 3; k++) { box_lo_[k] = std::min(box_lo_[k], b[k]); box_hi_[k] = std::max(box_hi_[k], b[3 + k]); }
     }
+    for (int k = 0; k < 3; k++) S.extent[k] = std::max(std::fabs(box_lo_[k]), std::fabs(box_hi_[k]));
     guide_steps_ = 0;
     wave_counter_ = nullptr;  // freed with the previous scene's buffers
     guide_.release(arena);  // a new scene trains a new network
@@ -1126,9 +1198,17 @@ int GpuScene::film_download(float* rgb_sum, float* weight, float* rgb_sumsq, std
 
 namespace {
 int g_raygen = 0, g_shade = 0, g_acc = 0, g_film = 0;
-// Persistent grids of the traversal kernels for one block size (64, 128 or 256 threads).
+// Traversal kernels: one ray per thread (reference tree, binary nodes), four-wide nodes with quantised
+// or with exact planes.
+enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_KINDS = 3 };
+int trace_kind(const DevScene& S) {
+    if (S.tree != C2G_TREE_SAH || S.sah_width != 4) return TRACE_PLAIN;
+    return S.nodes4x ? TRACE_EXACT4 : TRACE_QUANT4;
+}
+// Persistent grids of the traversal kernels for one block size (64, 128 or 256 threads), per kind and
+// without / with counters.
 struct TraceGrids {
-    int ext, ext_c, sh, sh_c, shf, shf_c, exf, exf_c, mis, mis_c;
+    int ext[TRACE_KINDS][2], sh[TRACE_KINDS][2], mis[TRACE_KINDS][2];
 };
 TraceGrids g_trace[3] = {};
 int trace_block_index(int threads) { return threads <= 64 ? 0 : (threads <= 128 ? 1 : 2); }
@@ -1141,17 +1221,69 @@ void ensure_grids() {
     for (int i = 0; i < 3; i++) {
         const int tb = 64 << i;
         TraceGrids& g = g_trace[i];
-        g.ext = grid_for((const void*)k_extend<false>, tb);
-        g.ext_c = grid_for((const void*)k_extend<true>, tb);
-        g.sh = grid_for((const void*)k_shadow<false>, tb);
-        g.sh_c = grid_for((const void*)k_shadow<true>, tb);
-        g.shf = grid_for((const void*)k_shadow_fetch<false>, tb);
-        g.shf_c = grid_for((const void*)k_shadow_fetch<true>, tb);
-        g.exf = grid_for((const void*)k_extend_fetch<false>, tb);
-        g.exf_c = grid_for((const void*)k_extend_fetch<true>, tb);
-        g.mis = grid_for((const void*)k_mis<false>, tb);
-        g.mis_c = grid_for((const void*)k_mis<true>, tb);
+        for (int c = 0; c < 2; c++) {
+            g.ext[0][c] = grid_for(c ? (const void*)k_extend<true> : (const void*)k_extend<false>, tb);
+            g.ext[1][c] = grid_for(c ? (const void*)k_extend_fetch<true, Ray4> : (const void*)k_extend_fetch<false, Ray4>, tb);
+            g.ext[2][c] = grid_for(c ? (const void*)k_extend_fetch<true, RayQ> : (const void*)k_extend_fetch<false, RayQ>, tb);
+            g.sh[0][c] = grid_for(c ? (const void*)k_shadow<true> : (const void*)k_shadow<false>, tb);
+            g.sh[1][c] = grid_for(c ? (const void*)k_shadow_fetch<true, Ray4> : (const void*)k_shadow_fetch<false, Ray4>, tb);
+            g.sh[2][c] = grid_for(c ? (const void*)k_shadow_fetch<true, RayQ> : (const void*)k_shadow_fetch<false, RayQ>, tb);
+            g.mis[0][c] = grid_for(c ? (const void*)k_mis<true> : (const void*)k_mis<false>, tb);
+            g.mis[1][c] = grid_for(c ? (const void*)k_mis_fetch<true, Ray4> : (const void*)k_mis_fetch<false, Ray4>, tb);
+            g.mis[2][c] = grid_for(c ? (const void*)k_mis_fetch<true, RayQ> : (const void*)k_mis_fetch<false, RayQ>, tb);
+        }
     }
+}
+
+// The traversal kernels' launches; the variant follows from the scene.  C: the wave's counters.
+void launch_extend(const DevScene& S, int tb, const WaveBuffers& w, int q, int* za, int* zb, int* zc, bool count,
+                   unsigned long long* cnt, cudaStream_t st) {
+    const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].ext[k][count];
+    int* C = w.counters;
+#define C2G_ARGS S, w.o[q], w.d[q], w.hit, C + q, za, zb, zc, C + kCntBucket, w.bucket_list, (int)w.P
+    if (k == TRACE_PLAIN) {
+        if (count) k_extend<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+        else k_extend<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+    } else if (k == TRACE_QUANT4) {
+        if (count) k_extend_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+        else k_extend_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+    } else {
+        if (count) k_extend_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+        else k_extend_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+    }
+#undef C2G_ARGS
+}
+void launch_shadow(const DevScene& S, int tb, const WaveBuffers& w, bool count, unsigned long long* cnt, cudaStream_t st) {
+    const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].sh[k][count];
+    int* C = w.counters;
+#define C2G_ARGS S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c
+    if (k == TRACE_PLAIN) {
+        if (count) k_shadow<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+        else k_shadow<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+    } else if (k == TRACE_QUANT4) {
+        if (count) k_shadow_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+        else k_shadow_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+    } else {
+        if (count) k_shadow_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+        else k_shadow_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+    }
+#undef C2G_ARGS
+}
+void launch_mis(const DevScene& S, int tb, const WaveBuffers& w, bool count, unsigned long long* cnt, cudaStream_t st) {
+    const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].mis[k][count];
+    int* C = w.counters;
+#define C2G_ARGS S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit
+    if (k == TRACE_PLAIN) {
+        if (count) k_mis<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+        else k_mis<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
+    } else if (k == TRACE_QUANT4) {
+        if (count) k_mis_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+        else k_mis_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+    } else {
+        if (count) k_mis_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+        else k_mis_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+    }
+#undef C2G_ARGS
 }
 
 __global__ void k_advance(int* sample0, int by) { *sample0 += by; }
@@ -1264,7 +1396,6 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
     unsigned long long* cnt = sb_->counts;
     launches = 0;
     const int tb = 64 << trace_block_index(trace_block_);
-    const TraceGrids& TG = g_trace[trace_block_index(trace_block_)];
     const bool overlap = overlap_ && side_stream(err) == C2G_OK;
     // fork: the side stream waits for everything enqueued on st so far; join: st waits for the side
     auto fork = [&](int k) {
@@ -1290,24 +1421,11 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         begin(C2G_K_EXTEND, es);
         // bucket sizes and the extension fetch counter C[5] start at zero on every level
         cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), es);
-        if (S.tree == C2G_TREE_SAH && S.sah_width == 4) {
-            if (count)
-                k_extend_fetch<true><<<TG.exf_c, tb, 0, es>>>(S, buf[q].o, buf[q].d, w.hit, C + q, za, zb, zc, C + kCntBucket,
-                                                              w.bucket_list, (int)w.P, C + 5, cnt);
-            else
-                k_extend_fetch<false><<<TG.exf, tb, 0, es>>>(S, buf[q].o, buf[q].d, w.hit, C + q, za, zb, zc, C + kCntBucket,
-                                                               w.bucket_list, (int)w.P, C + 5, cnt);
-        } else if (count) {
-            k_extend<true><<<TG.ext_c, tb, 0, es>>>(S, buf[q].o, buf[q].d, w.hit, C + q, za, zb, zc, C + kCntBucket,
-                                                    w.bucket_list, (int)w.P, cnt);
-        } else {
-            k_extend<false><<<TG.ext, tb, 0, es>>>(S, buf[q].o, buf[q].d, w.hit, C + q, za, zb, zc, C + kCntBucket,
-                                                     w.bucket_list, (int)w.P, cnt);
-        }
+        launch_extend(S, tb, w, q, za, zb, zc, count, cnt, es);
         end(es);
     };
     int* const spare = C + 56;  // counter slots no kernel reads
-    static_assert(kCntBucket + kBuckets <= 56, "counter layout");
+    static_assert(kCntBucket + kBuckets <= kCntMisFetch && kCntMisFetch < 56, "counter layout");
     bool ahead_done = false;    // this level's extension was launched during the previous level
     int cur = 0;
     for (int b = 0; b < plan.levels; b++) {
@@ -1380,31 +1498,21 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         if (overlap) {
             fork(1);
             begin(C2G_K_MIS, side_);
-            if (count) k_mis<true><<<TG.mis_c, tb, 0, side_>>>(S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit, cnt);
-            else k_mis<false><<<TG.mis, tb, 0, side_>>>(S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit, cnt);
+            launch_mis(S, tb, w, count, cnt, side_);
             end(side_);
         }
         begin(C2G_K_SHADOW, st);
-        if (S.tree == C2G_TREE_SAH && S.sah_width == 4) {
-            // four-wide nodes: the dynamic-fetch kernel (fetch counter C[4], zeroed by k_extend)
-            if (count) k_shadow_fetch<true><<<TG.shf_c, tb, 0, st>>>(S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c, C + 4, cnt);
-            else k_shadow_fetch<false><<<TG.shf, tb, 0, st>>>(S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c, C + 4, cnt);
-        } else if (count) {
-            k_shadow<true><<<TG.sh_c, tb, 0, st>>>(S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c, cnt);
-        } else {
-            k_shadow<false><<<TG.sh, tb, 0, st>>>(S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c, cnt);
-        }
+        launch_shadow(S, tb, w, count, cnt, st);
         end(st);
         if (overlap) {
             join(1);
         } else {
             begin(C2G_K_MIS, st);
-            if (count) k_mis<true><<<TG.mis_c, tb, 0, st>>>(S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit, cnt);
-            else k_mis<false><<<TG.mis, tb, 0, st>>>(S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit, cnt);
+            launch_mis(S, tb, w, count, cnt, st);
             end(st);
         }
         begin(C2G_K_ACCUM, st);
-        k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, gv);
+        k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, gv, C + kCntMisFetch);
         end(st);
         if (ahead_done) {
             // the counters the look-ahead extension left alone: the queue after the next level, the
@@ -1693,11 +1801,25 @@ int GpuScene::trace_rays_dev(int n, const float* o, const float* d, const float*
     if (!sb_->film) { err = "no scene loaded"; return C2G_ERR_STATE; }
     if (n <= 0) return C2G_OK;
     const DevScene& S = sb_->S;
-    if (S.tree == C2G_TREE_SAH && S.sah_width == 4 && sb_->fetch) {
-        static int grid = 0;
-        if (!grid) grid = grid_for((const void*)k_trace_rays_fetch, 128);
+    const int kind = trace_kind(S);
+    if (kind != TRACE_PLAIN) {
+        static int grids[2][2] = {};
+        if (!grids[0][0]) {
+            grids[0][0] = grid_for((const void*)k_closest_rays_fetch<Ray4>, 128);
+            grids[0][1] = grid_for((const void*)k_any_rays_fetch<Ray4>, 128);
+            grids[1][0] = grid_for((const void*)k_closest_rays_fetch<RayQ>, 128);
+            grids[1][1] = grid_for((const void*)k_any_rays_fetch<RayQ>, 128);
+        }
+        const bool exact = kind == TRACE_EXACT4;
+        const int g = grids[exact][any_hit ? 1 : 0];
         C2G_CUDA(cudaMemsetAsync(sb_->fetch, 0, sizeof(int), st));
-        k_trace_rays_fetch<<<grid, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, any_hit, obj, t, sb_->fetch);
+        if (any_hit) {
+            if (exact) k_any_rays_fetch<RayQ><<<g, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, obj, sb_->fetch);
+            else k_any_rays_fetch<Ray4><<<g, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, obj, sb_->fetch);
+        } else {
+            if (exact) k_closest_rays_fetch<RayQ><<<g, 128, 0, st>>>(S, n, o, d, obj, t, sb_->fetch);
+            else k_closest_rays_fetch<Ray4><<<g, 128, 0, st>>>(S, n, o, d, obj, t, sb_->fetch);
+        }
     } else {
         k_trace_rays<<<(n + 127) / 128, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, any_hit, obj, t);
     }
@@ -1868,10 +1990,7 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
     S.anyhit_clip = p.accel == C2G_ACCEL_BVH ? 1 : 0;
     S.closest_box = p.accel == C2G_ACCEL_BVH ? 1 : 0;
     S.seed = p.seed;
-    const int g_raygen = grid_for((const void*)k_raygen, 256), g_ext = grid_for((const void*)k_extend<false>, 128);
-    const int g_shade = grid_for((const void*)k_shade<MAT_DIFFUSE, false>, 128), g_sh = grid_for((const void*)k_shadow<false>, 128);
-    const int g_mis = grid_for((const void*)k_mis<false>, 128), g_acc = grid_for((const void*)k_accumulate, 256);
-    const int g_film = grid_for((const void*)k_film, 256);
+    ensure_grids();
     int* C = w.counters;
     PathRefs buf[2] = {{w.o[0], w.d[0], w.beta[0], w.L[0]}, {w.o[1], w.d[1], w.beta[1], w.L[1]}};
     C2G_CUDA(cudaMemsetAsync(m2, 0, P * 16, st));
@@ -1894,16 +2013,15 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
                 C2G_CUDA(cudaStreamSynchronize(st));
                 if (qn == 0) break;
             }
-            C2G_CUDA(cudaMemsetAsync(C + kCntBucket, 0, sizeof(int) * kBuckets, st));
-            k_extend<false><<<g_ext, 128, 0, st>>>(S, buf[cur].o, buf[cur].d, w.hit, C + cur, C + nxt, C + 2, C + 3,
-                                                     C + kCntBucket, w.bucket_list, (int)w.P, nullptr);
+            C2G_CUDA(cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), st));
+            launch_extend(S, 128, w, cur, C + nxt, C + 2, C + 3, false, nullptr, st);
             ShadeOut so{buf[nxt], C + nxt, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + 2, C + 3, w.acc, w.mis_hit};
             for (int bk = 0; bk < kBuckets; bk++)
                 if (present_buckets_ & (1 << bk))
                     launch_shade(bk, g_shade, st, S, a, buf[cur], w.hit, C + kCntBucket, w.bucket_list, (int)w.P, so, GuideView{}, false);
-            k_shadow<false><<<g_sh, 128, 0, st>>>(S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c, nullptr);
-            k_mis<false><<<g_mis, 128, 0, st>>>(S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit, nullptr);
-            k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, GuideView{});
+            launch_shadow(S, 128, w, false, nullptr, st);
+            launch_mis(S, 128, w, false, nullptr, st);
+            k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, GuideView{}, C + kCntMisFetch);
             cur = nxt;
         }
         // the caller's film gets the radiance sums and weights; the sums of squares stay in scratch

@@ -49,11 +49,8 @@ __device__ __forceinline__ void tri_surface(const DevScene& S, int shape, float3
 }
 
 __device__ __forceinline__ void sphere_surface(const Quadric& q, float3 o, float3 d, float t, Surface& s) {
-    RayQ r;
-    r.o = o;
-    r.d = d;
     float3 P, dl;
-    quadric_local(q, r, P, dl);
+    quadric_local(q, o, d, P, dl);
     float3 hp = P + dl * t;
     float3 N = normalize(hp);
     s.front = dot(dl, N) < 0;
@@ -65,11 +62,8 @@ __device__ __forceinline__ void sphere_surface(const Quadric& q, float3 o, float
 }
 
 __device__ __forceinline__ void disk_surface(const Quadric& q, float3 o, float3 d, float t, Surface& s) {
-    RayQ r;
-    r.o = o;
-    r.d = d;
     float3 P, dl;
-    quadric_local(q, r, P, dl);
+    quadric_local(q, o, d, P, dl);
     float3 hit = P + dl * t;
     float3 N = m3mul(q.l2w, f3(0.f, 1.f, 0.f));
     s.front = dl.y <= 0;
@@ -131,11 +125,8 @@ __device__ __forceinline__ float2 surface_uv(const DevScene& S, float3 o, float3
                            __fadd_rn(__fadd_rn(__fmul_rn(b0, t0.y), __fmul_rn(b1, t1.y)), __fmul_rn(b2, t2.y)));
     }
     const Quadric& q = S.quads[oi.shape];
-    RayQ r;
-    r.o = o;
-    r.d = d;
     float3 P, dl;
-    quadric_local(q, r, P, dl);
+    quadric_local(q, o, d, P, dl);
     const float3 hp = P + dl * h.t;
     if (oi.type == SHAPE_SPHERE)
         return make_float2(atan2f(-hp.z, hp.x) / kPiF, acosf(hp.y / q.c[3]) / kPiF + 1.0f);
@@ -158,18 +149,17 @@ __device__ __forceinline__ float3 area_Le(const Light& L, float3 n_actual, float
 // pdf, 0 on a miss.  The ray leaves pos + N * 1e-4 along wi (SurfaceInfo::SpawnRay, no side test).
 __device__ __forceinline__ float light_pdf(const DevScene& S, const Light& L, float3 pos, float3 N, float3 wi) {
     float3 o = pos + N * kSpawnEps;
-    RayQ r = make_rayq(o, wi);
     float3 hp, Nh;
     if (L.shape_type == SHAPE_TRI) {
         const float4* v = S.tri_pos + 3 * L.shape_idx;
         float u, vv, t;
-        if (!tri_solve<0>(f3(v[0]), f3(v[1]), f3(v[2]), r, u, vv, t)) return 0.f;
+        if (!tri_solve<0>(f3(v[0]), f3(v[1]), f3(v[2]), o, wi, u, vv, t)) return 0.f;
         hp = o + wi * t;
         Nh = tri_normal(S.tri_shade[L.shape_idx], u, vv);
         Nh = dot(wi, Nh) < 0 ? Nh : -Nh;
     } else {
         const Quadric& q = S.quads[L.shape_idx];
-        float t = L.shape_type == SHAPE_SPHERE ? sphere_hit(q, r) : disk_hit(q, r, 0.f, 0.f, false);
+        float t = L.shape_type == SHAPE_SPHERE ? sphere_hit(q, o, wi) : disk_hit(q, o, wi, 0.f, 0.f, false);
         if (t < 0.f) return 0.f;
         Surface s;
         if (L.shape_type == SHAPE_SPHERE) sphere_surface(q, o, wi, t, s);

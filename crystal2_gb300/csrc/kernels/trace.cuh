@@ -31,6 +31,56 @@ __device__ __forceinline__ RayQ make_rayq(float3 o, float3 d) {
     return r;
 }
 
+// Ray of the four-wide traversal with quantised planes: iv is the reciprocal direction clamped to a
+// finite value, m the amount by which its slab distances are widened (see node4_slabs).
+constexpr float kInvMax = 0x1p100f;
+constexpr float kSlabMargin = 20.f * 0x1p-24f;
+struct Ray4 {
+    float3 o, d, iv, m;
+};
+
+__device__ __forceinline__ float inv_clamped(float d) { return fminf(fmaxf(__frcp_rn(d), -kInvMax), kInvMax); }
+
+// R: Ray4 (quantised planes) or RayQ (exact planes)
+template <class R>
+__device__ __forceinline__ R make_ray(const DevScene& S, float3 o, float3 d);
+template <>
+__device__ __forceinline__ RayQ make_ray<RayQ>(const DevScene&, float3 o, float3 d) { return make_rayq(o, d); }
+template <>
+__device__ __forceinline__ Ray4 make_ray<Ray4>(const DevScene& S, float3 o, float3 d) {
+    Ray4 r;
+    r.o = o;
+    r.d = d;
+    r.iv = f3(inv_clamped(d.x), inv_clamped(d.y), inv_clamped(d.z));
+    r.m = f3((S.extent[0] + fabsf(o.x)) * kSlabMargin * fabsf(r.iv.x), (S.extent[1] + fabsf(o.y)) * kSlabMargin * fabsf(r.iv.y),
+             (S.extent[2] + fabsf(o.z)) * kSlabMargin * fabsf(r.iv.z));
+    return r;
+}
+
+// Thresholds of trace_queue.
+template <class R> struct QueueTuning;
+template <> struct QueueTuning<Ray4> { static constexpr int kWalkers = 10, kLeaves = 8; };
+template <> struct QueueTuning<RayQ> { static constexpr int kWalkers = 0, kLeaves = 1; };
+
+// Whether the boxes above a leaf may be larger than exact.
+__device__ __forceinline__ constexpr bool loose_boxes(const RayQ&) { return false; }
+__device__ __forceinline__ constexpr bool loose_boxes(const Ray4&) { return true; }
+// The exact ray of the primitive tests.
+__device__ __forceinline__ const RayQ& exact_ray(const RayQ& r) { return r; }
+__device__ __forceinline__ RayQ exact_ray(const Ray4& r) {
+    RayQ q;
+    q.o = r.o;
+    q.d = r.d;
+    q.inv = r.iv;
+    if (fabsf(r.iv.x) == kInvMax) q.inv.x = __frcp_rn(r.d.x);
+    if (fabsf(r.iv.y) == kInvMax) q.inv.y = __frcp_rn(r.d.y);
+    if (fabsf(r.iv.z) == kInvMax) q.inv.z = __frcp_rn(r.d.z);
+    q.neg[0] = q.inv.x < 0.f;
+    q.neg[1] = q.inv.y < 0.f;
+    q.neg[2] = q.inv.z < 0.f;
+    return q;
+}
+
 // RayBoxTest(ray, inv, invD, box, tMin, tMax): updates t0/t1 like the reference.
 __device__ __forceinline__ bool box_test(const RayQ& r, const float* mn, const float* mx, float& t0, float& t1) {
 #pragma unroll
@@ -50,11 +100,11 @@ __device__ __forceinline__ bool box_test(const RayQ& r, const float* mn, const f
 // Solve for res (see file comment).  Returns false as soon as a component is rejected.
 // mode 0: Intersect acceptance (u+v <= 1 + EPS); mode 1: IntersectTest acceptance (u+v <= 1).
 template <int MODE>
-__device__ __forceinline__ bool tri_solve(float3 v0, float3 v1, float3 v2, const RayQ& r, float& rx, float& ry, float& rz) {
+__device__ __forceinline__ bool tri_solve(float3 v0, float3 v1, float3 v2, float3 o, float3 d, float& rx, float& ry, float& rz) {
     const float m00 = __fsub_rn(v1.x, v0.x), m01 = __fsub_rn(v1.y, v0.y), m02 = __fsub_rn(v1.z, v0.z);
     const float m10 = __fsub_rn(v2.x, v0.x), m11 = __fsub_rn(v2.y, v0.y), m12 = __fsub_rn(v2.z, v0.z);
-    const float m20 = -r.d.x, m21 = -r.d.y, m22 = -r.d.z;
-    const float px = __fsub_rn(r.o.x, v0.x), py = __fsub_rn(r.o.y, v0.y), pz = __fsub_rn(r.o.z, v0.z);
+    const float m20 = -d.x, m21 = -d.y, m22 = -d.z;
+    const float px = __fsub_rn(o.x, v0.x), py = __fsub_rn(o.y, v0.y), pz = __fsub_rn(o.z, v0.z);
     const float c00 = __fsub_rn(__fmul_rn(m11, m22), __fmul_rn(m21, m12));
     const float c01 = __fsub_rn(__fmul_rn(m01, m22), __fmul_rn(m21, m02));
     const float c02 = __fsub_rn(__fmul_rn(m01, m12), __fmul_rn(m11, m02));
@@ -87,21 +137,21 @@ __device__ __forceinline__ bool tri_solve(float3 v0, float3 v1, float3 v2, const
 
 // Sphere quadratic (Sphere.cpp:39-91).  Returns the hit distance of Intersect semantics,
 // or -1 on a miss.  For IntersectTest semantics use sphere_test.
-__device__ __forceinline__ void quadric_local(const Quadric& q, const RayQ& r, float3& P, float3& d) {
+__device__ __forceinline__ void quadric_local(const Quadric& q, float3 o, float3 dir, float3& P, float3& d) {
     float3 c = f3(q.c[0], q.c[1], q.c[2]);
-    float3 rel = r.o - c;
+    float3 rel = o - c;
     // _world2Local * v: column-major mat3 times vector
     P = f3(q.w2l[0] * rel.x + q.w2l[4] * rel.y + q.w2l[8] * rel.z,
            q.w2l[1] * rel.x + q.w2l[5] * rel.y + q.w2l[9] * rel.z,
            q.w2l[2] * rel.x + q.w2l[6] * rel.y + q.w2l[10] * rel.z);
-    d = f3(q.w2l[0] * r.d.x + q.w2l[4] * r.d.y + q.w2l[8] * r.d.z,
-           q.w2l[1] * r.d.x + q.w2l[5] * r.d.y + q.w2l[9] * r.d.z,
-           q.w2l[2] * r.d.x + q.w2l[6] * r.d.y + q.w2l[10] * r.d.z);
+    d = f3(q.w2l[0] * dir.x + q.w2l[4] * dir.y + q.w2l[8] * dir.z,
+           q.w2l[1] * dir.x + q.w2l[5] * dir.y + q.w2l[9] * dir.z,
+           q.w2l[2] * dir.x + q.w2l[6] * dir.y + q.w2l[10] * dir.z);
 }
 
-__device__ __forceinline__ bool sphere_roots(const Quadric& q, const RayQ& r, float& t1, float& t2) {
+__device__ __forceinline__ bool sphere_roots(const Quadric& q, float3 o, float3 dir, float& t1, float& t2) {
     float3 P, d;
-    quadric_local(q, r, P, d);
+    quadric_local(q, o, dir, P, d);
     float rad = q.c[3];
     float a = dot(d, d);
     float b = 2 * dot(d, P);
@@ -114,9 +164,9 @@ __device__ __forceinline__ bool sphere_roots(const Quadric& q, const RayQ& r, fl
     return true;
 }
 
-__device__ __forceinline__ float sphere_hit(const Quadric& q, const RayQ& r) {
+__device__ __forceinline__ float sphere_hit(const Quadric& q, float3 o, float3 dir) {
     float t1, t2;
-    if (!sphere_roots(q, r, t1, t2)) return -1.f;
+    if (!sphere_roots(q, o, dir, t1, t2)) return -1.f;
     if (t1 > t2) { float t = t1; t1 = t2; t2 = t; }
     float t = t1;
     if (isnan(t1) || t1 < 0) t = t2;
@@ -124,17 +174,17 @@ __device__ __forceinline__ float sphere_hit(const Quadric& q, const RayQ& r) {
     return t;
 }
 
-__device__ __forceinline__ bool sphere_test(const Quadric& q, const RayQ& r, float tmin, float tmax) {
+__device__ __forceinline__ bool sphere_test(const Quadric& q, float3 o, float3 dir, float tmin, float tmax) {
     if (tmin > tmax) return false;
     float t1, t2;
-    if (!sphere_roots(q, r, t1, t2)) return false;
+    if (!sphere_roots(q, o, dir, t1, t2)) return false;
     return (t1 >= tmin && t1 <= tmax) || (t2 >= tmin && t2 <= tmax);
 }
 
 // Disk (Disk.cpp:45-78)
-__device__ __forceinline__ float disk_hit(const Quadric& q, const RayQ& r, float tmin, float tmax, bool test) {
+__device__ __forceinline__ float disk_hit(const Quadric& q, float3 o, float3 dir, float tmin, float tmax, bool test) {
     float3 P, d;
-    quadric_local(q, r, P, d);
+    quadric_local(q, o, dir, P, d);
     if (d.y == 0.f) return -1.f;
     float t = -P.y / d.y;
     if (test) {
@@ -167,8 +217,26 @@ struct TraceCounters {
     unsigned nodes, prims;
 };
 
+// Without object box tests (Brute semantics) a leaf's primitives are tested when the ray meets the
+// leaf's exact box (the union of its object boxes).  The quantised boxes of the four-wide nodes
+// contain the exact ones, so they alone would let through primitives grazed by rounding only.
+template <class R>
+__device__ __forceinline__ bool leaf_box_hit(const DevScene& S, int first, int count, const R& r, float t0, float t1) {
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = 0; i < count; i++) {
+        const float4* P = reinterpret_cast<const float4*>(S.prims + first + i);
+        const float4 a = __ldg(P), b = __ldg(P + 1), c = __ldg(P + 2);
+        float lo[3], hi[3];
+        prim_box(a, b, c, prim_type(__float_as_int(a.w)), lo, hi);
+#pragma unroll
+        for (int k = 0; k < 3; k++) { mn[k] = fminf(mn[k], lo[k]); mx[k] = fmaxf(mx[k], hi[k]); }
+    }
+    return box_test(exact_ray(r), mn, mx, t0, t1);
+}
+
 // Closest-hit test of one prim (the leaf body of BVH::Intersect, BVH.cpp:73-90).
-__device__ __forceinline__ void closest_prim(const DevScene& S, int pi, const RayQ& r, float tmax, Hit& h) {
+template <class R>
+__device__ __forceinline__ void closest_prim(const DevScene& S, int pi, const R& r, float tmax, Hit& h, int first = 0, int count = 0) {
     const float4* P = reinterpret_cast<const float4*>(S.prims + pi);
     float4 a = __ldg(P), b = __ldg(P + 1), c = __ldg(P + 2);
     int ot = __float_as_int(a.w);
@@ -177,20 +245,21 @@ __device__ __forceinline__ void closest_prim(const DevScene& S, int pi, const Ra
         float mn[3], mx[3];
         prim_box(a, b, c, type, mn, mx);
         float t0 = 0.f, t1 = smin(tmax, h.t);
-        if (!box_test(r, mn, mx, t0, t1)) return;
+        if (!box_test(exact_ray(r), mn, mx, t0, t1)) return;
     }
     float dis;
     float u = 0.f, v = 0.f;
     if (type == SHAPE_TRI) {
         float rz;
-        if (!tri_solve<0>(f3(a), f3(b), f3(c), r, u, v, rz)) return;
+        if (!tri_solve<0>(f3(a), f3(b), f3(c), r.o, r.d, u, v, rz)) return;
         dis = rz;
     } else {
         const Quadric& q = S.quads[__float_as_int(b.w)];
-        dis = type == SHAPE_SPHERE ? sphere_hit(q, r) : disk_hit(q, r, 0.f, 0.f, false);
+        dis = type == SHAPE_SPHERE ? sphere_hit(q, r.o, r.d) : disk_hit(q, r.o, r.d, 0.f, 0.f, false);
         if (dis < 0.f) return;
     }
     if (dis < h.t) {
+        if (count > 0 && !S.closest_box && !leaf_box_hit(S, first, count, r, 0.f, smin(tmax, h.t))) return;
         h.t = dis;
         h.u = u;
         h.v = v;
@@ -199,7 +268,9 @@ __device__ __forceinline__ void closest_prim(const DevScene& S, int pi, const Ra
 }
 
 // Any-hit test of one prim (leaf body of BVH::IntersectTest, BVH.cpp:127-136).
-__device__ __forceinline__ bool anyhit_prim(const DevScene& S, int pi, const RayQ& r, float tmin, float tmax, int ignore) {
+template <class R>
+__device__ __forceinline__ bool anyhit_prim(const DevScene& S, int pi, const R& r, float tmin, float tmax, int ignore, int first = 0,
+                                            int count = 0) {
     const float4* P = reinterpret_cast<const float4*>(S.prims + pi);
     float4 a = __ldg(P), b = __ldg(P + 1), c = __ldg(P + 2);
     int ot = __float_as_int(a.w);
@@ -209,17 +280,18 @@ __device__ __forceinline__ bool anyhit_prim(const DevScene& S, int pi, const Ray
     if (S.anyhit_clip) {
         float mn[3], mx[3];
         prim_box(a, b, c, type, mn, mx);
-        if (!box_test(r, mn, mx, t0, t1)) return false;
+        if (!box_test(exact_ray(r), mn, mx, t0, t1)) return false;
     }
     if (type == SHAPE_TRI) {
         if (t0 > t1) return false;
         float rx, ry, rz;
-        if (!tri_solve<1>(f3(a), f3(b), f3(c), r, rx, ry, rz)) return false;
-        return rz >= t0 && rz <= t1;
+        if (!tri_solve<1>(f3(a), f3(b), f3(c), r.o, r.d, rx, ry, rz)) return false;
+        if (!(rz >= t0 && rz <= t1)) return false;
+    } else {
+        const Quadric& q = S.quads[__float_as_int(b.w)];
+        if (type == SHAPE_SPHERE ? !sphere_test(q, r.o, r.d, t0, t1) : !(disk_hit(q, r.o, r.d, t0, t1, true) >= 0.f)) return false;
     }
-    const Quadric& q = S.quads[__float_as_int(b.w)];
-    if (type == SHAPE_SPHERE) return sphere_test(q, r, t0, t1);
-    return disk_hit(q, r, t0, t1, true) >= 0.f;
+    return !(count > 0 && !S.anyhit_clip) || leaf_box_hit(S, first, count, r, tmin, tmax);
 }
 
 constexpr int kStack = 64;
@@ -430,71 +502,103 @@ __device__ __forceinline__ bool trace_any_sah(const DevScene& S, const RayQ& r, 
 }
 
 // ---- four-wide SAH traversal --------------------------------------------------------------------
-// The per-axis slab distances are computed with the exact operations of box_test (subtract, then
-// multiply, each rounded) and combined with fmaxf/fminf, which ignore NaN exactly as the
-// reference's std::max/std::min argument order does; so a child is hit here exactly when box_test
-// would accept it, and the leaves reached are those of the binary traversal.
+// Node boxes are tested conservatively: every child whose exact box the reference's RayBoxTest would
+// accept is entered, so the primitives tested include all the reference's, and the exact tests of the
+// primitives (their own boxes under BVH semantics, their leaf's box under Brute semantics) decide.
+//
+// What bounds the traversal is the latency of dependent node loads with few lanes per warp active,
+// then issue.  A node is 64 bytes read as two 256-bit loads (it was 128 bytes in seven 128-bit loads
+// with FP32 planes): half the footprint in L1 and L2, 16 instead of 28 registers in flight, and the
+// planes decode with one byte permutation each into packed FMAs.  1080p many-material step, shadow
+// rays 21.4 -> 17.4 ms, extension 12.6 -> 11.2 ms; 2M closest-hit rays of a 65k-triangle soup
+// 1.38 -> 0.93 ms, any hit 0.82 -> 0.54 ms.  15-bit planes (96 bytes) measured 18.8 / 12.3 ms.
+//
+// Slab distances: t = v(q) * (scale * iv) + (org - o) * iv, widened by m per ray.  With u = 2^-24 and E
+// the largest coordinate of the scene on the axis, |scale| <= 1.35 E and v < 2, the roundings of t
+// (product, org - o, offset, final FMA) come to at most u (7.1 E + 3 |o|) |iv|, those of the exact
+// test to 2 u (E + |o|) |iv|, and a plane may lie inside its box by 2^-21 E = 8 u E (quantise_axis):
+// together below m = 20 u (E + |o|) |iv|.  iv is finite (a zero direction component gives 2^100): the
+// slab of a parallel axis then accepts exactly when the origin lies within it, up to the margin.
 constexpr int kStack4 = 128;
 
-__device__ __forceinline__ bool slab4(const RayQ& r, float lx, float hx, float ly, float hy, float lz, float hz,
-                                      float t0, float t1, float& tent) {
-    float ax = __fmul_rn(__fsub_rn(lx, r.o.x), r.inv.x), bx = __fmul_rn(__fsub_rn(hx, r.o.x), r.inv.x);
-    float ay = __fmul_rn(__fsub_rn(ly, r.o.y), r.inv.y), by = __fmul_rn(__fsub_rn(hy, r.o.y), r.inv.y);
-    float az = __fmul_rn(__fsub_rn(lz, r.o.z), r.inv.z), bz = __fmul_rn(__fsub_rn(hz, r.o.z), r.inv.z);
-    const float nx = r.neg[0] ? bx : ax, fx = r.neg[0] ? ax : bx;
-    const float ny = r.neg[1] ? by : ay, fy = r.neg[1] ? ay : by;
-    const float nz = r.neg[2] ? bz : az, fz = r.neg[2] ? az : bz;
-    const float tn = fmaxf(fmaxf(nx, ny), fmaxf(nz, t0));
-    const float tf = fminf(fminf(fx, fy), fminf(fz, t1));
-    tent = tn;
-    return tn <= tf;
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// (a0, a1) * s + b on both halves of a register pair
+__device__ __forceinline__ void fma2(float a0, float a1, float s, float b, float& r0, float& r1) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(a0, a1)), "l"(pack2(s, s)), "l"(pack2(b, b)));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r1) : "l"(r));
+}
+// byte K of a plane word as its plane value (Node4)
+template <int K>
+__device__ __forceinline__ float plane_byte(uint32_t w) {
+    return __uint_as_float(__byte_perm(w, 0x3f000000u, 0x7044u | (K << 8)));
+}
+__device__ __forceinline__ void slab_axis(uint32_t qlo, uint32_t qhi, float org, float scale, float o, float iv, float m,
+                                          float tn[4], float tf[4]) {
+    const float dx = org - o, a = scale * iv;
+    const float bn = __fmaf_rn(dx, iv, -m), bf = __fmaf_rn(dx, iv, m);
+    const uint32_t wn = iv < 0.f ? qhi : qlo, wf = iv < 0.f ? qlo : qhi;
+    fma2(plane_byte<0>(wn), plane_byte<1>(wn), a, bn, tn[0], tn[1]);
+    fma2(plane_byte<2>(wn), plane_byte<3>(wn), a, bn, tn[2], tn[3]);
+    fma2(plane_byte<0>(wf), plane_byte<1>(wf), a, bf, tf[0], tf[1]);
+    fma2(plane_byte<2>(wf), plane_byte<3>(wf), a, bf, tf[2], tf[3]);
+}
+// 32 bytes (32-byte aligned) of read-only data in one load
+__device__ __forceinline__ void ld256(const void* p, uint32_t v[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p));
+}
+// Entry and exit distances of a node's four child boxes, and its children.
+__device__ __forceinline__ int4 node4_slabs(const DevScene& S, int ref, const Ray4& r, float t0, float t1, float tn[4], float tf[4]) {
+    const Node4* nodes = S.nodes4;
+    uint32_t u[8], v[8];
+    ld256(nodes + ref, u);
+    ld256(reinterpret_cast<const char*>(nodes + ref) + 32, v);
+    float xn[4], xf[4], yn[4], yf[4], zn[4], zf[4];
+    slab_axis(u[6], u[7], __uint_as_float(u[0]), __uint_as_float(u[3]), r.o.x, r.iv.x, r.m.x, xn, xf);
+    slab_axis(v[0], v[1], __uint_as_float(u[1]), __uint_as_float(u[4]), r.o.y, r.iv.y, r.m.y, yn, yf);
+    slab_axis(v[2], v[3], __uint_as_float(u[2]), __uint_as_float(u[5]), r.o.z, r.iv.z, r.m.z, zn, zf);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        tn[k] = fmaxf(fmaxf(xn[k], yn[k]), fmaxf(zn[k], t0));
+        tf[k] = fminf(fminf(xf[k], yf[k]), fminf(zf[k], t1));
+    }
+    return make_int4((int)v[4], (int)v[5], (int)v[6], (int)v[7]);
 }
 
-// Near/far-ordered node loads: the ray's direction signs pick, per axis, which of a Node4's lo / hi
-// plane words holds the near planes, so the slab test needs no per-child swap (six selects per
-// child fewer; 1080p many-material step 605 -> 609 Mpaths/s).  slab_nf on the ordered planes
-// computes exactly what slab4 computes on (lo, hi).  C2G_NEARFAR=0 restores the plain loads.
-#ifndef C2G_NEARFAR
-#define C2G_NEARFAR 1
-#endif
-struct Node4Planes {
-    float4 nx, fx, ny, fy, nz, fz;
-    int4 ch;
-};
-__device__ __forceinline__ Node4Planes load_node4(const Node4* nodes, int ref, const RayQ& r) {
-    const float4* N = reinterpret_cast<const float4*>(nodes + ref);
-    Node4Planes p;
-#if C2G_NEARFAR
-    p.nx = __ldg(N + r.neg[0]);
-    p.fx = __ldg(N + (r.neg[0] ^ 1));
-    p.ny = __ldg(N + 2 + r.neg[1]);
-    p.fy = __ldg(N + 2 + (r.neg[1] ^ 1));
-    p.nz = __ldg(N + 4 + r.neg[2]);
-    p.fz = __ldg(N + 4 + (r.neg[2] ^ 1));
-#else
-    p.nx = __ldg(N);
-    p.fx = __ldg(N + 1);
-    p.ny = __ldg(N + 2);
-    p.fy = __ldg(N + 3);
-    p.nz = __ldg(N + 4);
-    p.fz = __ldg(N + 5);
-#endif
-    p.ch = __ldg(reinterpret_cast<const int4*>(N + 6));
-    return p;
+// The same with exact planes: RayBoxTest's own operations (subtract, multiply, each rounded; two planes
+// per packed instruction), combined with fmaxf / fminf, which ignore NaN as the reference's std::max /
+// std::min argument order does.  The ray's direction signs pick the near and far planes.
+__device__ __forceinline__ void slab_exact(const float4& p, float o, float iv, float t[4]) {
+    unsigned long long a = pack2(p.x, p.y), b = pack2(p.z, p.w);
+    const unsigned long long no = pack2(-o, -o), i2 = pack2(iv, iv);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(no));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(b) : "l"(no));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(i2));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(b) : "l"(i2));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t[0]), "=f"(t[1]) : "l"(a));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t[2]), "=f"(t[3]) : "l"(b));
 }
-__device__ __forceinline__ bool slab_nf(const RayQ& r, float nx, float fx, float ny, float fy, float nz, float fz, float t0,
-                                        float t1, float& tent) {
-#if C2G_NEARFAR
-    const float ax = __fmul_rn(__fsub_rn(nx, r.o.x), r.inv.x), bx = __fmul_rn(__fsub_rn(fx, r.o.x), r.inv.x);
-    const float ay = __fmul_rn(__fsub_rn(ny, r.o.y), r.inv.y), by = __fmul_rn(__fsub_rn(fy, r.o.y), r.inv.y);
-    const float az = __fmul_rn(__fsub_rn(nz, r.o.z), r.inv.z), bz = __fmul_rn(__fsub_rn(fz, r.o.z), r.inv.z);
-    const float tn = fmaxf(fmaxf(ax, ay), fmaxf(az, t0));
-    const float tf = fminf(fminf(bx, by), fminf(bz, t1));
-    tent = tn;
-    return tn <= tf;
-#else
-    return slab4(r, nx, fx, ny, fy, nz, fz, t0, t1, tent);
-#endif
+__device__ __forceinline__ int4 node4_slabs(const DevScene& S, int ref, const RayQ& r, float t0, float t1, float tn[4], float tf[4]) {
+    const float4* N = reinterpret_cast<const float4*>(S.nodes4x + ref);
+    float xn[4], xf[4], yn[4], yf[4], zn[4], zf[4];
+    slab_exact(__ldg(N + r.neg[0]), r.o.x, r.inv.x, xn);
+    slab_exact(__ldg(N + (r.neg[0] ^ 1)), r.o.x, r.inv.x, xf);
+    slab_exact(__ldg(N + 2 + r.neg[1]), r.o.y, r.inv.y, yn);
+    slab_exact(__ldg(N + 2 + (r.neg[1] ^ 1)), r.o.y, r.inv.y, yf);
+    slab_exact(__ldg(N + 4 + r.neg[2]), r.o.z, r.inv.z, zn);
+    slab_exact(__ldg(N + 4 + (r.neg[2] ^ 1)), r.o.z, r.inv.z, zf);
+    const int4 ch = __ldg(reinterpret_cast<const int4*>(N + 6));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        tn[k] = fmaxf(fmaxf(xn[k], yn[k]), fmaxf(zn[k], t0));
+        tf[k] = fminf(fminf(xf[k], yf[k]), fminf(zf[k], t1));
+    }
+    return ch;
 }
 
 __device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
@@ -504,237 +608,113 @@ __device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
     }
 }
 
-template <bool COUNT>
-__device__ __forceinline__ Hit trace_closest_bvh4(const DevScene& S, const RayQ& r, float tmax, TraceCounters* cnt) {
-    Hit h{INFINITY, 0.f, 0.f, -1};
-    int stack[kStack4];
-    float stack_t[kStack4];
-    int top = 0;
-    int ref = 0, leaf = kNoRef;
-    auto pop = [&]() -> int {
-        while (top > 0) {
-            --top;
-            if (stack_t[top] <= h.t) return stack[top];
-        }
-        return kNoRef;
-    };
-    while (ref != kNoRef || leaf != kNoRef) {
-        while (ref >= 0) {
-            const Node4Planes P = load_node4(S.nodes4, ref, r);
-            const int4 ch = P.ch;
-            if (COUNT) cnt->nodes++;
-            const float lim = smin(tmax, h.t);
-            float t[4];
-            int c[4] = {ch.x, ch.y, ch.z, ch.w};
-            if (!slab_nf(r, P.nx.x, P.fx.x, P.ny.x, P.fy.x, P.nz.x, P.fz.x, 0.f, lim, t[0])) { t[0] = INFINITY; c[0] = kNoRef; }
-            if (!slab_nf(r, P.nx.y, P.fx.y, P.ny.y, P.fy.y, P.nz.y, P.fz.y, 0.f, lim, t[1])) { t[1] = INFINITY; c[1] = kNoRef; }
-            if (!slab_nf(r, P.nx.z, P.fx.z, P.ny.z, P.fy.z, P.nz.z, P.fz.z, 0.f, lim, t[2])) { t[2] = INFINITY; c[2] = kNoRef; }
-            if (!slab_nf(r, P.nx.w, P.fx.w, P.ny.w, P.fy.w, P.nz.w, P.fz.w, 0.f, lim, t[3])) { t[3] = INFINITY; c[3] = kNoRef; }
-            // nearest first: sort the four (entry, child) pairs, push the far ones far-to-near
-            cswap(t[0], c[0], t[1], c[1]);
-            cswap(t[2], c[2], t[3], c[3]);
-            cswap(t[0], c[0], t[2], c[2]);
-            cswap(t[1], c[1], t[3], c[3]);
-            cswap(t[1], c[1], t[2], c[2]);
-            if (top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); return h; }
-#pragma unroll
-            for (int k = 3; k >= 1; k--)
-                if (c[k] != kNoRef) { stack[top] = c[k]; stack_t[top] = t[k]; top++; }
-            ref = c[0] != kNoRef ? c[0] : pop();
-            if (is_leaf(ref) && leaf == kNoRef) {
-                leaf = ref;
-                ref = pop();
-            }
-            if (!__any_sync(__activemask(), leaf == kNoRef)) break;
-        }
-        while (leaf != kNoRef) {
-            int first, count;
-            leaf_range(leaf, first, count);
-            for (int i = 0; i < count; i++) {
-                if (COUNT) cnt->prims++;
-                closest_prim(S, first + i, r, tmax, h);
-            }
-            leaf = kNoRef;
-            if (is_leaf(ref)) {
-                leaf = ref;
-                ref = pop();
-            }
-        }
-    }
-    return h;
-}
-
-template <bool COUNT>
-__device__ __forceinline__ bool trace_any_bvh4(const DevScene& S, const RayQ& r, float tmin, float tmax, int ignore, TraceCounters* cnt) {
-    int stack[kStack4];
-    int top = 0;
-    int ref = 0, leaf = kNoRef;
-    while (ref != kNoRef || leaf != kNoRef) {
-        while (ref >= 0) {
-            const Node4Planes P = load_node4(S.nodes4, ref, r);
-            const int4 ch = P.ch;
-            if (COUNT) cnt->nodes++;
-            float te;
-            const bool h0 = slab_nf(r, P.nx.x, P.fx.x, P.ny.x, P.fy.x, P.nz.x, P.fz.x, tmin, tmax, te);
-            const bool h1 = slab_nf(r, P.nx.y, P.fx.y, P.ny.y, P.fy.y, P.nz.y, P.fz.y, tmin, tmax, te);
-            const bool h2 = slab_nf(r, P.nx.z, P.fx.z, P.ny.z, P.fy.z, P.nz.z, P.fz.z, tmin, tmax, te);
-            const bool h3 = slab_nf(r, P.nx.w, P.fx.w, P.ny.w, P.fy.w, P.nz.w, P.fz.w, tmin, tmax, te);
-            if (top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); return false; }
-            int next = kNoRef;
-            if (h3) next = ch.w;
-            if (h2) { if (next != kNoRef) stack[top++] = next; next = ch.z; }
-            if (h1) { if (next != kNoRef) stack[top++] = next; next = ch.y; }
-            if (h0) { if (next != kNoRef) stack[top++] = next; next = ch.x; }
-            ref = next != kNoRef ? next : (top ? stack[--top] : kNoRef);
-            if (is_leaf(ref) && leaf == kNoRef) {
-                leaf = ref;
-                ref = top ? stack[--top] : kNoRef;
-            }
-            if (!__any_sync(__activemask(), leaf == kNoRef)) break;
-        }
-        while (leaf != kNoRef) {
-            int first, count;
-            leaf_range(leaf, first, count);
-            for (int i = 0; i < count; i++) {
-                if (COUNT) cnt->prims++;
-                if (anyhit_prim(S, first + i, r, tmin, tmax, ignore)) return true;
-            }
-            leaf = kNoRef;
-            if (is_leaf(ref)) {
-                leaf = ref;
-                ref = top ? stack[--top] : kNoRef;
-            }
-        }
-    }
-    return false;
-}
-
-// ---- resumable four-wide traversal rounds (dynamic ray fetch) ----------------------------------
-// One while-while round of the traversal above: inner nodes until every active lane of the warp
-// holds a leaf, then the leaves.  The state survives between rounds, so a kernel can hand a lane a
-// new ray as soon as its previous one is done (see k_shadow_fetch / k_extend_fetch).
-struct Bvh4AnyState {       // any hit: no entry distances
-    int stack[kStack4];
+// Traversal state of one ray: the next subtree (inner node, leaf or kNoRef), a postponed leaf, and
+// the stacked subtrees.  A lane keeps walking inner nodes past its first leaf while the other lanes
+// of its warp walk too; the exact primitive tests then run with many lanes active.  The stack is an
+// array of its own (any hit: subtrees; closest hit: (subtree, entry distance) pairs), so that the
+// rest of the state stays in registers.
+struct Bvh4State {
     int top, ref, leaf;
 };
-struct Bvh4State {          // closest hit: entry distance per stacked subtree
-    int stack[kStack4];
-    float stack_t[kStack4];
-    int top, ref, leaf;
-};
+__device__ __forceinline__ int bvh4_pop(const int* stack, Bvh4State& st) { return st.top > 0 ? stack[--st.top] : kNoRef; }
+// subtrees beyond the current hit are dropped
+__device__ __forceinline__ int bvh4_pop(const float2* stack, Bvh4State& st, float t) {
+    while (st.top > 0) {
+        const float2 e = stack[--st.top];
+        if (e.y <= t) return __float_as_int(e.x);
+    }
+    return kNoRef;
+}
 
-template <class St>
-__device__ __forceinline__ void bvh4_begin(St& st) {
+__device__ __forceinline__ void bvh4_begin(Bvh4State& st) {
     st.top = 0;
     st.ref = 0;
     st.leaf = kNoRef;
 }
+__device__ __forceinline__ bool bvh4_done(const Bvh4State& st) { return st.ref == kNoRef && st.leaf == kNoRef; }
 
-// Any hit in (tmin, tmax); returns true when the ray is finished (occluded or exhausted).
-template <bool COUNT>
-__device__ __forceinline__ bool bvh4_any_round(const DevScene& S, const RayQ& r, float tmin, float tmax, int ignore,
-                                               Bvh4AnyState& st, TraceCounters* cnt, bool& occluded) {
-    occluded = false;
-    int top = st.top, ref = st.ref, leaf = st.leaf;
-    while (ref >= 0) {
-        const Node4Planes P = load_node4(S.nodes4, ref, r);
-        const int4 ch = P.ch;
-        if (COUNT) cnt->nodes++;
-        float te;
-        const bool h0 = slab_nf(r, P.nx.x, P.fx.x, P.ny.x, P.fy.x, P.nz.x, P.fz.x, tmin, tmax, te);
-        const bool h1 = slab_nf(r, P.nx.y, P.fx.y, P.ny.y, P.fy.y, P.nz.y, P.fz.y, tmin, tmax, te);
-        const bool h2 = slab_nf(r, P.nx.z, P.fx.z, P.ny.z, P.fy.z, P.nz.z, P.fz.z, tmin, tmax, te);
-        const bool h3 = slab_nf(r, P.nx.w, P.fx.w, P.ny.w, P.fy.w, P.nz.w, P.fz.w, tmin, tmax, te);
-        if (top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); top = 0; ref = kNoRef; leaf = kNoRef; break; }
-        int next = kNoRef;
-        if (h3) next = ch.w;
-        if (h2) { if (next != kNoRef) st.stack[top++] = next; next = ch.z; }
-        if (h1) { if (next != kNoRef) st.stack[top++] = next; next = ch.y; }
-        if (h0) { if (next != kNoRef) st.stack[top++] = next; next = ch.x; }
-        ref = next != kNoRef ? next : (top ? st.stack[--top] : kNoRef);
-        if (is_leaf(ref) && leaf == kNoRef) {
-            leaf = ref;
-            ref = top ? st.stack[--top] : kNoRef;
-        }
-        if (!__any_sync(__activemask(), leaf == kNoRef)) break;
+// One inner node (st.ref >= 0) of an any-hit ray on (tmin, tmax).
+template <bool COUNT, class R>
+__device__ __forceinline__ void bvh4_any_node(const DevScene& S, const R& r, float tmin, float tmax, int* stack, Bvh4State& st,
+                                              TraceCounters* cnt) {
+    if (COUNT) cnt->nodes++;
+    float tn[4], tf[4];
+    const int4 ch = node4_slabs(S, st.ref, r, tmin, tmax, tn, tf);
+    if (st.top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); st.top = 0; st.ref = kNoRef; st.leaf = kNoRef; return; }
+    int next = kNoRef;
+    if (tn[3] <= tf[3]) next = ch.w;
+    if (tn[2] <= tf[2]) { if (next != kNoRef) stack[st.top++] = next; next = ch.z; }
+    if (tn[1] <= tf[1]) { if (next != kNoRef) stack[st.top++] = next; next = ch.y; }
+    if (tn[0] <= tf[0]) { if (next != kNoRef) stack[st.top++] = next; next = ch.x; }
+    st.ref = next != kNoRef ? next : bvh4_pop(stack, st);
+    if (is_leaf(st.ref) && st.leaf == kNoRef) {
+        st.leaf = st.ref;
+        st.ref = bvh4_pop(stack, st);
     }
-    while (leaf != kNoRef && !occluded) {
-        int first, count;
-        leaf_range(leaf, first, count);
-        for (int k = 0; k < count; k++) {
-            if (COUNT) cnt->prims++;
-            if (anyhit_prim(S, first + k, r, tmin, tmax, ignore)) { occluded = true; break; }
-        }
-        leaf = kNoRef;
-        if (!occluded && is_leaf(ref)) {
-            leaf = ref;
-            ref = top ? st.stack[--top] : kNoRef;
-        }
-    }
-    st.top = top;
-    st.ref = ref;
-    st.leaf = leaf;
-    return occluded || (ref == kNoRef && leaf == kNoRef);
 }
 
-// Closest hit (h carries the running result); returns true when the ray is finished.
-template <bool COUNT>
-__device__ __forceinline__ bool bvh4_closest_round(const DevScene& S, const RayQ& r, float tmax, Hit& h, Bvh4State& st,
-                                                   TraceCounters* cnt) {
-    int top = st.top, ref = st.ref, leaf = st.leaf;
-    auto pop = [&]() -> int {
-        while (top > 0) {
-            --top;
-            if (st.stack_t[top] <= h.t) return st.stack[top];
-        }
-        return kNoRef;
-    };
-    while (ref >= 0) {
-        const Node4Planes P = load_node4(S.nodes4, ref, r);
-        const int4 ch = P.ch;
-        if (COUNT) cnt->nodes++;
-        const float lim = smin(tmax, h.t);
-        float t[4];
-        int c[4] = {ch.x, ch.y, ch.z, ch.w};
-        if (!slab_nf(r, P.nx.x, P.fx.x, P.ny.x, P.fy.x, P.nz.x, P.fz.x, 0.f, lim, t[0])) { t[0] = INFINITY; c[0] = kNoRef; }
-        if (!slab_nf(r, P.nx.y, P.fx.y, P.ny.y, P.fy.y, P.nz.y, P.fz.y, 0.f, lim, t[1])) { t[1] = INFINITY; c[1] = kNoRef; }
-        if (!slab_nf(r, P.nx.z, P.fx.z, P.ny.z, P.fy.z, P.nz.z, P.fz.z, 0.f, lim, t[2])) { t[2] = INFINITY; c[2] = kNoRef; }
-        if (!slab_nf(r, P.nx.w, P.fx.w, P.ny.w, P.fy.w, P.nz.w, P.fz.w, 0.f, lim, t[3])) { t[3] = INFINITY; c[3] = kNoRef; }
-        cswap(t[0], c[0], t[1], c[1]);
-        cswap(t[2], c[2], t[3], c[3]);
-        cswap(t[0], c[0], t[2], c[2]);
-        cswap(t[1], c[1], t[3], c[3]);
-        cswap(t[1], c[1], t[2], c[2]);
-        if (top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); top = 0; ref = kNoRef; leaf = kNoRef; break; }
+// The postponed leaf of an any-hit ray; true when the ray is occluded.
+template <bool COUNT, class R>
+__device__ __forceinline__ bool bvh4_any_leaf(const DevScene& S, const R& r, float tmin, float tmax, int ignore,
+                                              int* stack, Bvh4State& st, TraceCounters* cnt) {
+    int first, count;
+    leaf_range(st.leaf, first, count);
+    st.leaf = kNoRef;
+    for (int k = 0; k < count; k++) {
+        if (COUNT) cnt->prims++;
+        if (anyhit_prim(S, first + k, r, tmin, tmax, ignore, first, loose_boxes(r) ? count : 0)) return true;
+    }
+    if (is_leaf(st.ref)) {
+        st.leaf = st.ref;
+        st.ref = bvh4_pop(stack, st);
+    }
+    return false;
+}
+
+// One inner node of a closest-hit ray (h carries the running result): children nearest first.
+template <bool COUNT, class R>
+__device__ __forceinline__ void bvh4_closest_node(const DevScene& S, const R& r, float tmax, const Hit& h, float2* stack, Bvh4State& st,
+                                                  TraceCounters* cnt) {
+    if (COUNT) cnt->nodes++;
+    float t[4], tf[4];
+    const int4 ch = node4_slabs(S, st.ref, r, 0.f, smin(tmax, h.t), t, tf);
+    int c[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
-        for (int k = 3; k >= 1; k--)
-            if (c[k] != kNoRef) { st.stack[top] = c[k]; st.stack_t[top] = t[k]; top++; }
-        ref = c[0] != kNoRef ? c[0] : pop();
-        if (is_leaf(ref) && leaf == kNoRef) {
-            leaf = ref;
-            ref = pop();
-        }
-        if (!__any_sync(__activemask(), leaf == kNoRef)) break;
+    for (int k = 0; k < 4; k++)
+        if (!(t[k] <= tf[k])) { t[k] = INFINITY; c[k] = kNoRef; }
+    cswap(t[0], c[0], t[1], c[1]);
+    cswap(t[2], c[2], t[3], c[3]);
+    cswap(t[0], c[0], t[2], c[2]);
+    cswap(t[1], c[1], t[3], c[3]);
+    cswap(t[1], c[1], t[2], c[2]);
+    if (st.top + 3 > kStack4) { dev_flag_error(S.err, DEVERR_STACK); st.top = 0; st.ref = kNoRef; st.leaf = kNoRef; return; }
+#pragma unroll
+    for (int k = 3; k >= 1; k--)
+        if (c[k] != kNoRef) stack[st.top++] = make_float2(__int_as_float(c[k]), t[k]);
+    st.ref = c[0] != kNoRef ? c[0] : bvh4_pop(stack, st, h.t);
+    if (is_leaf(st.ref) && st.leaf == kNoRef) {
+        st.leaf = st.ref;
+        st.ref = bvh4_pop(stack, st, h.t);
     }
-    while (leaf != kNoRef) {
-        int first, count;
-        leaf_range(leaf, first, count);
-        for (int k = 0; k < count; k++) {
-            if (COUNT) cnt->prims++;
-            closest_prim(S, first + k, r, tmax, h);
-        }
-        leaf = kNoRef;
-        if (is_leaf(ref)) {
-            leaf = ref;
-            ref = pop();
-        }
-    }
-    st.top = top;
-    st.ref = ref;
-    st.leaf = leaf;
-    return ref == kNoRef && leaf == kNoRef;
 }
 
+template <bool COUNT, class R>
+__device__ __forceinline__ void bvh4_closest_leaf(const DevScene& S, const R& r, float tmax, Hit& h, float2* stack, Bvh4State& st,
+                                                  TraceCounters* cnt) {
+    int first, count;
+    leaf_range(st.leaf, first, count);
+    st.leaf = kNoRef;
+    for (int k = 0; k < count; k++) {
+        if (COUNT) cnt->prims++;
+        closest_prim(S, first + k, r, tmax, h, first, loose_boxes(r) ? count : 0);
+    }
+    if (is_leaf(st.ref)) {
+        st.leaf = st.ref;
+        st.ref = bvh4_pop(stack, st, h.t);
+    }
+}
+
+// ---- persistent warps with ray replacement -----------------------------------------------------
 // Warp-wide refill: lanes that need a ray take consecutive indices from *fetch.  Returns the index
 // for this lane (-1: none left) and must be called by all 32 lanes.
 __device__ __forceinline__ int warp_fetch(int* fetch, bool need, int n) {
@@ -750,6 +730,68 @@ __device__ __forceinline__ int warp_fetch(int* fetch, bool need, int n) {
     return idx < n ? idx : -1;
 }
 
+// Traces the n queued rays with every lane of the grid: rounds of inner nodes, then postponed leaves; a
+// lane whose ray is finished takes the next ray of the queue after the round (persistent threads with
+// ray replacement).  All 32 lanes take part in the votes, so the warp reconverges at every step.
+//
+// The node loop ends when at most Lane::kWalkers lanes still walk (they wait for the leaves and the
+// refill instead of the others for them), the leaf loop when fewer than Lane::kLeaves lanes hold a
+// leaf.  Quantised planes (scenes of some size) take 10 and 8: 1080p many-material step, extension +
+// shadow rays, 27.6 ms; 10 and 32 28.5; 10 and 1 29.4; 14 and 1 30.9; 6 and 1 30.1; 0 and 1 33.3; a
+// refill as soon as 8 lanes are idle, without rounds, 31.7 (coherent rays lose their common path).
+// Exact planes (a handful of nodes, all in L1: bound by issue) take 0 and 1: Cornell box at 64 spp,
+// extension + shadow rays, 1.64 ms against 1.90 with 10 and 32, 1.83 with 10 and 8.  An empty queue
+// ends the waiting for a refill.
+//
+// The first rays are dealt out by thread index, the others by the counter *fetch.  Fewer rays than
+// threads are spread over the warps (one ray in every 2nd, 4th, ... lane): a late bounce level's time
+// is its slowest warp's, and a warp of few rays diverges less.
+// `L` is one lane's tracer:
+//   begin(idx)                 loads ray idx and resets the traversal
+//   node(stack), leaf(stack)   one step on L.st
+//   end(idx, done)             called by all lanes of the warp: the lanes with `done` store their result
+template <class Lane>
+__device__ __forceinline__ void trace_queue(Lane& L, int* fetch, int n) {
+    typename Lane::Stack stack[kStack4];
+    const int threads = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    int spread = 0;  // log2
+    while (spread < 5 && (long long)n << (spread + 1) <= threads) spread++;
+    int ray = (tid & ((1 << spread) - 1)) == 0 && tid >> spread < n ? tid >> spread : -1;
+    L.st.top = 0;
+    L.st.ref = L.st.leaf = kNoRef;  // an idle lane has nothing to walk
+    if (ray >= 0) L.begin(ray);
+    bool more = n > threads;        // rays may be left in the queue (warp-uniform)
+    while (true) {
+        if (__ballot_sync(0xffffffffu, ray >= 0) == 0) break;
+        const int enough = more ? Lane::kWalkers : 0;
+        unsigned walk = __ballot_sync(0xffffffffu, L.st.ref >= 0);
+        while (walk) {
+            if (L.st.ref >= 0) L.node(stack);
+            walk = __ballot_sync(0xffffffffu, L.st.ref >= 0);
+            if (__popc(walk) <= enough) break;
+        }
+        unsigned leaves = __ballot_sync(0xffffffffu, L.st.leaf != kNoRef);
+        while (leaves) {
+            if (L.st.leaf != kNoRef) L.leaf(stack);
+            leaves = __ballot_sync(0xffffffffu, L.st.leaf != kNoRef);
+            if (__popc(leaves) < Lane::kLeaves) break;
+        }
+        const bool done = ray >= 0 && bvh4_done(L.st);
+        if (__any_sync(0xffffffffu, done)) {
+            L.end(ray, done);
+            if (done) ray = -1;
+        }
+        if (more) {
+            const int idx = warp_fetch(fetch, ray < 0, n - threads);
+            if (idx >= 0) {
+                ray = threads + idx;
+                L.begin(ray);
+            }
+            more = !__any_sync(0xffffffffu, ray < 0);
+        }
+    }
+}
+
 // Brute semantics (Brute.cpp:19-55): every object, no box tests.
 __device__ __forceinline__ Hit trace_closest_brute(const DevScene& S, const RayQ& r) {
     Hit h{INFINITY, 0.f, 0.f, -1};
@@ -762,17 +804,18 @@ __device__ __forceinline__ bool trace_any_brute(const DevScene& S, const RayQ& r
     return false;
 }
 
+// One ray per thread: the reference tree and the binary SAH tree (four-wide nodes: trace_queue).
 template <bool COUNT>
 __device__ __forceinline__ Hit trace_closest(const DevScene& S, float3 o, float3 d, TraceCounters* cnt) {
     RayQ r = make_rayq(o, d);
-    if (S.tree == 1) return S.sah_width == 4 ? trace_closest_bvh4<COUNT>(S, r, INFINITY, cnt) : trace_closest_sah<COUNT>(S, r, INFINITY, cnt);
+    if (S.tree == 1) return trace_closest_sah<COUNT>(S, r, INFINITY, cnt);
     return trace_closest_ref<COUNT>(S, r, INFINITY, cnt);
 }
 
 template <bool COUNT>
 __device__ __forceinline__ bool trace_any(const DevScene& S, float3 o, float3 d, float tmin, float tmax, int ignore, TraceCounters* cnt) {
     RayQ r = make_rayq(o, d);
-    if (S.tree == 1) return S.sah_width == 4 ? trace_any_bvh4<COUNT>(S, r, tmin, tmax, ignore, cnt) : trace_any_sah<COUNT>(S, r, tmin, tmax, ignore, cnt);
+    if (S.tree == 1) return trace_any_sah<COUNT>(S, r, tmin, tmax, ignore, cnt);
     return trace_any_ref<COUNT>(S, r, tmin, tmax, ignore, cnt);
 }
 
