@@ -57,7 +57,7 @@ class RenderParams(C.Structure):
 K_RAYGEN, K_EXTEND, K_SHADE, K_SHADOW, K_MIS, K_ACCUM, K_FILM, K_GUIDE, K_TRAIN = range(9)
 K_KINDS = 10
 LEVELS = 64
-KERNEL_NAMES = ["raygen", "extend", "shade", "shadow", "mis", "accumulate", "film", "guide", "train", "-"]
+KERNEL_NAMES = ["raygen", "extend", "shade", "shadow", "mis", "accumulate", "film", "guide", "train", "tail"]
 COUNT_TRAVERSAL = 1
 COUNT_TIMING = 2
 COUNT_SERIAL = 4

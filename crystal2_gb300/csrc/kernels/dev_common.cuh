@@ -197,6 +197,14 @@ __device__ __forceinline__ float2 path_sample2(const DevScene& S, int vidx, int 
                        fminf(__fmul_rn(inv, __fadd_rn((float)row, jy)), kOneMinusEps));
 }
 
+// One component of path_sample2 (part 0 or 1), or path_sample1 (part -1).
+__device__ __forceinline__ float path_sample_part(const DevScene& S, int vidx, int dim, int part, uint32_t pixel, uint32_t sample) {
+    if (part < 0) return path_sample1(S, vidx, dim, pixel, sample);
+    if (S.sampler == SAMPLER_HALTON) return halton_sample(S, vidx, dim + part, pixel, sample);
+    const float2 v = path_sample2(S, vidx, dim, pixel, sample);
+    return part ? v.y : v.x;
+}
+
 // GetVectorIndexForSample (HaltonSampler.cpp:251-270), integer arithmetic as the reference.
 __device__ __forceinline__ int halton_vector_index(const HaltonParams& hp, int px, int py, int sample) {
     long long off = 0;

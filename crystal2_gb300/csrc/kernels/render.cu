@@ -106,6 +106,7 @@ GpuScene::GpuScene() : sb_(new DeviceSceneBuffers()), wb_(new WaveBuffers()) {}
 GpuScene::~GpuScene() {
     if (side_) cudaStreamDestroy(side_);
     if (ahead_) cudaStreamDestroy(ahead_);
+    if (report_host_) cudaFreeHost(report_host_);
     for (int k = 0; k < 4; k++) {
         if (fork_ev_[k]) cudaEventDestroy(fork_ev_[k]);
         if (join_ev_[k]) cudaEventDestroy(join_ev_[k]);
@@ -125,6 +126,13 @@ int GpuScene::side_stream(std::string& err) {
         err = "cannot create the look-ahead stream";
         ahead_ = nullptr;
         return C2G_ERR_CUDA;
+    }
+    // page-locked counters the device writes to; without them every level is enqueued
+    if (cudaHostAlloc((void**)&report_host_, 256 * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&report_dev_, report_host_, 0) != cudaSuccess) {
+        cudaGetLastError();
+        if (report_host_) cudaFreeHost(report_host_);
+        report_host_ = report_dev_ = nullptr;
     }
     for (int k = 0; k < 4; k++)
         if (cudaEventCreateWithFlags(&fork_ev_[k], cudaEventDisableTiming) != cudaSuccess ||
@@ -180,6 +188,7 @@ struct PathRefs {
 // k_shade<bucket> per bucket then runs without material divergence.
 constexpr int kCntBucket = 8;  // counters[8 .. 8 + kBuckets): bucket sizes
 constexpr int kCntMisFetch = 24;  // MIS rays handed out (zeroed by k_accumulate)
+constexpr int kCntFinish = 32;    // paths handed out by k_finish (once per wave)
 
 // Warp-aggregated append into per-key lists (lanes with equal keys share one atomic).
 // Must be called by all 32 lanes; key < 0 appends nothing.
@@ -250,9 +259,12 @@ __device__ __forceinline__ void flush_counts(unsigned long long* cnt, int kind, 
 template <bool COUNT>
 __global__ void k_extend(DevScene S, const float4* __restrict__ qo, const float4* __restrict__ qd, float4* hit,
                          const int* qcount, int* zero_a, int* zero_b, int* zero_c, int* bucket_cnt, int* bucket_list,
-                         int cap, unsigned long long* cnt) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) { *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0; }  // + shadow fetch counter
+                         int cap, volatile int* report, unsigned long long* cnt) {
     const int n = *qcount;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0;  // + shadow fetch counter
+        if (report) *report = n;
+    }
     const int stride = gridDim.x * blockDim.x;
     TraceCounters tc{0, 0};
     unsigned rays = 0;
@@ -318,9 +330,12 @@ struct ExtendLane : QueueTuning<R> {
 template <bool COUNT, class R>
 __global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_extend_fetch(DevScene S, const float4* __restrict__ qo, const float4* __restrict__ qd,
                                                       float4* hit, const int* qcount, int* zero_a, int* zero_b, int* zero_c,
-                                                      int* bucket_cnt, int* bucket_list, int cap, int* fetch,
-                                                      unsigned long long* cnt) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) { *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0; }  // + shadow fetch counter
+                                                      int* bucket_cnt, int* bucket_list, int cap, volatile int* report,
+                                                      int* fetch, unsigned long long* cnt) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0;  // + shadow fetch counter
+        if (report) *report = *qcount;
+    }
     ExtendLane<COUNT, R> L{{}, S, qo, qd, hit, bucket_cnt, bucket_list, cap};
     trace_queue(L, fetch, *qcount);
     if (COUNT) flush_counts(cnt, C2G_K_EXTEND, L.rays, L.tc);
@@ -765,6 +780,368 @@ __global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_mis_fetch(DevSce
     if (COUNT) flush_counts(cnt, C2G_K_MIS, L.rays, L.tc);
 }
 
+// ---- finishing a small queue --------------------------------------------------------------------
+// A wave's late bounce levels hold few paths, and a level then costs the latency of its slowest path
+// through five kernels and the launches between them (about 110 us on the 640 x 360 many-material
+// step, whether 500 or 20 paths are left).  k_finish instead follows each path to its end: a group of
+// lanes holds one path, lane l of the group takes light l, the last two lanes the MIS ray and the
+// extension, the sampler's dimensions are evaluated one per lane, and the rays of all the warp's
+// groups are traced together.  Arithmetic and order of every sum are those of the level kernels.
+// 64 x 64 Cornell box at 1 spp: 0.36 ms in 58 launches -> 0.19 in 3; the 640 x 360 step 1.99 -> 1.44 ms.
+// Its bound is latency, then instruction fetch: four groups of one warp at four materials run one after
+// another (a version without the per-material functions was 0.15 ms, but its other contraction of
+// multiplies and adds turned paths behind mirrors and lenses).
+struct FinishRay {
+    bool any;       // shadow ray (any hit up to h.t), else closest hit
+    int ign;
+    bool occluded;
+};
+template <class R>
+__device__ __forceinline__ void trace_group_rays(const DevScene& S, bool has, float3 o, float3 d, FinishRay& q, Hit& h) {
+    float2 stack[kStack4];
+    Bvh4State st;
+    st.top = 0;
+    st.ref = has ? 0 : kNoRef;
+    st.leaf = kNoRef;
+    const R r = make_ray<R>(S, o, d);
+    const float tmax = h.t;
+    while (__any_sync(0xffffffffu, !bvh4_done(st))) {
+        while (__any_sync(0xffffffffu, st.ref >= 0))
+            if (st.ref >= 0) bvh4_closest_node<false>(S, r, INFINITY, h, stack, st, nullptr);
+        while (__any_sync(0xffffffffu, st.leaf != kNoRef)) {
+            if (st.leaf != kNoRef) {
+                int first, count;
+                leaf_range(st.leaf, first, count);
+                st.leaf = kNoRef;
+                const int loose = loose_boxes(r) ? count : 0;
+                for (int k = 0; k < count; k++) {
+                    if (!q.any) closest_prim(S, first + k, r, INFINITY, h, first, loose);
+                    else if (anyhit_prim(S, first + k, r, 0.f, tmax, q.ign, first, loose)) { q.occluded = true; break; }
+                }
+                if (q.occluded) {
+                    st.ref = kNoRef;
+                } else if (is_leaf(st.ref)) {
+                    st.leaf = st.ref;
+                    st.ref = bvh4_pop(stack, st, h.t);
+                }
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ float3 shfl3(float3 v, int src) {
+    return f3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src), __shfl_sync(0xffffffffu, v.z, src));
+}
+
+// One path of a group: its state before and after a vertex, and the rays that the vertex asks for.
+struct FinishPath {
+    float3 ro, rd, beta, L;
+    int vidx, dim, bounce, light_path;
+    uint32_t pixel, sample;
+    Hit hit;
+    bool cont, nee, mis_ray;        // the path goes on along (ro, rd); direct light is due; an MIS ray is due
+    float3 mis_o, mis_d;
+    // this lane's light: shadow ray, its contribution, and the MIS ray's multiplier
+    bool has;
+    int ign;
+    float3 o, d, sh_c, mis_c;
+};
+
+__device__ __noinline__ float finish_sample(const DevScene& S, const FinishPath& P, int dim, int part) {
+    return path_sample_part(S, P.vidx, dim, part, P.pixel, P.sample);
+}
+
+// What a vertex's direct light needs of it.
+struct NeeVertex {
+    Surface s;
+    BxDF bx;
+    Frame fr;
+    float3 wo, beta;
+    float2 uL, uB;      // the light pair and the BSDF pair
+};
+
+// Direct light of a vertex: this lane's light (sub), and the BSDF sample that all lights share.
+// One function for every material, not inlined: the BSDF switches stay in one place.
+__device__ __noinline__ void finish_nee(const DevScene& S, unsigned group, int sub, bool eligible, bool any_area, const NeeVertex& v, FinishPath& P) {
+    const int nsflags = BXDF_ALL & ~BXDF_SPECULAR;
+    bool mis_ok = false, lane_mis = false;
+    float3 f2 = f3(0.f, 0.f, 0.f), wi2 = f3(0.f, 0.f, 0.f);
+    float pdf_b2 = 0.f;
+    if (any_area) {
+        int stype = 0;
+        f2 = bsdf_sample(v.bx, v.fr, 0.f, v.uB, v.wo, wi2, pdf_b2, nsflags, stype, mis_ok);
+        if (mis_ok) f2 = f2 * fmaxf(0.f, dot(v.s.N, wi2));
+    }
+    if (eligible) {
+        const Light Lg = S.lights[sub];
+        // light-sampling half (EsimateDirect, PathTracingIntegrator.cpp:195-227)
+        float3 lpos;
+        float pdf_l;
+        float3 Li = light_sample_li(S, Lg, v.s.pos, v.s.N, v.uL, lpos, pdf_l);
+        float3 wi = normalize(lpos - v.s.pos);
+        if (pdf_l != 0.f && !is_zero(Li)) {
+            float pdf_b;
+            float3 f = bsdf_f_pdf(v.bx, v.fr, v.wo, wi, nsflags, pdf_b) * fmaxf(0.f, dot(v.s.N, wi));
+            if (!is_zero(f)) {
+                bool back = dot(lpos - v.s.pos, v.s.N) < 0;
+                float3 org = v.s.pos + (back ? -v.s.N : v.s.N) * kSpawnEps;
+                float3 c;
+                if (Lg.type == LIGHT_POINT) c = f * Li / pdf_l;
+                else c = f * Li * power_heuristic(pdf_l, pdf_b) / pdf_l;
+                P.sh_c = v.beta * c;
+                P.has = true;
+                P.ign = Lg.type == LIGHT_AREA ? Lg.obj : -1;
+                P.o = org;
+                P.d = lpos - org;
+            }
+        }
+        // BSDF-sampling half (:229-270): weight for this light of the shared sample
+        if (mis_ok && Lg.type != LIGHT_POINT) {
+            float pdf_l2 = light_pdf(S, Lg, v.s.pos, v.s.N, wi2);
+            if (pdf_l2 != 0.f) {
+                P.mis_c = v.beta * (f2 * power_heuristic(pdf_b2, pdf_l2) / pdf_b2);
+                lane_mis = true;
+            }
+        }
+    }
+    if (__any_sync(group, lane_mis)) {
+        P.mis_ray = true;
+        P.mis_o = spawn_origin(v.s, wi2);
+        P.mis_d = wi2;
+    }
+}
+
+// A vertex of material bucket MT, with k_shade's steps and arithmetic: the surface and the continuation
+// are compiled for the material as there, since the last bit of a direction matters (a few mirrors and
+// lenses further on it decides the path).  Every lane of the group holds the same path; the sampler
+// dimensions and the lights are divided over the lanes.
+template <int MT>
+__device__ __noinline__ void finish_shade(const DevScene& S, const WaveArgs& a, unsigned group, int sub, int lead, FinishPath& P) {
+    const bool direct = a.integrator == C2G_INTEGRATOR_DIRECT;
+    float3 ro = P.ro, rd = P.rd;
+    float3 beta = P.beta, L = P.L;
+    float3 wo = -rd;
+    float3 next_o = ro, next_d = rd;
+    bool cont = false;
+    int light_path = P.light_path, dim = P.dim;
+    const int bounce = P.bounce;
+    const Hit h = P.hit;
+    Surface s;
+    make_surface(S, ro, rd, h, s);
+    if ((light_path || direct) && s.light >= 0) {
+        const Light& Lg = S.lights[s.light];
+        float3 n_actual = s.front ? s.N : -s.N;
+        L = L + beta * area_Le(Lg, n_actual, -rd);
+    }
+    if (MT == kBucketNone) {
+        if (!(direct && s.light >= 0)) {
+            next_o = spawn_origin(s, rd);
+            next_d = rd;
+            cont = true;
+        }
+    } else {
+        BxDF bx = make_bxdf(S.mats[s.mat], s.front);
+        const int tex = S.mats[s.mat].tex;
+        if (tex >= 0) bx.R = tex_lookup(S, tex, surface_uv(S, ro, rd, h));
+        bx.mtype = MT;
+        bx.flags = material_flags(MT);
+        Frame fr;
+        fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
+        // eligible area lights: one unused 1D sample each
+        bool eligible = false, area = false;
+        if (sub < S.n_lights) {
+            const Light& Lg = S.lights[sub];
+            eligible = !(Lg.flux_zero != 0.f) && (direct || sub != s.light);
+            area = eligible && Lg.type != LIGHT_POINT;
+        }
+        const int n_area = __popc(__ballot_sync(group, area));
+        // sampler dimensions, one per lane: light pair, BSDF pair of the MIS ray, BSDF pair of the
+        // continuation, roulette (after the unused 1D sample of the continuation)
+        const int dim2 = dim + 4 + n_area;
+        float u = 0.f;
+        if (sub < 7) u = finish_sample(S, P, sub < 4 ? dim + (sub & 2) : dim2 + (sub == 6 ? 3 : 0), sub == 6 ? -1 : sub & 1);
+        const float2 uL = make_float2(__shfl_sync(group, u, lead), __shfl_sync(group, u, lead + 1));
+        const float2 uB = make_float2(__shfl_sync(group, u, lead + 2), __shfl_sync(group, u, lead + 3));
+        const float2 u2 = make_float2(__shfl_sync(group, u, lead + 4), __shfl_sync(group, u, lead + 5));
+        const float ur = __shfl_sync(group, u, lead + 6);
+        dim = dim2;
+        P.nee = true;
+        if ((bx.flags & BXDF_SPECULAR) == 0) {
+            const NeeVertex v{s, bx, fr, wo, beta, uL, uB};
+            finish_nee(S, group, sub, eligible, n_area > 0, v, P);
+        }
+        if (!direct) {
+            dim += 3;
+            float3 wi = f3(0.f, 0.f, 0.f);
+            float pdf = 0.f;
+            int stype = 0;
+            bool ok = false;
+            float3 f = bsdf_sample(bx, fr, 0.f, u2, wo, wi, pdf, BXDF_ALL, stype, ok);
+            if (ok && fabsf(pdf) != 0.f) {
+                bool specular = (stype & BXDF_SPECULAR) != 0;
+                float cosine = specular ? 1.0f : fmaxf(0.f, (stype & BXDF_TRANSMISSION) ? dot(-s.N, wi) : dot(s.N, wi));
+                light_path = (specular || (stype & BXDF_TRANSMISSION)) ? 1 : 0;
+                next_o = spawn_origin(s, wi);
+                next_d = wi;
+                beta = beta * (f * cosine / pdf);
+                cont = true;
+                if (bounce > 3) {
+                    float q = fmaxf(.05f, 1.f - length(beta));
+                    dim += 1;
+                    if (ur < q) cont = false;
+                    else beta = beta / (1 - q);
+                }
+            }
+        }
+    }
+    if (cont && (direct ? bounce + 1 >= 255 : bounce + 1 >= a.max_depth)) cont = false;
+    P.L = L;
+    P.cont = cont;
+    if (cont) {
+        P.ro = next_o;
+        P.rd = next_d;
+        P.beta = beta;
+        P.dim = dim;
+        P.bounce = bounce + 1;
+        P.light_path = light_path;
+    }
+}
+
+// log2g: log2 of the lanes per path (8, 16 or 32; at least two more than the lights).  hits: the
+// queue's closest hits where they are known already.
+template <class R>
+__global__ void __launch_bounds__(128, 4) k_finish(const __grid_constant__ DevScene S, const __grid_constant__ WaveArgs a, PathRefs cur, const float4* __restrict__ hits, float4* out_L,
+                                                   const int* qcount, int* fetch, int log2g) {
+    const int n = *qcount;
+    const int G = 1 << log2g, lane = lane_id(), sub = lane & (G - 1), lead = lane - sub;
+    const unsigned group = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << lead;
+    const int ext = lead + G - 1, misl = lead + G - 2;
+    const int groups = (gridDim.x * blockDim.x) >> log2g;
+    const int K = a.K;
+    int path = (blockIdx.x * blockDim.x + threadIdx.x) >> log2g;
+    bool fresh = true;          // load `path` next
+    bool active = path < n;
+    bool more = n > groups;     // paths may be left in the queue (warp-uniform)
+    FinishPath P;               // the same in every lane of the group, but for its light's part
+    int pid = 0;
+    bool ended = false;         // no continuation; the last vertex's direct light is still due
+    bool nee = false;           // direct light of the last vertex is due
+    // this lane's ray and, for a light's lane, its contribution and MIS multiplier
+    bool has = false;
+    float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f);
+    FinishRay q{false, -1, false};
+    Hit h{INFINITY, 0.f, 0.f, -1};
+    float3 sh_c = o, mis_c = o;
+    while (true) {
+        if (active && fresh) {
+            const float4 o4 = cur.o[path], d4 = cur.d[path], b4 = cur.beta[path], L4 = cur.L[path];
+            P.ro = f3(o4);
+            P.rd = f3(d4);
+            P.beta = f3(b4);
+            P.L = f3(L4);
+            pid = __float_as_int(o4.w);
+            P.vidx = __float_as_int(b4.w);
+            const int packed = __float_as_int(d4.w);
+            P.dim = packed & 0xffff;
+            P.bounce = (packed >> 16) & 0xff;
+            P.light_path = (packed >> 24) & 1;
+            const int s_local = pid / a.nslots;
+            int px, py;
+            slot_pixel(a, pid - s_local * a.nslots, px, py);
+            P.pixel = (uint32_t)(py * a.W + px);
+            P.sample = (uint32_t)(wave_sample0(a) + s_local);
+            ended = nee = false;
+            has = false;
+            h = Hit{INFINITY, 0.f, 0.f, -1};
+            q.occluded = false;
+            if (sub == G - 1) {
+                q.any = false;
+                o = P.ro;
+                d = P.rd;
+                if (hits) {
+                    const float4 h4 = hits[path];
+                    h = Hit{h4.x, h4.y, h4.z, __float_as_int(h4.w)};
+                } else {
+                    has = true;
+                }
+            }
+            fresh = false;
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        trace_group_rays<R>(S, active && has, o, d, q, h);
+        // ---- direct light of the last vertex, summed light by light as k_accumulate does
+        float4 mh = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+        if (active && has && sub == G - 2) mh = mis_emitted(S, o, d, h);
+        const int hl = __shfl_sync(0xffffffffu, __float_as_int(mh.w), misl);
+        const float3 Le = shfl3(f3(mh), misl);
+        float3 s = has && q.occluded ? f3(0.f, 0.f, 0.f) : sh_c, m = f3(0.f, 0.f, 0.f);
+        if (sub == hl) m = mis_c * Le;
+        float3 dl = f3(0.f, 0.f, 0.f);
+        const float3 sm = s + m;
+        for (int l = 0; l < K; l++) dl = dl + shfl3(sm, lead + l);
+        if (active && nee) P.L = P.L + dl;
+        P.hit.t = __shfl_sync(0xffffffffu, h.t, ext);
+        P.hit.u = __shfl_sync(0xffffffffu, h.u, ext);
+        P.hit.v = __shfl_sync(0xffffffffu, h.v, ext);
+        P.hit.obj = __shfl_sync(0xffffffffu, h.obj, ext);
+        bool finished = active && ended;
+        // ---- shade the hit
+        P.o = P.d = P.sh_c = P.mis_c = f3(0.f, 0.f, 0.f);
+        P.has = P.nee = P.mis_ray = P.cont = false;
+        const bool shade = active && !ended;
+        int key = -1;
+        if (shade) {
+            if (P.hit.obj >= 0) {
+                const int mt = S.objs[P.hit.obj].material;
+                key = mt < 0 ? kBucketNone : S.mats[mt].type;
+            } else if (S.sky[0] >= 0 && P.bounce < a.max_depth) {
+                P.L = P.L + P.beta * sky_lookup(S, P.rd);
+            }
+        }
+        switch (key) {
+#define C2G_FINISH_CASE(B) case B: finish_shade<B>(S, a, group, sub, lead, P); break;
+            C2G_FINISH_CASE(0) C2G_FINISH_CASE(1) C2G_FINISH_CASE(2) C2G_FINISH_CASE(3) C2G_FINISH_CASE(4)
+            C2G_FINISH_CASE(5) C2G_FINISH_CASE(6) C2G_FINISH_CASE(7) C2G_FINISH_CASE(8) C2G_FINISH_CASE(9)
+            C2G_FINISH_CASE(kBucketNone)
+#undef C2G_FINISH_CASE
+        }
+        __syncwarp();
+        has = P.has;
+        o = P.o;
+        d = P.d;
+        q = FinishRay{true, P.ign, false};
+        h = Hit{1.f - kEpsTri, 0.f, 0.f, -1};
+        sh_c = P.sh_c;
+        mis_c = P.mis_c;
+        nee = P.nee;
+        if (shade) {
+            if (sub >= G - 2) {
+                q.any = false;
+                h.t = INFINITY;
+                has = sub == G - 1 ? P.cont : P.mis_ray;
+                o = sub == G - 1 ? P.ro : P.mis_o;
+                d = sub == G - 1 ? P.rd : P.mis_d;
+            }
+            if (!P.cont) {
+                ended = true;
+                finished = !nee;
+            }
+        }
+        if (finished) {
+            if (sub == 0) out_L[pid] = make_float4(P.L.x, P.L.y, P.L.z, 0.f);
+            active = false;
+        }
+        if (more) {
+            const int idx = warp_fetch(fetch, !active && sub == 0, n - groups);
+            path = groups + __shfl_sync(0xffffffffu, idx, lead);
+            if (!active && path >= groups) {
+                active = fresh = true;
+            }
+            more = !__any_sync(0xffffffffu, !active);
+        }
+    }
+}
+
 // ---- accumulate ------------------------------------------------------------------------------------
 __global__ void k_accumulate(WaveArgs a, PathRefs cur, PathRefs nxt, const int2* __restrict__ acc, const float4* __restrict__ sc,
                              const float4* __restrict__ mc, const float4* __restrict__ mis_hit, float4* out_L, const int* qcount,
@@ -1197,7 +1574,13 @@ int GpuScene::film_download(float* rgb_sum, float* weight, float* rgb_sumsq, std
 }
 
 namespace {
-int g_raygen = 0, g_shade = 0, g_acc = 0, g_film = 0;
+// When k_finish takes over: a queue of at most kFinishPaths paths (its groups hold about that many at
+// once), in a scene of at most kFinishMaterials materials (its warps would wait on instruction fetch: the
+// material box, eight materials, 201 x 149 at 9 spp takes 1.93 ms when k_finish takes its last 12092
+// paths and 1.35 ms without).  Measured limits: 640 x 360 many-material step 1.99 ms without, 1.50 at
+// 4096 paths, 1.44 at 8192, 1.43 at 16384; the 1080p step 44.07, 44.03, 44.08, 44.97.
+constexpr int kFinishPaths = 8192, kFinishMaterials = 5;
+int g_raygen = 0, g_shade = 0, g_acc = 0, g_film = 0, g_finish[2] = {0, 0};
 // Traversal kernels: one ray per thread (reference tree, binary nodes), four-wide nodes with quantised
 // or with exact planes.
 enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_KINDS = 3 };
@@ -1218,6 +1601,8 @@ void ensure_grids() {
     g_shade = grid_for((const void*)k_shade<MAT_DIFFUSE, false>, 128);
     g_acc = grid_for((const void*)k_accumulate, 256);
     g_film = grid_for((const void*)k_film, 256);
+    g_finish[0] = grid_for((const void*)k_finish<Ray4>, 128);
+    g_finish[1] = grid_for((const void*)k_finish<RayQ>, 128);
     for (int i = 0; i < 3; i++) {
         const int tb = 64 << i;
         TraceGrids& g = g_trace[i];
@@ -1236,11 +1621,11 @@ void ensure_grids() {
 }
 
 // The traversal kernels' launches; the variant follows from the scene.  C: the wave's counters.
-void launch_extend(const DevScene& S, int tb, const WaveBuffers& w, int q, int* za, int* zb, int* zc, bool count,
-                   unsigned long long* cnt, cudaStream_t st) {
+void launch_extend(const DevScene& S, int tb, const WaveBuffers& w, int q, int* za, int* zb, int* zc, int* report,
+                   bool count, unsigned long long* cnt, cudaStream_t st) {
     const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].ext[k][count];
     int* C = w.counters;
-#define C2G_ARGS S, w.o[q], w.d[q], w.hit, C + q, za, zb, zc, C + kCntBucket, w.bucket_list, (int)w.P
+#define C2G_ARGS S, w.o[q], w.d[q], w.hit, C + q, za, zb, zc, C + kCntBucket, w.bucket_list, (int)w.P, report
     if (k == TRACE_PLAIN) {
         if (count) k_extend<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_extend<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
@@ -1284,6 +1669,17 @@ void launch_mis(const DevScene& S, int tb, const WaveBuffers& w, bool count, uns
         else k_mis_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
     }
 #undef C2G_ARGS
+}
+
+// Lanes per path of k_finish: two more than the lights, as a power of two from 8 on.
+int finish_log2g(int K) { return K <= 6 ? 3 : (K <= 14 ? 4 : 5); }
+void launch_finish(const DevScene& S, const WaveArgs& a, const WaveBuffers& w, int q, bool have_hits, cudaStream_t st) {
+    const bool exact = trace_kind(S) == TRACE_EXACT4;
+    const PathRefs cur{w.o[q], w.d[q], w.beta[q], w.L[q]};
+    const float4* hits = have_hits ? w.hit : nullptr;
+    int* C = w.counters;
+    if (exact) k_finish<RayQ><<<g_finish[1], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q, C + kCntFinish, finish_log2g(a.K));
+    else k_finish<Ray4><<<g_finish[0], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q, C + kCntFinish, finish_log2g(a.K));
 }
 
 __global__ void k_advance(int* sample0, int by) { *sample0 += by; }
@@ -1417,20 +1813,51 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
     // shadow queue and its fetch counter) and *zc (the MIS queue): the live counters when it runs in
     // order, spare slots when it runs ahead beside the previous level's shadow rays (the live ones
     // are then zeroed on st after that level's accumulation).
-    auto extend = [&](int q, int* za, int* zb, int* zc, cudaStream_t es) {
+    auto extend = [&](int q, int* za, int* zb, int* zc, int* report, cudaStream_t es) {
         begin(C2G_K_EXTEND, es);
         // bucket sizes and the extension fetch counter C[5] start at zero on every level
         cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), es);
-        launch_extend(S, tb, w, q, za, zb, zc, count, cnt, es);
+        launch_extend(S, tb, w, q, za, zb, zc, report, count, cnt, es);
         end(es);
     };
     int* const spare = C + 56;  // counter slots no kernel reads
     static_assert(kCntBucket + kBuckets <= kCntMisFetch && kCntMisFetch < 56, "counter layout");
     bool ahead_done = false;    // this level's extension was launched during the previous level
     int cur = 0;
-    for (int b = 0; b < plan.levels; b++) {
+    // k_finish takes over a queue of at most kFinishPaths paths.  An eager render learns the queue's size
+    // from the look-ahead extension, which reports it to page-locked host memory; a captured wave
+    // cannot ask, and switches where a wave of its size has usually come down to that.
+    const int materials = __builtin_popcount(present_buckets_ & ~(1 << kBucketMiss));
+    const bool can_finish = !guided && !count && trace_kind(S) != TRACE_PLAIN && a.K <= 30 && plan.levels > 0 && materials <= kFinishMaterials;
+    const bool poll = overlap && report_host_ && !guided && !count;
+    if (poll)
+        for (int b = 0; b <= plan.levels; b++) report_host_[b] = -1;
+    auto finish = [&](int q, bool have_hits) {
+        begin(C2G_K_TAIL, st);
+        launch_finish(S, a, w, q, have_hits, st);
+        end(st);
+        launches++;
+    };
+    int levels = plan.levels;
+    const double paths = (double)a.W * a.H * a.wave_samples;
+    if (can_finish && paths <= kFinishPaths) {
+        finish(0, false);
+        levels = 0;
+    }
+    // captured: roulette starts after the fourth bounce; about 6.5% of a closed room's paths enter level 5,
+    // and 0.6 of them each following level
+    int captured_switch = 1 << 30;
+    if (can_finish && a.sample0_dev) {
+        double left = 0.065 * paths;
+        for (captured_switch = 5; left > kFinishPaths; captured_switch++) left *= 0.6;
+    }
+    for (int b = 0; b < levels; b++) {
+        if (b == captured_switch) {
+            finish(cur, false);
+            break;
+        }
         int nxt = cur ^ 1;
-        if (b >= a.max_depth && a.integrator == C2G_INTEGRATOR_DIRECT) {
+        if (b >= a.max_depth && a.integrator == C2G_INTEGRATOR_DIRECT && !poll) {
             // pass-through hops past the depth: stop once the queue is empty
             int qn = 0;
             C2G_CUDA(cudaMemcpyAsync(&qn, C + cur, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1441,7 +1868,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         if (count) k_level_add<<<1, 1, 0, st>>>(w.levels + std::min(b, C2G_LEVELS - 1), C + cur);
         const bool pre = ahead_done;
         if (pre) cudaStreamWaitEvent(st, join_ev_[2], 0);
-        else extend(cur, C + nxt, C + 2, C + 3, st);
+        else extend(cur, C + nxt, C + 2, C + 3, nullptr, st);
         // the guide serves the first guide_levels_ bounce levels; deeper vertices shade plainly
         const bool glevel = guided && (guide_levels_ <= 0 || b < guide_levels_);
         if (gv.sample && glevel && !pre) {
@@ -1477,10 +1904,10 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         // this level's shadow and MIS rays and accumulation (none of which reads the hits or the
         // buckets it writes).  Not for direct lighting, whose walk checks the queue on the host.
         ahead_done = false;
-        if (overlap && a.integrator != C2G_INTEGRATOR_DIRECT && b + 1 < plan.levels) {
+        if (overlap && (poll || a.integrator != C2G_INTEGRATOR_DIRECT) && b + 1 < levels) {
             cudaEventRecord(fork_ev_[2], st);
             cudaStreamWaitEvent(ahead_, fork_ev_[2], 0);
-            extend(nxt, spare, spare + 1, spare + 4, ahead_);
+            extend(nxt, spare, spare + 1, spare + 4, poll ? report_dev_ + b + 1 : nullptr, ahead_);
             launches++;
             // the next level's guide inference needs only its rays and hits: it follows on the
             // same stream (this level's shading has read its mixtures already)
@@ -1522,6 +1949,14 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         }
         launches += pre ? 3 : 4;
         cur = nxt;
+        if (poll && ahead_done) {
+            const int left = wait_report(report_host_ + b + 1, ahead_);
+            if (left == 0 || (left > 0 && left <= kFinishPaths && can_finish)) {
+                cudaStreamWaitEvent(st, join_ev_[2], 0);
+                if (left) finish(cur, true);
+                break;
+            }
+        }
     }
     begin(C2G_K_FILM, st);
     k_film<<<g_film, 256, 0, st>>>(a, w.out_L, sb_->film, sb_->film_m2);
@@ -1539,6 +1974,15 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         launches++;
     }
     return C2G_OK;
+}
+
+// The value the device writes to *p from a kernel on stream st; -1 when that stream ends without it.
+int GpuScene::wait_report(const volatile int* p, cudaStream_t st) {
+    for (;;) {
+        for (int i = 0; i < 256; i++)
+            if (*p >= 0) return *p;
+        if (cudaStreamQuery(st) != cudaErrorNotReady) return *p;
+    }
 }
 
 void GpuScene::set_sah_width(int w) {
@@ -2014,7 +2458,7 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
                 if (qn == 0) break;
             }
             C2G_CUDA(cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), st));
-            launch_extend(S, 128, w, cur, C + nxt, C + 2, C + 3, false, nullptr, st);
+            launch_extend(S, 128, w, cur, C + nxt, C + 2, C + 3, nullptr, false, nullptr, st);
             ShadeOut so{buf[nxt], C + nxt, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + 2, C + 3, w.acc, w.mis_hit};
             for (int bk = 0; bk < kBuckets; bk++)
                 if (present_buckets_ & (1 << bk))

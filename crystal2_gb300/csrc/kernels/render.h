@@ -159,6 +159,11 @@ private:
     // shading has filled the next queue, beside this level's shadow and MIS rays and accumulation.
     cudaStream_t ahead_ = nullptr;
     cudaEvent_t fork_ev_[4] = {nullptr, nullptr, nullptr, nullptr}, join_ev_[4] = {nullptr, nullptr, nullptr, nullptr};
+    // Paths entering each bounce level, written by the look-ahead extension (page-locked host memory and
+    // its device address): the host stops enqueuing levels when a queue is empty or small.
+    int* report_host_ = nullptr;
+    int* report_dev_ = nullptr;
+    static int wait_report(const volatile int* p, cudaStream_t st);
     int side_stream(std::string& err);
     float box_lo_[3] = {0, 0, 0}, box_hi_[3] = {1, 1, 1};  // scene bounds (network input range)
     c2g_stats stats_{};

@@ -89,6 +89,7 @@ typedef struct {
 #define C2G_K_FILM 6
 #define C2G_K_GUIDE 7   /* guide network inference */
 #define C2G_K_TRAIN 8   /* guide training: batch build, fused forward/backward, Adam */
+#define C2G_K_TAIL 9    /* paths of a small queue followed to their end by one kernel */
 #define C2G_K_KINDS 10  /* size of the per-kind arrays */
 
 /* Counting / timing switches of c2g_set_counting. */
