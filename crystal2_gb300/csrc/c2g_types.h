@@ -144,6 +144,14 @@ struct alignas(16) Camera {
     float W, H, zNear, pad;
 };
 
+// One dimension's base: n / base == mulhi(n, magic) >> shift for n < 2^31; off: its permutation table;
+// tail: p0 / base / (1 - 1 / base), the sum of the endless leading digits (HaltonSampler.cpp:134-149).
+struct alignas(16) HaltonDim {
+    uint32_t magic;
+    int shift, base, off;
+    float fbase, inv_base, tail, pad;
+};
+
 // Halton sampler constants (HaltonSampler.cpp:204-229).
 struct HaltonParams {
     int baseScales[2];

@@ -565,4 +565,25 @@ void halton_perm_tables(std::vector<uint16_t>& perm, std::vector<int>& offset) {
     }
 }
 
+void halton_dim_tables(const std::vector<uint16_t>& perm, const std::vector<int>& offset, HaltonDim* out) {
+    const int* primes = halton_primes();
+    for (int i = 0; i < kHaltonDims; i++) {
+        HaltonDim& h = out[i];
+        const uint32_t p = (uint32_t)primes[i];
+        // magic = ceil(2^(32 + shift) / p) with 2^shift < p <= 2^(shift + 1): the error magic * p - 2^(32 + shift)
+        // is below p <= 2^(shift + 1), so the quotient is exact for n < 2^31
+        int shift = 0;
+        while ((2u << shift) < p) shift++;
+        h.magic = (uint32_t)((((uint64_t)1 << (32 + shift)) + p - 1) / p);
+        h.shift = shift;
+        h.base = (int)p;
+        h.off = offset[i];
+        h.fbase = (float)p;
+        h.inv_base = 1.0f / h.fbase;
+        const float lead = h.inv_base * (float)perm[offset[i]], rest = 1.0f - h.inv_base;
+        h.tail = lead / rest;
+        h.pad = 0.f;
+    }
+}
+
 }  // namespace c2g

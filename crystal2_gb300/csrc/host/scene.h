@@ -68,6 +68,8 @@ HaltonParams halton_params(int width, int height);
 // 100 permutation tables from one default-seeded std::mt19937 and std::shuffle, concatenated in
 // prime order (24133 entries), plus each table's start offset.
 void halton_perm_tables(std::vector<uint16_t>& perm, std::vector<int>& offset);
+// Per-dimension constants of the sampler kernels (kHaltonDims entries).
+void halton_dim_tables(const std::vector<uint16_t>& perm, const std::vector<int>& offset, HaltonDim* out);
 // Radical-inverse primes of dims 0..99.
 const int* halton_primes();
 

@@ -31,8 +31,7 @@ struct DevScene {
     int closest_box;              // 1: per-object box prefilter on closest hits
     Camera cam;
     HaltonParams hp;
-    const uint16_t* perm;         // 100 concatenated permutation tables
-    const int* perm_off;          // table offsets
+    const float* perm;            // 100 concatenated permutation tables (digits as floats; offsets in HaltonDim)
     uint64_t seed;
     int sampler;                  // SAMPLER_HALTON / SAMPLER_DEFAULT / SAMPLER_STRATIFIED
     int spp;                      // SamplesPerPixel (the stratified sampler's strata per dimension)

@@ -375,11 +375,16 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
         const bool mis_emit = (packed >> 25) & 1;
         const float prev_pdf = L4.w;
         const int vidx = __float_as_int(b4.w);
-        int s_local = valid ? pid / a.nslots : 0;
-        int px = 0, py = 0;
-        if (valid) slot_pixel(a, pid - s_local * a.nslots, px, py);
-        const uint32_t pixel = (uint32_t)(py * a.W + px);
-        const uint32_t sample = (uint32_t)(wave_sample0(a) + s_local);
+        // pixel and sample number: only hashed draws use them (guided vertices, the Default and Stratified
+        // samplers, Halton dimensions past the tables)
+        uint32_t pixel = 0, sample = 0;
+        if (G || S.sampler != SAMPLER_HALTON || dim + 8 + S.n_lights >= kHaltonDims) {
+            const int s_local = valid ? pid / a.nslots : 0;
+            int px = 0, py = 0;
+            if (valid) slot_pixel(a, pid - s_local * a.nslots, px, py);
+            pixel = (uint32_t)(py * a.W + px);
+            sample = (uint32_t)(wave_sample0(a) + s_local);
+        }
         float3 ro = f3(o4), rd = f3(d4);
         float3 beta = f3(b4), L = f3(L4);
         Hit h{h4.x, h4.y, h4.z, __float_as_int(h4.w)};
@@ -470,8 +475,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
         float3 f2 = f3(0.f, 0.f, 0.f), wi2 = f3(0.f, 0.f, 0.f);
         float pdf_b2 = 0.f;
         if (do_nee) {
-            uL = path_sample2(S, vidx, dim, pixel, sample);
-            uB = path_sample2(S, vidx, dim + 2, pixel, sample);
+            path_sample2x2(S, vidx, dim, pixel, sample, uL, uB);
             dim += 4;
             int n_area = 0;
             for (int l = 0; l < S.n_lights; l++) {
@@ -1156,9 +1160,10 @@ __global__ void k_accumulate(WaveArgs a, PathRefs cur, PathRefs nxt, const int2*
             float4 mh = mis_hit[i];
             int hl = __float_as_int(mh.w);
             for (int l = 0; l < a.K; l++) {
-                float4 s = sc[i * a.K + l];
+                const int e = i * a.K + l;
+                float4 s = sc[e];
                 float3 m = f3(0.f, 0.f, 0.f);
-                if (l == hl) m = f3(mc[i * a.K + l]) * f3(mh);
+                if (l == hl) m = f3(mc[e]) * f3(mh);
                 direct = direct + (f3(s) + m);
             }
         }
@@ -1467,20 +1472,16 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
     std::vector<uint16_t> perm;
     std::vector<int> off;
     halton_perm_tables(perm, off);
-    S.perm = upload_vec(perm, arena, sb_->owned, err, rc);
-    if (rc) return rc;
-    S.perm_off = upload_vec(off, arena, sb_->owned, err, rc);
+    S.perm = upload_vec(std::vector<float>(perm.begin(), perm.end()), arena, sb_->owned, err, rc);
     if (rc) return rc;
     S.seed = (uint64_t)s.cfg.seed;
     S.sampler = s.cfg.sampler == "Default" ? SAMPLER_DEFAULT : s.cfg.sampler == "Stratified" ? SAMPLER_STRATIFIED : SAMPLER_HALTON;
     S.spp = std::max(1, s.cfg.spp);
     S.strata_side = 1;
     while ((S.strata_side + 1) * (S.strata_side + 1) <= S.spp) S.strata_side++;
-    const int* primes = halton_primes();
-    uint64_t magic[kHaltonDims];
-    for (int i = 0; i < kHaltonDims; i++) magic[i] = UINT64_MAX / (uint64_t)primes[i] + 1;
-    C2G_CUDA(cudaMemcpyToSymbol(c_primes, primes, sizeof(int) * kHaltonDims));
-    C2G_CUDA(cudaMemcpyToSymbol(c_divmagic, magic, sizeof(magic)));
+    HaltonDim dims[kHaltonDims];
+    halton_dim_tables(perm, off, dims);
+    C2G_CUDA(cudaMemcpyToSymbol(c_hd, dims, sizeof(dims)));
     sb_->err = (int*)arena.alloc(sizeof(int) * 4, err);
     if (!sb_->err) return C2G_ERR_OOM;
     sb_->owned.push_back(sb_->err);
