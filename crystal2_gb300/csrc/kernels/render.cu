@@ -353,6 +353,11 @@ struct ShadeOut {
     float4* mis_hit;   // per path slot: emitted radiance reaching the MIS ray, light index in w
 };
 
+// Direct-light flags of a shaded vertex (acc.y): done at all, an MIS ray follows, and which of the first
+// lights have a shadow ray (the others of those have no entry in sh_c; later lights always have one).
+constexpr uint32_t kNeeDone = 1u, kNeeMis = 2u;
+__device__ __forceinline__ uint32_t nee_bit(int l) { return l < 30 ? 4u << l : 0u; }
+
 template <int MT, bool G>
 __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S, WaveArgs a, PathRefs cur, const float4* __restrict__ hits,
                                                 const int* bucket_cnt, const int* __restrict__ bucket_list, int cap, ShadeOut out,
@@ -490,8 +495,9 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                 if (mis_ok) f2 = f2 * fmaxf(0.f, dot(s.N, wi2));
             }
         }
+        uint32_t nee_flags = do_nee ? kNeeDone : 0u, mis_mask = 0u;
         for (int l = 0; l < K; l++) {
-            bool sh_valid = false;
+            bool sh_valid = false, mis_valid = false;
             float4 sh_o4, sh_d4, sh_c4 = make_float4(0, 0, 0, 0), mis_c4 = make_float4(0, 0, 0, 0);
             if (nee_work && l < S.n_lights) {
                 const Light Lg = S.lights[l];
@@ -528,16 +534,20 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                         if (pdf_l2 != 0.f) {
                             float3 m = beta * (f2 * power_heuristic(pdf_b2, pdf_l2) / pdf_b2);
                             mis_c4 = make_float4(m.x, m.y, m.z, 0.f);
-                            any_mis = true;
+                            any_mis = mis_valid = true;
                         }
                     }
                 }
             }
             const int e = i * K + l;
-            if (do_nee) {
+            if (sh_valid) {
                 out.sh_c[e] = sh_c4;
-                out.mis_c[e] = mis_c4;
+                nee_flags |= nee_bit(l);
             }
+            // lights past the mask's bits always have an entry
+            if (mis_valid || (do_nee && l >= 32)) out.mis_c[e] = mis_c4;
+            if (mis_valid && l < 32) mis_mask |= 1u << l;
+            if (!sh_valid && do_nee && nee_bit(l) == 0u) out.sh_c[e] = sh_c4;
             // shadow rays are stored densely in append order (coalesced reads in k_shadow); the
             // list keeps the (slot, light) entry the result belongs to
             int js = warp_append(out.sh_count, sh_valid);
@@ -549,10 +559,10 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
             if (any_mis) {
                 float3 org = spawn_origin(s, wi2);
                 out.mis_list[jm] = i;
-                out.mis_o[jm] = make_float4(org.x, org.y, org.z, 0.f);
+                out.mis_o[jm] = make_float4(org.x, org.y, org.z, __uint_as_float(mis_mask));
                 out.mis_d[jm] = make_float4(wi2.x, wi2.y, wi2.z, 0.f);
+                nee_flags |= kNeeMis;
             }
-            if (do_nee) out.mis_hit[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
         }
         // ---- continuation: BSDF sample (PathTracingIntegrator.cpp:73-102); none for direct lighting
         if (do_nee && !direct) {
@@ -646,7 +656,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
             } else {
                 cur.L[i] = make_float4(L.x, L.y, L.z, 0.f);
             }
-            out.acc[i] = make_int2(cont ? j : -1, do_nee ? 1 : 0);
+            out.acc[i] = make_int2(cont ? j : -1, (int)nee_flags);
         }
     }
 }
@@ -715,13 +725,13 @@ __global__ void __launch_bounds__(256, C2G_SHADOW_MIN_BLOCKS) k_shadow_fetch(Dev
 
 // ---- mis: closest hit of the NEE BSDF sample; records the emitter it reaches ---------------------
 // Radiance the ray's hit emits towards it and the light it belongs to (-1: none).  No hit: Light::Le of
-// an area light is zero (Light.h:52).
-__device__ __forceinline__ float4 mis_emitted(const DevScene& S, float3 o, float3 d, const Hit& h) {
+// an area light is zero (Light.h:52).  mask: which of the first 32 lights weigh this sample.
+__device__ __forceinline__ float4 mis_emitted(const DevScene& S, float3 o, float3 d, const Hit& h, uint32_t mask = 0xffffffffu) {
     float3 Le = f3(0.f, 0.f, 0.f);
     int light = -1;
     if (h.obj >= 0) {
         const ObjInfo oi = S.objs[h.obj];
-        if (oi.light >= 0) {
+        if (oi.light >= 32 || (oi.light >= 0 && (mask >> oi.light & 1u))) {
             Surface s;
             make_surface(S, o, d, h, s);
             float3 n_actual = s.front ? s.N : -s.N;
@@ -744,7 +754,7 @@ __global__ void k_mis(DevScene S, const int* __restrict__ list, const int* count
         float4 o = mo[i], d = md[i];
         Hit h = trace_closest<COUNT>(S, f3(o), f3(d), &tc);
         rays++;
-        mis_hit[slot] = mis_emitted(S, f3(o), f3(d), h);
+        mis_hit[slot] = mis_emitted(S, f3(o), f3(d), h, __float_as_uint(o.w));
     }
     if (COUNT) flush_counts(cnt, C2G_K_MIS, rays, tc);
 }
@@ -772,7 +782,7 @@ struct MisLane : QueueTuning<R> {
     __device__ __forceinline__ void node(Stack* stack) { bvh4_closest_node<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
     __device__ __forceinline__ void leaf(Stack* stack) { bvh4_closest_leaf<COUNT>(S, r, INFINITY, h, stack, st, &tc); }
     __device__ __forceinline__ void end(int ray, bool done) {
-        if (done) mis_hit[list[ray]] = mis_emitted(S, r.o, r.d, h);
+        if (done) mis_hit[list[ray]] = mis_emitted(S, r.o, r.d, h, __float_as_uint(mo[ray].w));
     }
 };
 template <bool COUNT, class R>
@@ -1156,14 +1166,21 @@ __global__ void k_accumulate(WaveArgs a, PathRefs cur, PathRefs nxt, const int2*
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         int2 ac = acc[i];
         float3 direct = f3(0.f, 0.f, 0.f);
-        if (ac.y) {
-            float4 mh = mis_hit[i];
-            int hl = __float_as_int(mh.w);
+        const uint32_t fl = (uint32_t)ac.y;
+        if (fl) {
+            int hl = -1;
+            float4 mh = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (fl & kNeeMis) {
+                mh = mis_hit[i];
+                hl = __float_as_int(mh.w);
+            }
             for (int l = 0; l < a.K; l++) {
-                const int e = i * a.K + l;
-                float4 s = sc[e];
+                const uint32_t bit = nee_bit(l);
+                if (bit != 0u && !(fl & bit) && l != hl) continue;  // nothing to add
+                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (bit == 0u || (fl & bit)) s = sc[i * a.K + l];
                 float3 m = f3(0.f, 0.f, 0.f);
-                if (l == hl) m = f3(mc[e]) * f3(mh);
+                if (l == hl) m = f3(mc[i * a.K + l]) * f3(mh);
                 direct = direct + (f3(s) + m);
             }
         }
