@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 
 #include <cmath>
+#include <cstring>
 #include <random>
 #include <vector>
 
@@ -340,9 +341,18 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_guide_mlp_tc(GuideNet net, co
 // ---- records -> weighted training samples ------------------------------------------------------
 // Record (4 float4): (x, valid), (n, lum L at the vertex after its direct light), (wo, lum beta at
 // the vertex), (wi, BSDF density at wi).  Sample (4 float4): (x, w), (n, 0), (wo, 0), (wi, p_bsdf).
-__global__ void k_guide_batch(float4* rec, int rec_cap, int rec_depth, int rec_stride, const float4* __restrict__ out_L,
-                              int wave_paths, float4* batch, int* batch_count, float* stats, int batch_cap) {
-    const int stride = gridDim.x * blockDim.x;
+// One thread per record slot.  Most slots hold no record (a path records until it ends), and every warp
+// took two atomics on two addresses: now one reservation per block and iteration, and the weight sum once
+// per block (640 x 360 at 8 spp, one million slots: 69 -> 40 us).
+constexpr int kBatchThreads = 256;
+__global__ void __launch_bounds__(kBatchThreads) k_guide_batch(float4* rec, int rec_cap, int rec_depth, int rec_stride,
+                                                               const float4* __restrict__ out_L, int wave_paths, float4* batch,
+                                                               int* batch_count, float* stats, int batch_cap) {
+    __shared__ int counts[kBatchThreads / 32];
+    __shared__ int first;
+    __shared__ float sums[kBatchThreads / 32];
+    const int stride = gridDim.x * blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float ws = 0.f;
     for (int base = blockIdx.x * blockDim.x; base < rec_cap; base += stride) {
         int r = base + threadIdx.x;
         bool ok = false;
@@ -363,21 +373,36 @@ __global__ void k_guide_batch(float4* rec, int rec_cap, int rec_depth, int rec_s
                 }
             }
         }
-        unsigned m = __ballot_sync(0xffffffffu, ok);
-        int basei = 0;
-        if ((threadIdx.x & 31) == 0 && m) basei = atomicAdd(batch_count, __popc(m));
-        basei = __shfl_sync(0xffffffffu, basei, 0);
-        int j = basei + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
-        bool keep = ok && j < batch_cap;
-        if (keep) {
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) counts[warp] = __popc(m);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int total = 0;
+            for (int k = 0; k < kBatchThreads / 32; k++) {
+                const int c = counts[k];
+                counts[k] = total;
+                total += c;
+            }
+            first = total ? atomicAdd(batch_count, total) : 0;
+        }
+        __syncthreads();
+        const int j = first + counts[warp] + __popc(m & ((1u << lane) - 1u));
+        if (ok && j < batch_cap) {
             batch[4 * j] = make_float4(r0.x, r0.y, r0.z, w);
             batch[4 * j + 1] = make_float4(r1.x, r1.y, r1.z, 0.f);
             batch[4 * j + 2] = make_float4(r2.x, r2.y, r2.z, 0.f);
             batch[4 * j + 3] = r3;  // wi, BSDF density
+            ws += w;
         }
-        float ws = keep ? w : 0.f;
-        for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
-        if ((threadIdx.x & 31) == 0 && ws != 0.f) atomicAdd(stats + 2, ws);
+        __syncthreads();  // counts and first are rewritten
+    }
+    for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    if (lane == 0) sums[warp] = ws;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float total = 0.f;
+        for (int k = 0; k < kBatchThreads / 32; k++) total += sums[k];
+        if (total != 0.f) atomicAdd(stats + 2, total);
     }
 }
 
@@ -750,20 +775,47 @@ __global__ void __launch_bounds__(kTgThreads, 1) k_guide_train_tc(GuideNet net, 
     }
 }
 
+// Sum over the training kernel's per-warpgroup partial gradients, for 32 consecutive parameters per
+// block: lane = parameter (each row of a partial is read as one 128-byte run), the eight warps take
+// every eighth partial, then the first warp adds the eight sums.  The partials (20 MB) sit in L2; one
+// thread per parameter with 304 dependent-latency loads on 64 blocks took 42 us, this takes 13 (cold caches).
+constexpr int kSumThreads = 256;
+__device__ __forceinline__ float sum_partials(const float* __restrict__ part, int nparts, int p, float (*rows)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float s = 0.f;
+    if (p < kGuideParams) {
+#pragma unroll 8
+        for (int q = warp; q < nparts; q += kSumThreads / 32) s += part[(size_t)q * kGuideParams + p];
+    }
+    rows[warp][lane] = s;
+    __syncthreads();
+    float sum = 0.f;
+    if (warp == 0)
+        for (int k = 0; k < kSumThreads / 32; k++) sum += rows[k][lane];
+    return sum;
+}
+constexpr int kSumBlocks = (kGuideParams + 31) / 32;
+
 // Adam on the FP32 master weights: the gradient is the sum of the training kernel's per-warpgroup
 // partials, normalised by the batch weight sum; then the two BF16 layouts the kernels read.  The
-// padded output columns stay zero.
-__global__ void k_guide_adam(float* params, const float* __restrict__ part, int nparts, float* m, float* v,
-                             __nv_bfloat16* bfw, const float* stats, float lr, float b1, float b2, float eps,
-                             const int* step, float decay_steps) {
-    const float norm = 1.f / fmaxf(stats[1], 1e-12f);
-    // bias corrections of Adam step t = *step + 1 (the counter lives on the device so that captured
-    // graphs replay correctly; k_guide_tick advances it)
-    const float t = (float)(*step + 1);
-    const float c1 = 1.f - powf(b1, t), c2 = 1.f - powf(b2, t);
-    // learning rate lr / (1 + t / decay_steps) (decay_steps 0: constant)
-    if (decay_steps > 0.f) lr = lr / (1.f + t / decay_steps);
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < kGuideParams; p += gridDim.x * blockDim.x) {
+// padded output columns stay zero.  The last block to finish (step[1] counts them) advances the step
+// counter, keeps the step's loss and weight sum for reporting (stats[4..5]) and clears the
+// accumulators for the next step.
+__global__ void __launch_bounds__(kSumThreads) k_guide_adam(float* params, const float* __restrict__ part, int nparts, float* m, float* v,
+                                                            __nv_bfloat16* bfw, float* stats, float lr, float b1, float b2, float eps,
+                                                            int* step, float decay_steps) {
+    __shared__ float rows[kSumThreads / 32][32];
+    const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float sum = sum_partials(part, nparts, p, rows);
+    if (threadIdx.x >= 32) return;
+    if (p < kGuideParams) {
+        const float norm = 1.f / fmaxf(stats[1], 1e-12f);
+        // bias corrections of Adam step t = *step + 1 (the counter lives on the device so that captured
+        // graphs replay correctly)
+        const float t = (float)(*step + 1);
+        const float c1 = 1.f - powf(b1, t), c2 = 1.f - powf(b2, t);
+        // learning rate lr / (1 + t / decay_steps) (decay_steps 0: constant)
+        if (decay_steps > 0.f) lr = lr / (1.f + t / decay_steps);
         int l = 3;
         while (l > 0 && p < guide_w_off(l)) l--;
         int K = guide_k(l), N = guide_n(l);
@@ -771,8 +823,6 @@ __global__ void k_guide_adam(float* params, const float* __restrict__ part, int 
         bool is_bias = rel >= K * N;
         int kk = is_bias ? 0 : rel / N, nn = is_bias ? rel - K * N : rel % N;
         bool pad = (l == 3) && (nn >= kGuideOut);
-        float sum = 0.f;
-        for (int q = 0; q < nparts; q++) sum += part[(size_t)q * kGuideParams + p];
         float g = pad ? 0.f : sum * norm;
         if (!isfinite(g)) g = 0.f;  // a non-finite batch leaves the weights unchanged
         float mm = b1 * m[p] + (1.f - b1) * g;
@@ -788,25 +838,52 @@ __global__ void k_guide_adam(float* params, const float* __restrict__ part, int 
             bfw[guide_bf_off(l) + K * N + kk * N + nn] = h;   // wn: K x N
         }
     }
-}
-
-// Sum of the per-warpgroup partial gradients (the explicit-batch gradient entry point).
-__global__ void k_guide_reduce(const float* __restrict__ part, int nparts, float* grad) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < kGuideParams; p += gridDim.x * blockDim.x) {
-        float sum = 0.f;
-        for (int q = 0; q < nparts; q++) sum += part[(size_t)q * kGuideParams + p];
-        grad[p] = sum;
+    __syncwarp();  // this block has read the step counter and the statistics
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(step + 1, 1) == (int)gridDim.x - 1) {
+            step[1] = 0;
+            step[0] += 1;
+            stats[4] = stats[0];
+            stats[5] = stats[1];
+            stats[0] = 0.f;
+            stats[1] = 0.f;
+        }
     }
 }
 
-// After an Adam step: advance the step counter, keep the step's loss and weight sum for reporting
-// (stats[4..5]) and clear the accumulators for the next step.
-__global__ void k_guide_tick(int* step, float* stats) {
-    *step += 1;
-    stats[4] = stats[0];
-    stats[5] = stats[1];
-    stats[0] = 0.f;
-    stats[1] = 0.f;
+// The explicit-batch gradient: sums of the partials, then the loss statistics and the error word in
+// the words behind them (one download fetches all), and cleared accumulators.
+__global__ void __launch_bounds__(kSumThreads) k_guide_reduce(const float* __restrict__ part, int nparts, float* grad, float* stats,
+                                                              int* err) {
+    __shared__ float rows[kSumThreads / 32][32];
+    const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float sum = sum_partials(part, nparts, p, rows);
+    if (threadIdx.x < 32 && p < kGuideParams) grad[p] = sum;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        grad[kGuideParams] = stats[0];
+        grad[kGuideParams + 1] = stats[1];
+        grad[kGuideParams + 2] = __int_as_float(*err);
+        for (int k = 0; k < 8; k++) stats[k] = 0.f;
+    }
+}
+
+// Explicit samples of 14 floats (x, n, wo, wi, w, p_bsdf) -> the batch layout; sets the batch size and
+// the statistics (a weight sum of n makes the mean weight exactly 1) and clears the error word.
+__global__ void k_guide_pack(const float* __restrict__ samples, int n, float4* batch, int* batch_count, float* stats, int* err) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) {
+        const float* v = samples + (size_t)14 * j;
+        batch[4 * (size_t)j] = make_float4(v[0], v[1], v[2], v[12]);
+        batch[4 * (size_t)j + 1] = make_float4(v[3], v[4], v[5], 0.f);
+        batch[4 * (size_t)j + 2] = make_float4(v[6], v[7], v[8], 0.f);
+        batch[4 * (size_t)j + 3] = make_float4(v[9], v[10], v[11], v[13]);
+    }
+    if (j == 0) {
+        *batch_count = n;
+        *err = 0;
+        for (int k = 0; k < 8; k++) stats[k] = k == 2 ? (float)n : 0.f;
+    }
 }
 
 __global__ void k_guide_bf16_from_params(const float* params, __nv_bfloat16* bfw) {
@@ -853,7 +930,7 @@ int GuideTrainer::init(DeviceArena& arena, size_t paths, int max_depth, const fl
         prepare_launch();
         nparts_ = train_parts();
         params_ = (float*)A(kGuideParams * 4);
-        grad_ = (float*)A(kGuideParams * 4);
+        grad_ = (float*)A(kGuideParams * 4 + 16);  // and the loss statistics and error word of a gradient call
         part_ = (float*)A((size_t)nparts_ * kGuideParams * 4);
         adam_m_ = (float*)A(kGuideParams * 4);
         adam_v_ = (float*)A(kGuideParams * 4);
@@ -968,20 +1045,19 @@ int GuideTrainer::train_parts() {
 void GuideTrainer::train(cudaStream_t st, const float4* out_L, int wave_paths, int steps, int* err) {
     cudaMemsetAsync(batch_count_, 0, 16, st);
     cudaMemsetAsync(loss_acc_, 0, 32, st);
-    k_guide_batch<<<(int)std::min<size_t>(4096, (rec_cap_ + 255) / 256), 256, 0, st>>>(
+    k_guide_batch<<<(int)std::min<size_t>(4096, (rec_cap_ + kBatchThreads - 1) / kBatchThreads), kBatchThreads, 0, st>>>(
         rec_, (int)rec_cap_, rec_depth_, rec_stride_, out_L, wave_paths, batch_, batch_count_, loss_acc_, (int)rec_cap_);
     prepare_launch();
     GuideNet net = view(false, false).net;
     // per Adam step: the fused tensor-core forward/backward over one minibatch window (partial
-    // gradients per warpgroup), Adam over their sum, and the step counter; k_guide_tick clears the
-    // loss accumulators for the next step
+    // gradients per warpgroup), then Adam over their sum, which also advances the step counter and
+    // clears the loss accumulators for the next step
     for (int s = 0; s < steps; s++) {
         k_guide_train_tc<<<g_train_grid, kTgThreads, kTgSmem, st>>>(net, batch_, batch_count_, (int)rec_cap_, part_, loss_acc_,
                                                                    std::min(steps, windows_), step_dev_, err);
         steps_++;
-        k_guide_adam<<<64, 256, 0, st>>>(params_, part_, nparts_, adam_m_, adam_v_, bf_, loss_acc_, lr_, 0.9f, 0.99f, 1e-8f,
-                                         step_dev_, lr_decay_);
-        k_guide_tick<<<1, 1, 0, st>>>(step_dev_, loss_acc_);
+        k_guide_adam<<<kSumBlocks, kSumThreads, 0, st>>>(params_, part_, nparts_, adam_m_, adam_v_, bf_, loss_acc_, lr_, 0.9f, 0.99f,
+                                                         1e-8f, step_dev_, lr_decay_);
     }
 }
 
@@ -1055,44 +1131,37 @@ int GuideTrainer::eval(DeviceArena& arena, const float* host_xnw, int n, float* 
 int GuideTrainer::gradient(DeviceArena& arena, const float* host_samples, int n, float* host_grad, double* loss, std::string& err) {
     if (!params_) { err = "guide network not initialised"; return C2G_ERR_STATE; }
     if (n <= 0) { err = "empty batch"; return C2G_ERR_INVALID; }
-    std::vector<float4> b((size_t)n * 4);
-    for (int j = 0; j < n; j++) {
-        const float* v = host_samples + (size_t)14 * j;
-        b[4 * j] = make_float4(v[0], v[1], v[2], v[12]);
-        b[4 * j + 1] = make_float4(v[3], v[4], v[5], 0.f);
-        b[4 * j + 2] = make_float4(v[6], v[7], v[8], 0.f);
-        b[4 * j + 3] = make_float4(v[9], v[10], v[11], v[13]);
-    }
-    float4* db = (float4*)arena.alloc(b.size() * 16, err);
-    int* derr = (int*)arena.alloc(16, err);
-    if (!db || !derr) {
-        if (db) arena.free(db);
-        if (derr) arena.free(derr);
-        return C2G_ERR_OOM;
-    }
-    // stats[2] = n makes the kernel's weight normaliser (mean weight) exactly 1
-    float st[8] = {0.f, 0.f, (float)n, 0.f, 0.f, 0.f, 0.f, 0.f};
-    cudaMemcpy(db, b.data(), b.size() * 16, cudaMemcpyHostToDevice);
-    cudaMemcpy(batch_count_, &n, 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(loss_acc_, st, 32, cudaMemcpyHostToDevice);
-    cudaMemset(derr, 0, 16);
+    // batch (64 bytes per sample), the samples as given, the error word
+    const size_t raw = (size_t)n * 14 * 4, packed = (size_t)n * 64;
+    unsigned char* buf = (unsigned char*)arena.alloc(packed + raw + 16, err);
+    if (!buf) return C2G_ERR_OOM;
+    float4* db = (float4*)buf;
+    float* ds = (float*)(buf + packed);
+    int* derr = (int*)(buf + packed + raw);
+    cudaMemcpy(ds, host_samples, raw, cudaMemcpyHostToDevice);
     prepare_launch();
+    k_guide_pack<<<(n + 255) / 256, 256>>>(ds, n, db, batch_count_, loss_acc_, derr);
     k_guide_train_tc<<<g_train_grid, kTgThreads, kTgSmem>>>(view(false, false).net, db, batch_count_, n, part_, loss_acc_, 1,
                                                            step_dev_, derr);
-    k_guide_reduce<<<64, 256>>>(part_, nparts_, grad_);
-    int rc = C2G_OK, h = 0;
-    if (cudaDeviceSynchronize() != cudaSuccess) { err = cudaGetErrorString(cudaGetLastError()); rc = C2G_ERR_CUDA; }
-    else if (cudaMemcpy(&h, derr, 4, cudaMemcpyDeviceToHost) == cudaSuccess && h) {
-        err = "guide training: tensor-core completion wait timed out";
-        rc = C2G_ERR_DEVICE;
+    k_guide_reduce<<<kSumBlocks, kSumThreads>>>(part_, nparts_, grad_, loss_acc_, derr);
+    int rc = C2G_OK;
+    std::vector<float> out(kGuideParams + 4);
+    if (cudaMemcpy(out.data(), grad_, out.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+        err = cudaGetErrorString(cudaGetLastError());
+        rc = C2G_ERR_CUDA;
     } else {
-        cudaMemcpy(host_grad, grad_, kGuideParams * 4, cudaMemcpyDeviceToHost);
-        cudaMemcpy(st, loss_acc_, 32, cudaMemcpyDeviceToHost);
-        if (loss) *loss = st[1] > 0 ? (double)st[0] / st[1] : 0.0;
+        int h = 0;
+        std::memcpy(&h, &out[kGuideParams + 2], 4);
+        if (h) {
+            err = "guide training: tensor-core completion wait timed out";
+            rc = C2G_ERR_DEVICE;
+        } else {
+            std::memcpy(host_grad, out.data(), kGuideParams * 4);
+            const float ls = out[kGuideParams], wsum = out[kGuideParams + 1];
+            if (loss) *loss = wsum > 0 ? (double)ls / wsum : 0.0;
+        }
     }
-    cudaMemset(loss_acc_, 0, 32);
-    arena.free(db);
-    arena.free(derr);
+    arena.free(buf);
     return rc;
 }
 

@@ -1985,7 +1985,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         begin(C2G_K_TRAIN, st);
         guide_.train(st, w.out_L, a.nslots * a.wave_samples, guide_train_steps_, S.err);
         end(st);
-        launches += 1 + 3 * guide_train_steps_;
+        launches += 1 + 2 * guide_train_steps_;
     }
     if (a.sample0_dev && advance) {
         k_advance<<<1, 1, 0, st>>>(const_cast<int*>(a.sample0_dev), a.wave_samples);
