@@ -202,34 +202,33 @@ __device__ __forceinline__ int warp_append_keyed(int* counters, int key) {
 }
 
 // ---- raygen (SamplerIntegrator.cpp:42-55 + PerspCamera::GenerateRay) -----------------------------
+// A path's place in the queue is the number of valid slots before its own, in closed form (8 x 8 tiles,
+// cut at the right and lower edge): taking it from a counter serialised the kernel on one address, about
+// 1.5 ns per warp (33.2M paths at 1080p: 1.65 -> 0.60 ms).
 __global__ void k_raygen(DevScene S, WaveArgs a, PathRefs out, float4* out_L, int* qcount) {
     const int total = a.nslots * a.wave_samples;
     const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x; base < total; base += stride) {
-        int pid = base + threadIdx.x;
-        bool valid = pid < total;
-        int x = 0, y = 0, s_local = 0;
-        if (valid) {
-            s_local = pid / a.nslots;
-            slot_pixel(a, pid - s_local * a.nslots, x, y);
-            valid = x < a.W && y < a.H;
-            out_L[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        int j = warp_append(qcount, valid);
-        if (valid) {
-            int sample = wave_sample0(a) + s_local;
-            int vidx = S.sampler == SAMPLER_HALTON ? halton_vector_index(S.hp, x, y, sample) : 0;
-            const float2 sj = path_sample2(S, vidx, 0, (uint32_t)(y * a.W + x), (uint32_t)sample);
-            float sx = sj.x, sy = sj.y;
-            float nx, ny;
-            pixel_ndc(x, y, sx, sy, a.W, a.H, nx, ny);
-            float3 o, d;
-            camera_ray(S.cam, nx, ny, o, d);
-            out.o[j] = make_float4(o.x, o.y, o.z, __int_as_float(pid));
-            out.d[j] = make_float4(d.x, d.y, d.z, __int_as_float(pack_state(2, 0, 1)));
-            out.beta[j] = make_float4(1.f, 1.f, 1.f, __int_as_float(vidx));
-            out.L[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *qcount = a.W * a.H * a.wave_samples;
+    for (int pid = blockIdx.x * blockDim.x + threadIdx.x; pid < total; pid += stride) {
+        const int s_local = pid / a.nslots, slot = pid - s_local * a.nslots;
+        const int tile = slot >> 6, w = slot & 63, ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
+        const int x = tx * 8 + (w & 7), y = ty * 8 + (w >> 3);
+        if (x >= a.W || y >= a.H) continue;
+        const int tw = min(8, a.W - tx * 8), th = min(8, a.H - ty * 8);  // the tile's valid width and height
+        const int j = s_local * a.W * a.H + ty * 8 * a.W + tx * 8 * th + (w >> 3) * tw + (w & 7);
+        out_L[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        int sample = wave_sample0(a) + s_local;
+        int vidx = S.sampler == SAMPLER_HALTON ? halton_vector_index(S.hp, x, y, sample) : 0;
+        const float2 sj = path_sample2(S, vidx, 0, (uint32_t)(y * a.W + x), (uint32_t)sample);
+        float sx = sj.x, sy = sj.y;
+        float nx, ny;
+        pixel_ndc(x, y, sx, sy, a.W, a.H, nx, ny);
+        float3 o, d;
+        camera_ray(S.cam, nx, ny, o, d);
+        out.o[j] = make_float4(o.x, o.y, o.z, __int_as_float(pid));
+        out.d[j] = make_float4(d.x, d.y, d.z, __int_as_float(pack_state(2, 0, 1)));
+        out.beta[j] = make_float4(1.f, 1.f, 1.f, __int_as_float(vidx));
+        out.L[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
