@@ -97,7 +97,7 @@ struct WaveBuffers {
     int* sh_list = nullptr;
     int* mis_list = nullptr;
     int* bucket_list = nullptr;  // kBuckets lists of P slots
-    int* counters = nullptr;  // [0],[1] path queues, [2] shadow, [3] mis, [4] shadow and [5] extension rays handed out, [8..20) material buckets, [24] MIS rays handed out
+    int* counters = nullptr;  // kCntTotal of them
     int* levels = nullptr;    // statistics: paths entering each bounce level (C2G_LEVELS)
     std::vector<void*> owned;
 };
@@ -186,9 +186,22 @@ struct PathRefs {
 // Hits are shaded per material bucket: 0..7 = MatType of the hit's material, 8 = no material
 // (pass-through), 9 = miss.  k_extend appends each queue slot to its bucket; one specialised
 // k_shade<bucket> per bucket then runs without material divergence.
-constexpr int kCntBucket = 8;  // counters[8 .. 8 + kBuckets): bucket sizes
-constexpr int kCntMisFetch = 24;  // MIS rays handed out (zeroed by k_accumulate)
-constexpr int kCntFinish = 32;    // paths handed out by k_finish (once per wave)
+//
+// Each counter has 256 bytes to itself.  An address serves an atomic in about 1.5 ns and neighbours in a
+// line wait for each other: with all of them in one line the extension kernel, whose warps fetch rays
+// from one counter while they append to the buckets' (Cornell box, 4.2M paths), took 1.03 ms, now 0.90.
+// The bucket sizes stay side by side; apart they measured the same.
+constexpr int kLine = 64;
+constexpr int kCntShadow = 2 * kLine;       // after path queues 0 and 1 (at q * kLine)
+constexpr int kCntMis = 3 * kLine;
+constexpr int kCntShadowFetch = 4 * kLine;  // rays handed out
+constexpr int kCntExtendFetch = 5 * kLine;
+constexpr int kCntBucket = 6 * kLine;       // kBuckets sizes
+constexpr int kCntMisFetch = 7 * kLine;     // zeroed by k_accumulate
+constexpr int kCntFinish = 8 * kLine;       // paths handed out by k_finish (once per wave)
+constexpr int kCntSpare = 9 * kLine;        // slots no kernel reads
+constexpr int kCntTotal = 12 * kLine;
+static_assert(kBuckets <= kLine, "the bucket sizes share a line");
 
 // Warp-aggregated append into per-key lists (lanes with equal keys share one atomic).
 // Must be called by all 32 lanes; key < 0 appends nothing.
@@ -261,7 +274,7 @@ __global__ void k_extend(DevScene S, const float4* __restrict__ qo, const float4
                          int cap, volatile int* report, unsigned long long* cnt) {
     const int n = *qcount;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0;  // + shadow fetch counter
+        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[kCntShadowFetch - kCntShadow] = 0;  // + shadow fetch counter
         if (report) *report = n;
     }
     const int stride = gridDim.x * blockDim.x;
@@ -332,7 +345,7 @@ __global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_extend_fetch(Dev
                                                       int* bucket_cnt, int* bucket_list, int cap, volatile int* report,
                                                       int* fetch, unsigned long long* cnt) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[2] = 0;  // + shadow fetch counter
+        *zero_a = 0; *zero_b = 0; *zero_c = 0; zero_b[kCntShadowFetch - kCntShadow] = 0;  // + shadow fetch counter
         if (report) *report = *qcount;
     }
     ExtendLane<COUNT, R> L{{}, S, qo, qd, hit, bucket_cnt, bucket_list, cap};
@@ -1642,39 +1655,39 @@ void launch_extend(const DevScene& S, int tb, const WaveBuffers& w, int q, int* 
                    bool count, unsigned long long* cnt, cudaStream_t st) {
     const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].ext[k][count];
     int* C = w.counters;
-#define C2G_ARGS S, w.o[q], w.d[q], w.hit, C + q, za, zb, zc, C + kCntBucket, w.bucket_list, (int)w.P, report
+#define C2G_ARGS S, w.o[q], w.d[q], w.hit, C + q * kLine, za, zb, zc, C + kCntBucket, w.bucket_list, (int)w.P, report
     if (k == TRACE_PLAIN) {
         if (count) k_extend<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_extend<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
     } else if (k == TRACE_QUANT4) {
-        if (count) k_extend_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
-        else k_extend_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+        if (count) k_extend_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
+        else k_extend_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
     } else {
-        if (count) k_extend_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
-        else k_extend_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 5, cnt);
+        if (count) k_extend_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
+        else k_extend_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
     }
 #undef C2G_ARGS
 }
 void launch_shadow(const DevScene& S, int tb, const WaveBuffers& w, bool count, unsigned long long* cnt, cudaStream_t st) {
     const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].sh[k][count];
     int* C = w.counters;
-#define C2G_ARGS S, w.sh_list, C + 2, w.sh_o, w.sh_d, w.sh_c
+#define C2G_ARGS S, w.sh_list, C + kCntShadow, w.sh_o, w.sh_d, w.sh_c
     if (k == TRACE_PLAIN) {
         if (count) k_shadow<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_shadow<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
     } else if (k == TRACE_QUANT4) {
-        if (count) k_shadow_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
-        else k_shadow_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+        if (count) k_shadow_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
+        else k_shadow_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
     } else {
-        if (count) k_shadow_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
-        else k_shadow_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + 4, cnt);
+        if (count) k_shadow_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
+        else k_shadow_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
     }
 #undef C2G_ARGS
 }
 void launch_mis(const DevScene& S, int tb, const WaveBuffers& w, bool count, unsigned long long* cnt, cudaStream_t st) {
     const int k = trace_kind(S), g = g_trace[trace_block_index(tb)].mis[k][count];
     int* C = w.counters;
-#define C2G_ARGS S, w.mis_list, C + 3, w.mis_o, w.mis_d, w.mis_hit
+#define C2G_ARGS S, w.mis_list, C + kCntMis, w.mis_o, w.mis_d, w.mis_hit
     if (k == TRACE_PLAIN) {
         if (count) k_mis<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_mis<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
@@ -1695,8 +1708,8 @@ void launch_finish(const DevScene& S, const WaveArgs& a, const WaveBuffers& w, i
     const PathRefs cur{w.o[q], w.d[q], w.beta[q], w.L[q]};
     const float4* hits = have_hits ? w.hit : nullptr;
     int* C = w.counters;
-    if (exact) k_finish<RayQ><<<g_finish[1], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q, C + kCntFinish, finish_log2g(a.K));
-    else k_finish<Ray4><<<g_finish[0], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q, C + kCntFinish, finish_log2g(a.K));
+    if (exact) k_finish<RayQ><<<g_finish[1], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q * kLine, C + kCntFinish, finish_log2g(a.K));
+    else k_finish<Ray4><<<g_finish[0], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q * kLine, C + kCntFinish, finish_log2g(a.K));
 }
 
 __global__ void k_advance(int* sample0, int by) { *sample0 += by; }
@@ -1779,7 +1792,7 @@ int GpuScene::prepare(const c2g_render_params& p, DeviceArena& arena, WavePlan& 
              (wb_->sh_o = (float4*)A(PK * 16)) && (wb_->sh_d = (float4*)A(PK * 16)) && (wb_->sh_c = (float4*)A(PK * 16)) &&
              (wb_->mis_o = (float4*)A(P * 16)) && (wb_->mis_d = (float4*)A(P * 16)) && (wb_->mis_c = (float4*)A(PK * 16)) &&
              (wb_->mis_hit = (float4*)A(P * 16)) && (wb_->sh_list = (int*)A(PK * 4)) && (wb_->mis_list = (int*)A(P * 4)) &&
-             (wb_->bucket_list = (int*)A(P * 4 * kBuckets)) && (wb_->counters = (int*)A(256)) &&
+             (wb_->bucket_list = (int*)A(P * 4 * kBuckets)) && (wb_->counters = (int*)A(kCntTotal * sizeof(int))) &&
              (wb_->levels = (int*)A(4 * C2G_LEVELS));
         if (!ok) {
             for (void* q : wb_->owned) arena.free(q);
@@ -1820,25 +1833,24 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         cudaStreamWaitEvent(st, join_ev_[k], 0);
     };
     int* C = w.counters;
-    C2G_CUDA(cudaMemsetAsync(C, 0, 256, st));
+    C2G_CUDA(cudaMemsetAsync(C, 0, kCntTotal * sizeof(int), st));
     PathRefs buf[2] = {{w.o[0], w.d[0], w.beta[0], w.L[0]}, {w.o[1], w.d[1], w.beta[1], w.L[1]}};
     begin(C2G_K_RAYGEN, st);
     k_raygen<<<g_raygen, 256, 0, st>>>(S, a, buf[0], w.out_L, C + 0);
     end(st);
     // Extension of the paths in queue q on stream es: closest hits, appended to the material buckets.
-    // Block 0 zeroes *za (the count of the queue this level's shading fills), *zb and zb[2] (the
-    // shadow queue and its fetch counter) and *zc (the MIS queue): the live counters when it runs in
+    // Block 0 zeroes *za (the count of the queue this level's shading fills), *zb and its fetch counter (the
+    // shadow queue) and *zc (the MIS queue): the live counters when it runs in
     // order, spare slots when it runs ahead beside the previous level's shadow rays (the live ones
     // are then zeroed on st after that level's accumulation).
     auto extend = [&](int q, int* za, int* zb, int* zc, int* report, cudaStream_t es) {
         begin(C2G_K_EXTEND, es);
-        // bucket sizes and the extension fetch counter C[5] start at zero on every level
-        cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), es);
+        // the extension fetch counter and the bucket sizes start at zero on every level
+        cudaMemsetAsync(C + kCntExtendFetch, 0, sizeof(int) * (kCntBucket - kCntExtendFetch + kBuckets), es);
         launch_extend(S, tb, w, q, za, zb, zc, report, count, cnt, es);
         end(es);
     };
-    int* const spare = C + 56;  // counter slots no kernel reads
-    static_assert(kCntBucket + kBuckets <= kCntMisFetch && kCntMisFetch < 56, "counter layout");
+    int* const spare = C + kCntSpare;  // counter slots no kernel reads
     bool ahead_done = false;    // this level's extension was launched during the previous level
     int cur = 0;
     // k_finish takes over a queue of at most kFinishPaths paths.  An eager render learns the queue's size
@@ -1877,15 +1889,15 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         if (b >= a.max_depth && a.integrator == C2G_INTEGRATOR_DIRECT && !poll) {
             // pass-through hops past the depth: stop once the queue is empty
             int qn = 0;
-            C2G_CUDA(cudaMemcpyAsync(&qn, C + cur, sizeof(int), cudaMemcpyDeviceToHost, st));
+            C2G_CUDA(cudaMemcpyAsync(&qn, C + cur * kLine, sizeof(int), cudaMemcpyDeviceToHost, st));
             C2G_CUDA(cudaStreamSynchronize(st));
             if (qn == 0) break;
         }
         // statistics: the paths entering this level
-        if (count) k_level_add<<<1, 1, 0, st>>>(w.levels + std::min(b, C2G_LEVELS - 1), C + cur);
+        if (count) k_level_add<<<1, 1, 0, st>>>(w.levels + std::min(b, C2G_LEVELS - 1), C + cur * kLine);
         const bool pre = ahead_done;
         if (pre) cudaStreamWaitEvent(st, join_ev_[2], 0);
-        else extend(cur, C + nxt, C + 2, C + 3, nullptr, st);
+        else extend(cur, C + nxt * kLine, C + kCntShadow, C + kCntMis, nullptr, st);
         // the guide serves the first guide_levels_ bounce levels; deeper vertices shade plainly
         const bool glevel = guided && (guide_levels_ <= 0 || b < guide_levels_);
         if (gv.sample && glevel && !pre) {
@@ -1894,7 +1906,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
                                      present_buckets_);
             end(st);
         }
-        ShadeOut so{buf[nxt], C + nxt, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + 2, C + 3, w.acc, w.mis_hit};
+        ShadeOut so{buf[nxt], C + nxt * kLine, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + kCntShadow, C + kCntMis, w.acc, w.mis_hit};
         // the material buckets are independent (they append to the shared queues with atomics):
         // with overlap the present buckets take the three streams in turn
         if (overlap) {
@@ -1924,7 +1936,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         if (overlap && (poll || a.integrator != C2G_INTEGRATOR_DIRECT) && b + 1 < levels) {
             cudaEventRecord(fork_ev_[2], st);
             cudaStreamWaitEvent(ahead_, fork_ev_[2], 0);
-            extend(nxt, spare, spare + 1, spare + 4, poll ? report_dev_ + b + 1 : nullptr, ahead_);
+            extend(nxt, spare, spare, spare, poll ? report_dev_ + b + 1 : nullptr, ahead_);
             launches++;
             // the next level's guide inference needs only its rays and hits: it follows on the
             // same stream (this level's shading has read its mixtures already)
@@ -1956,13 +1968,13 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
             end(st);
         }
         begin(C2G_K_ACCUM, st);
-        k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, gv, C + kCntMisFetch);
+        k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur * kLine, gv, C + kCntMisFetch);
         end(st);
         if (ahead_done) {
             // the counters the look-ahead extension left alone: the queue after the next level, the
             // shadow and MIS queues and the shadow fetch counter
-            cudaMemsetAsync(C + cur, 0, sizeof(int), st);
-            cudaMemsetAsync(C + 2, 0, 3 * sizeof(int), st);
+            cudaMemsetAsync(C + cur * kLine, 0, sizeof(int), st);
+            cudaMemsetAsync(C + kCntShadow, 0, (kCntShadowFetch - kCntShadow + 1) * sizeof(int), st);
         }
         launches += pre ? 3 : 4;
         cur = nxt;
@@ -2375,7 +2387,7 @@ constexpr size_t kNoAllocPathBytes = 2 * 4 * 16   // o, d, beta, L (ping-pong)
                                    + 3 * 16 + 4   // mis_o, mis_d, mis_hit, mis_list
                                    + 4 * kBuckets // bucket lists
                                    + (size_t)kNoAllocLights * (4 * 16 + 4);  // sh_o, sh_d, sh_c, mis_c, sh_list
-constexpr size_t kNoAllocBytes = (size_t)kNoAllocSlots * kNoAllocPathBytes + 256;
+constexpr size_t kNoAllocBytes = (size_t)kNoAllocSlots * kNoAllocPathBytes + kCntTotal * sizeof(int);
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 namespace {
@@ -2443,7 +2455,7 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
     w.mis_c = (float4*)take(PK * 16);
     w.sh_list = (int*)take(PK * 4);
     float4* m2 = (float4*)take(P * 16);
-    w.counters = (int*)take(256);
+    w.counters = (int*)take(kCntTotal * sizeof(int));
     if ((size_t)(q - (unsigned char*)g_noalloc_ptr[dev]) > kNoAllocBytes) { err = "allocation-free render: scratch layout overflow"; return C2G_ERR_INVALID; }
     w.P = P;
     w.K = a.K;
@@ -2462,7 +2474,7 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
     for (int s0 = 0; s0 < p.sample_count; s0++) {
         a.wave_samples = 1;
         a.sample0 = p.sample_begin + s0;
-        C2G_CUDA(cudaMemsetAsync(C, 0, 256, st));  // counters start at zero for every wave
+        C2G_CUDA(cudaMemsetAsync(C, 0, kCntTotal * sizeof(int), st));  // counters start at zero for every wave
         k_raygen<<<g_raygen, 256, 0, st>>>(S, a, buf[0], w.out_L, C + 0);
         int cur = 0;
         for (int b = 0; b < levels; b++) {
@@ -2470,19 +2482,19 @@ int GpuScene::render_noalloc(const c2g_render_params& p, float4* film_dev, cudaS
             if (b >= a.max_depth) {
                 // the queue count goes to a host stack variable: no allocation
                 int qn = 0;
-                C2G_CUDA(cudaMemcpyAsync(&qn, C + cur, sizeof(int), cudaMemcpyDeviceToHost, st));
+                C2G_CUDA(cudaMemcpyAsync(&qn, C + cur * kLine, sizeof(int), cudaMemcpyDeviceToHost, st));
                 C2G_CUDA(cudaStreamSynchronize(st));
                 if (qn == 0) break;
             }
-            C2G_CUDA(cudaMemsetAsync(C + 5, 0, sizeof(int) * (kCntBucket - 5 + kBuckets), st));
-            launch_extend(S, 128, w, cur, C + nxt, C + 2, C + 3, nullptr, false, nullptr, st);
-            ShadeOut so{buf[nxt], C + nxt, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + 2, C + 3, w.acc, w.mis_hit};
+            C2G_CUDA(cudaMemsetAsync(C + kCntExtendFetch, 0, sizeof(int) * (kCntBucket - kCntExtendFetch + kBuckets), st));
+            launch_extend(S, 128, w, cur, C + nxt * kLine, C + kCntShadow, C + kCntMis, nullptr, false, nullptr, st);
+            ShadeOut so{buf[nxt], C + nxt * kLine, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + kCntShadow, C + kCntMis, w.acc, w.mis_hit};
             for (int bk = 0; bk < kBuckets; bk++)
                 if (present_buckets_ & (1 << bk))
                     launch_shade(bk, g_shade, st, S, a, buf[cur], w.hit, C + kCntBucket, w.bucket_list, (int)w.P, so, GuideView{}, false);
             launch_shadow(S, 128, w, false, nullptr, st);
             launch_mis(S, 128, w, false, nullptr, st);
-            k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur, GuideView{}, C + kCntMisFetch);
+            k_accumulate<<<g_acc, 256, 0, st>>>(a, buf[cur], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + cur * kLine, GuideView{}, C + kCntMisFetch);
             cur = nxt;
         }
         // the caller's film gets the radiance sums and weights; the sums of squares stay in scratch
