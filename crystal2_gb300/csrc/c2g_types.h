@@ -50,7 +50,7 @@ struct alignas(16) Material {
     float color[4];        // Color / Kd
     float ks[4];           // Ks (Plastic)
     int tex;               // Kd texture (UVTexture) index, -1: the constant color
-    int pad[3];
+    float color_pi[3];     // color / pi, as Lambert and Oren-Nayar reflection use it
 };
 
 enum LightType : int { LIGHT_AREA = 0, LIGHT_POINT = 1 };

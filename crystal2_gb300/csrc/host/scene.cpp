@@ -259,6 +259,7 @@ struct Loader {
         } else {
             throw SceneError(C2G_ERR_INVALID, "Invalid material name");
         }
+        for (int i = 0; i < 3; i++) m.color_pi[i] = m.color[i] / fm::kPi;
         s.mats.push_back(m);
         return (int)s.mats.size() - 1;
     }

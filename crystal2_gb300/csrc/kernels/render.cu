@@ -459,7 +459,10 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
             } else {
                 bx = make_bxdf(S.mats[s.mat], s.front);
                 const int tex = S.mats[s.mat].tex;
-                if (tex >= 0) bx.R = tex_lookup(S, tex, surface_uv(S, ro, rd, h));  // Kd texture
+                if (tex >= 0) {  // Kd texture
+                    bx.R = tex_lookup(S, tex, surface_uv(S, ro, rd, h));
+                    bx.R_pi = bx.R / kPiF;
+                }
                 bx.mtype = MT;  // compile-time material: the BxDF switches fold away
                 bx.flags = material_flags(MT);
                 fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
@@ -968,7 +971,10 @@ __device__ __noinline__ void finish_shade(const DevScene& S, const WaveArgs& a, 
     } else {
         BxDF bx = make_bxdf(S.mats[s.mat], s.front);
         const int tex = S.mats[s.mat].tex;
-        if (tex >= 0) bx.R = tex_lookup(S, tex, surface_uv(S, ro, rd, h));
+        if (tex >= 0) {
+            bx.R = tex_lookup(S, tex, surface_uv(S, ro, rd, h));
+            bx.R_pi = bx.R / kPiF;
+        }
         bx.mtype = MT;
         bx.flags = material_flags(MT);
         Frame fr;
