@@ -28,6 +28,8 @@ struct BxDF {
     float3 S;           // ks (plastic)
     float ax, ay;
     float etaA, etaB;
+    float eta_ab, eta_ba;  // etaA / etaB, etaB / etaA
+    float term_o;       // what f takes from wo alone (bsdf_prepare)
 };
 
 __device__ __forceinline__ int material_flags(int mtype) {
@@ -61,6 +63,8 @@ __device__ __forceinline__ BxDF make_bxdf(const Material& m, bool front_face) {
     const bool dielectric = m.type != MAT_MIRROR && m.type != MAT_DIFFUSE && m.type != MAT_ORENNAYAR && m.type != MAT_BLINNPHONG;
     b.etaB = dielectric ? m.ior : 1.f;
     if (!front_face && dielectric) { float t = b.etaA; b.etaA = b.etaB; b.etaB = t; }
+    b.eta_ab = b.etaA / b.etaB;
+    b.eta_ba = b.etaB / b.etaA;
     if (m.type == MAT_BLINNPHONG) b.ax = m.ior;  // the exponent K
     return b;
 }
@@ -78,25 +82,26 @@ __device__ __forceinline__ float over_pi(float x) {
 }
 
 // ---- Fresnel (BSDFs/Models/Fresnel.cpp) -------------------------------------------------
-__device__ __forceinline__ float fresnel_dielectric(float etaA, float etaB, float cosI) {
+__device__ __forceinline__ float fresnel_dielectric(const BxDF& b, float cosI) {
+    const float etaA = b.etaA, etaB = b.etaB;
     float sinI = sqrtf(fmaxf(0.f, 1.f - cosI * cosI));
-    float sinT = etaA / etaB * sinI;
+    float sinT = b.eta_ab * sinI;
     if (sinT >= 1.f) return 1.f;
     float cosT = sqrtf(fmaxf(0.f, 1.f - sinT * sinT));
     float rparl = ((etaB * cosI) - (etaA * cosT)) / ((etaB * cosI) + (etaA * cosT));
     float rperp = ((etaA * cosI) - (etaB * cosT)) / ((etaA * cosI) + (etaB * cosT));
     return (rparl * rparl + rperp * rperp) / 2;
 }
-__device__ __forceinline__ float fresnel_schlick(float r0, float etaA, float etaB, float cosI) {
+__device__ __forceinline__ float fresnel_schlick(float r0, const BxDF& b, float cosI) {
     float sinI = sqrtf(fmaxf(0.f, 1.f - cosI * cosI));
-    float sinT = etaA / etaB * sinI;
+    float sinT = b.eta_ab * sinI;
     if (sinT >= 1.f) return 1.f;
     return r0 + (1.f - r0) * powf(1.f - cosI, 5.f);
 }
 // Micro uses Schlick with R0 = 0.99 (MicrofacetMaterial.cpp:23); glass uses the dielectric.
 __device__ __forceinline__ float bxdf_fresnel(const BxDF& b, float cosI) {
-    if (b.mtype == MAT_MICRO_GGX || b.mtype == MAT_MICRO_BECKMANN) return fresnel_schlick(0.99f, b.etaA, b.etaB, cosI);
-    return fresnel_dielectric(b.etaA, b.etaB, cosI);
+    if (b.mtype == MAT_MICRO_GGX || b.mtype == MAT_MICRO_BECKMANN) return fresnel_schlick(0.99f, b, cosI);
+    return fresnel_dielectric(b, cosI);
 }
 
 // ---- microfacet distributions (BSDFs/Models/MicrofacetDistribution.cpp) -------------------
@@ -147,11 +152,8 @@ __device__ __forceinline__ float ndf_lambda(const BxDF& b, float3 w) {
     return (1 - 1.259f * a + 0.396f * a * a) / (3.535f * a + 2.181f * a * a);
 }
 
-__device__ __forceinline__ float ndf_G(const BxDF& b, float3 wo, float3 wi) {
-    return 1.f / (1.f + ndf_lambda(b, wo) + ndf_lambda(b, wi));
-}
-
-__device__ __forceinline__ float ndf_pdf(const BxDF& b, float3 wh) { return ndf_D(b, wh) * fabsf(wh.y); }
+// Smith's G of the prepared wo (b.term_o is its Lambda) and wi.
+__device__ __forceinline__ float ndf_G(const BxDF& b, float3 wi) { return 1.f / (1.f + b.term_o + ndf_lambda(b, wi)); }
 
 // GetUnitVectorUsingCos (Utils.h:79-83)
 __device__ __forceinline__ float3 unit_from_cos(float cosT, float phi) {
@@ -209,54 +211,74 @@ __device__ __forceinline__ bool refract(float3 wo, float3 wh, float eta, float3&
 }
 
 // ---- microfacet BxDFs (BSDFs/Microfacet.cpp) --------------------------------------------
-__device__ __forceinline__ float mf_refl_pdf(const BxDF& b, float3 wo, float3 wi) {
-    float3 H = normalize(wo + wi);
-    return ndf_pdf(b, H) / (4 * dot(wo, H));
-}
-__device__ __forceinline__ float3 mf_refl_f(const BxDF& b, float3 wo, float3 wi) {
+// The density of a direction and the value of the BxDF share the half vector H and D(H); a vertex
+// evaluates them for every light and for two samples of its own, and a GGX evaluation is some twenty
+// divisions and square roots.  So Lambda(wo), and the Fresnel blend's power of wo, are kept for the vertex
+// (bsdf_prepare), and a sampled direction uses its H and D twice, unless the clamp that follows the
+// density changed it.  Shading of the slit room (most of it GGX): 4.65 -> 4.30 ms, of the many-material frame 12.7 -> 11.3.
+__device__ __forceinline__ float mf_refl_pdf(float3 wo, float3 H, float D) { return D * fabsf(H.y) / (4 * dot(wo, H)); }
+__device__ __forceinline__ float3 mf_refl_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
     if (wo.y * wi.y < 0) return f3(0.f, 0.f, 0.f);
-    float3 H = normalize(wo + wi);
     float F = bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wo, wi);
-    float D = ndf_D(b, H);
+    float G = ndf_G(b, wi);
     return b.R * D * G * F / (4 * fmaxf(0.f, wi.y) * fmaxf(0.f, wo.y));
 }
-__device__ __forceinline__ float mf_trans_pdf(const BxDF& b, float3 wo, float3 wi) {
+__device__ __forceinline__ float mf_trans_pdf(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
     if (wo.y * wi.y > 0) return 0.f;
-    float eta = b.etaB / b.etaA;
-    float3 H = normalize(wo + wi * eta);
-    float absDot = fabsf(dot(H, wi));
-    float dwh = eta * eta * absDot / sq(dot(wo, H) + eta * dot(wi, H));
-    return ndf_pdf(b, H) * dwh;
+    float eta = b.eta_ba;
+    float s = dot(wo, H) + eta * dot(wi, H);
+    return D * fabsf(H.y) * (eta * eta * fabsf(dot(H, wi)) / sq(s));
 }
-__device__ __forceinline__ float3 mf_trans_f(const BxDF& b, float3 wo, float3 wi) {
+__device__ __forceinline__ float3 mf_trans_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
     if (wi.y * wo.y > 0) return f3(0.f, 0.f, 0.f);
     if (wo.y == 0.f) return f3(0.f, 0.f, 0.f);
-    float eta = b.etaB / b.etaA;
-    float3 H = normalize(wo + wi * eta);
-    if (H.y < 0) H = -H;
+    float eta = b.eta_ba;
+    if (H.y < 0) H = -H;  // D is even in H
     float bot = sq(dot(wo, H) + eta * dot(wi, H));
     float F = 1.f - bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wo, wi);
-    float D = ndf_D(b, H);
+    float G = ndf_G(b, wi);
     return b.R * D * G * F * fabsf(dot(H, wo)) * fabsf(dot(H, wi)) / (bot * fmaxf(0.f, -wi.y) * fmaxf(0.f, wo.y));
+}
+// Half vector of a reflection, or of a transmission.
+__device__ __forceinline__ float3 mf_half(const BxDF& b, bool trans, float3 wo, float3 wi) {
+    return normalize(wo + wi * (trans ? b.eta_ba : 1.f));
+}
+// f and pdf of one (wo, wi) pair.
+__device__ __forceinline__ float3 mf_f_pdf(const BxDF& b, bool trans, float3 wo, float3 wi, float& pdf) {
+    const float3 H = mf_half(b, trans, wo, wi);
+    const float D = ndf_D(b, H);
+    pdf = trans ? mf_trans_pdf(b, wo, wi, H, D) : mf_refl_pdf(wo, H, D);
+    return trans ? mf_trans_f(b, wo, wi, H, D) : mf_refl_f(b, wo, wi, H, D);
+}
+// f and pdf of a sampled direction: the density of wi as drawn, then f of wi clamped to [-1, 1].  The
+// density takes the technique from wi's side (glass), f from the technique that drew it.
+__device__ __forceinline__ float3 mf_sampled(const BxDF& b, bool trans, float3 wo, float3& wi, float& pdf) {
+    const bool across = b.mtype == MAT_GLASS_ROUGH && wo.y * wi.y < 0;
+    float3 H = mf_half(b, across, wo, wi);
+    float D = ndf_D(b, H);
+    pdf = across ? mf_trans_pdf(b, wo, wi, H, D) : mf_refl_pdf(wo, H, D);
+    const float3 c = clamp1(wi);
+    if (c.x != wi.x || c.y != wi.y || c.z != wi.z || trans != across) {
+        H = mf_half(b, trans, wo, c);
+        D = ndf_D(b, H);
+    }
+    wi = c;
+    return trans ? mf_trans_f(b, wo, wi, H, D) : mf_refl_f(b, wo, wi, H, D);
 }
 
 // ---- FresnelBlend (BSDFs/FresnelBlend.cpp) ----------------------------------------------
-__device__ __forceinline__ float fb_pdf(const BxDF& b, float3 wo, float3 wi) {
+__device__ __forceinline__ float fb_power(float cosT) { return 1.f - powf(1.f - 0.5f * cosT, 5.f); }
+__device__ __forceinline__ float3 fb_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
     float3 H = normalize(wo + wi);
-    return 0.5f * (over_pi(fmaxf(0.f, wi.y)) + ndf_pdf(b, H) / (4 * dot(wo, H)));
-}
-__device__ __forceinline__ float3 fb_f(const BxDF& b, float3 wo, float3 wi) {
+    float D = ndf_D(b, H);
+    pdf = 0.5f * (over_pi(fmaxf(0.f, wi.y)) + D * fabsf(H.y) / (4 * dot(wo, H)));
     float cosI = fmaxf(0.f, wi.y), cosO = fmaxf(0.f, wo.y);
     float k = (28.f / (23.f * kPiF));
-    float3 diffuse = k * b.R * (f3(1.f, 1.f, 1.f) - b.S) * (1.f - powf(1.f - 0.5f * cosO, 5.f)) * (1.f - powf(1.f - 0.5f * cosI, 5.f));
-    float3 H = normalize(wo + wi);
+    float3 diffuse = k * b.R * (f3(1.f, 1.f, 1.f) - b.S) * b.term_o * fb_power(cosI);
     float cwh = dot(wi, H);
-    float s = ndf_D(b, H) / (4 * cwh * fmaxf(cosI, cosO));
-    float p5 = powf(1.f - cwh, 5.f);
-    float3 schlick = b.S + (f3(1.f, 1.f, 1.f) - b.S) * p5;
-    return diffuse + s * schlick;
+    float sp = D / (4 * cwh * fmaxf(cosI, cosO));
+    float3 schlick = b.S + (f3(1.f, 1.f, 1.f) - b.S) * powf(1.f - cwh, 5.f);
+    return diffuse + sp * schlick;
 }
 
 // ---- Oren-Nayar (BSDFs/Reflections.cpp:7-66); A, B in ax, ay -----------------------------
@@ -298,77 +320,13 @@ __device__ __forceinline__ float2 phong_redraw(float2 u, int attempt) {
 }
 
 // ---- per-BxDF dispatch (local frame) ------------------------------------------------------
-__device__ __forceinline__ float3 bxdf_f(const BxDF& b, float3 wo, float3 wi) {
-    switch (b.mtype) {
-        case MAT_DIFFUSE: return b.R_pi;
-        case MAT_MICRO_GGX:
-        case MAT_MICRO_BECKMANN: return mf_refl_f(b, wo, wi);
-        case MAT_GLASS_ROUGH: return (wo.y * wi.y < 0) ? mf_trans_f(b, wo, wi) : mf_refl_f(b, wo, wi);
-        case MAT_PLASTIC_GGX:
-        case MAT_PLASTIC_BECKMANN: return fb_f(b, wo, wi);
-        case MAT_ORENNAYAR: return on_f(b, wo, wi);
-        case MAT_BLINNPHONG: return bp_f(b, wo, wi);
-    }
-    return f3(0.f, 0.f, 0.f);  // specular BxDFs
-}
-__device__ __forceinline__ float bxdf_pdf(const BxDF& b, float3 wo, float3 wi) {
-    switch (b.mtype) {
-        case MAT_DIFFUSE: return over_pi(fmaxf(0.f, wi.y));
-        case MAT_MICRO_GGX:
-        case MAT_MICRO_BECKMANN: return mf_refl_pdf(b, wo, wi);
-        case MAT_GLASS_ROUGH: return (wo.y * wi.y < 0) ? mf_trans_pdf(b, wo, wi) : mf_refl_pdf(b, wo, wi);
-        case MAT_PLASTIC_GGX:
-        case MAT_PLASTIC_BECKMANN: return fb_pdf(b, wo, wi);
-        case MAT_ORENNAYAR: return over_pi(fmaxf(0.f, wi.y));
-        case MAT_BLINNPHONG: return bp_pdf(b, wo, wi);
-    }
-    return 0.f;
-}
-
-// f and pdf of the BxDF at one (wo, wi) pair, sharing the half vector and D() between them.
-// Same values as bxdf_f / bxdf_pdf.
-__device__ __forceinline__ float3 mf_refl_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
-    float3 H = normalize(wo + wi);
-    float D = ndf_D(b, H);
-    pdf = D * fabsf(H.y) / (4 * dot(wo, H));
-    if (wo.y * wi.y < 0) return f3(0.f, 0.f, 0.f);
-    float F = bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wo, wi);
-    return b.R * D * G * F / (4 * fmaxf(0.f, wi.y) * fmaxf(0.f, wo.y));
-}
-__device__ __forceinline__ float3 mf_trans_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
-    const float3 zero = f3(0.f, 0.f, 0.f);
-    if (wo.y * wi.y > 0) { pdf = 0.f; return zero; }
-    float eta = b.etaB / b.etaA;
-    float3 H = normalize(wo + wi * eta);
-    float D = ndf_D(b, H);  // D is even in H
-    float s = dot(wo, H) + eta * dot(wi, H);
-    pdf = D * fabsf(H.y) * (eta * eta * fabsf(dot(H, wi)) / sq(s));
-    if (wo.y == 0.f) return zero;
-    if (H.y < 0) H = -H;
-    float bot = sq(dot(wo, H) + eta * dot(wi, H));
-    float F = 1.f - bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wo, wi);
-    return b.R * D * G * F * fabsf(dot(H, wo)) * fabsf(dot(H, wi)) / (bot * fmaxf(0.f, -wi.y) * fmaxf(0.f, wo.y));
-}
-__device__ __forceinline__ float3 fb_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
-    float3 H = normalize(wo + wi);
-    float D = ndf_D(b, H);
-    pdf = 0.5f * (over_pi(fmaxf(0.f, wi.y)) + D * fabsf(H.y) / (4 * dot(wo, H)));
-    float cosI = fmaxf(0.f, wi.y), cosO = fmaxf(0.f, wo.y);
-    float k = (28.f / (23.f * kPiF));
-    float3 diffuse = k * b.R * (f3(1.f, 1.f, 1.f) - b.S) * (1.f - powf(1.f - 0.5f * cosO, 5.f)) * (1.f - powf(1.f - 0.5f * cosI, 5.f));
-    float cwh = dot(wi, H);
-    float sp = D / (4 * cwh * fmaxf(cosI, cosO));
-    float3 schlick = b.S + (f3(1.f, 1.f, 1.f) - b.S) * powf(1.f - cwh, 5.f);
-    return diffuse + sp * schlick;
-}
+// f and pdf of the BxDF at one (wo, wi) pair.
 __device__ __forceinline__ float3 bxdf_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
     switch (b.mtype) {
         case MAT_DIFFUSE: pdf = over_pi(fmaxf(0.f, wi.y)); return b.R_pi;
         case MAT_MICRO_GGX:
-        case MAT_MICRO_BECKMANN: return mf_refl_f_pdf(b, wo, wi, pdf);
-        case MAT_GLASS_ROUGH: return (wo.y * wi.y < 0) ? mf_trans_f_pdf(b, wo, wi, pdf) : mf_refl_f_pdf(b, wo, wi, pdf);
+        case MAT_MICRO_BECKMANN: return mf_f_pdf(b, false, wo, wi, pdf);
+        case MAT_GLASS_ROUGH: return mf_f_pdf(b, wo.y * wi.y < 0, wo, wi, pdf);
         case MAT_PLASTIC_GGX:
         case MAT_PLASTIC_BECKMANN: return fb_f_pdf(b, wo, wi, pdf);
         case MAT_ORENNAYAR: pdf = over_pi(fmaxf(0.f, wi.y)); return on_f(b, wo, wi);
@@ -405,7 +363,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
             return b.R;  // FresnelNoOp
         }
         case MAT_GLASS_SMOOTH: {  // SpecularFresnel (SpecularFresnel.cpp:28-46)
-            float fr = fresnel_dielectric(b.etaA, b.etaB, wo.y);
+            float fr = fresnel_dielectric(b, wo.y);
             if (u.x < fr) {
                 stype = BXDF_REFLECTION | BXDF_SPECULAR;
                 wi = f3(-wo.x, wo.y, -wo.z);
@@ -413,7 +371,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
                 return fr * b.R;
             }
             stype = BXDF_TRANSMISSION | BXDF_SPECULAR;
-            refract(wo, f3(0.f, 1.f, 0.f), b.etaA / b.etaB, wi);
+            refract(wo, f3(0.f, 1.f, 0.f), b.eta_ab, wi);
             pdf = 1.f - fr;
             return (1.f - fr) * b.R;
         }
@@ -422,34 +380,20 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
             float3 wh = ndf_sample(b, u);
             if (dot(wo, wh) <= 0) return zero;
             wi = reflect(-wo, wh);
-            pdf = mf_refl_pdf(b, wo, wi);
-            wi = clamp1(wi);
-            return mf_refl_f(b, wo, wi);
+            return mf_sampled(b, false, wo, wi, pdf);
         }
         case MAT_GLASS_ROUGH: {  // MicrofacetBlend (Microfacet.cpp:164-199)
             float3 wh = ndf_sample(b, u);
             if (dot(wo, wh) <= 0) return zero;
-            float fr = fresnel_dielectric(b.etaA, b.etaB, dot(wo, wh));
-            if (u.x < fr) {
-                stype = BXDF_REFLECTION | BXDF_GLOSSY;
-                wi = reflect(-wo, wh);
-                pdf = bxdf_pdf(b, wo, wi) * fr;
-                wi = clamp1(wi);
-                return mf_refl_f(b, wo, wi);
-            }
+            float fr = fresnel_dielectric(b, dot(wo, wh));
+            const bool refl = u.x < fr;
             float3 t;
-            if (refract(wo, wh, b.etaA / b.etaB, t)) {
-                stype = BXDF_TRANSMISSION | BXDF_GLOSSY;
-                wi = t;
-                pdf = bxdf_pdf(b, wo, wi) * (1 - fr);
-                wi = clamp1(wi);
-                return mf_trans_f(b, wo, wi);
-            }
-            stype = BXDF_REFLECTION | BXDF_GLOSSY;
-            wi = reflect(-wo, wh);
-            pdf = bxdf_pdf(b, wo, wi) * (1 - fr);
-            wi = clamp1(wi);
-            return mf_refl_f(b, wo, wi);
+            const bool trans = !refl && refract(wo, wh, b.eta_ab, t);  // else total reflection
+            stype = (trans ? BXDF_TRANSMISSION : BXDF_REFLECTION) | BXDF_GLOSSY;
+            wi = trans ? t : reflect(-wo, wh);
+            const float3 f = mf_sampled(b, trans, wo, wi, pdf);
+            pdf = pdf * (refl ? fr : 1 - fr);
+            return f;
         }
         case MAT_PLASTIC_GGX:
         case MAT_PLASTIC_BECKMANN: {  // FresnelBlend::SampleDirection
@@ -464,8 +408,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
                 if (L.y * wo.y <= 0) return zero;
                 wi = clamp1(L);
             }
-            pdf = fb_pdf(b, wo, wi);
-            return fb_f(b, wo, wi);
+            return fb_f_pdf(b, wo, wi, pdf);
         }
         case MAT_ORENNAYAR: {
             wi = cosine_hemisphere(u, pdf);
@@ -493,20 +436,17 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
 // ---- BSDF container (BSDF.cpp) --------------------------------------------------------------
 __device__ __forceinline__ bool matches(int bxdf_flags, int flags) { return (bxdf_flags & flags) == bxdf_flags; }
 
-__device__ __forceinline__ float3 bsdf_f(const BxDF& b, const Frame& fr, float3 wo_w, float3 wi_w) {
-    float3 wo = to_local(fr, wo_w), wi = to_local(fr, wi_w);
-    bool refl = wi.y * wo.y > 0;
-    if ((refl && (b.flags & BXDF_REFLECTION)) || (!refl && (b.flags & BXDF_TRANSMISSION))) return bxdf_f(b, wo, wi);
-    return f3(0.f, 0.f, 0.f);
-}
-
-__device__ __forceinline__ float bsdf_pdf(const BxDF& b, const Frame& fr, float3 wo_w, float3 wi_w, int flags) {
-    float3 wo = to_local(fr, wo_w), wi = to_local(fr, wi_w);
-    bool refl = wi.y * wo.y > 0;
-    // `Matches(flags) && (reflect && R) || (!reflect && T)` parses as (A && B) || C (BSDF.cpp:39-40)
-    if ((matches(b.flags, flags) && refl && (b.flags & BXDF_REFLECTION)) || (!refl && (b.flags & BXDF_TRANSMISSION)))
-        return bxdf_pdf(b, wo, wi);
-    return 0.f;
+// The terms of f that depend on wo alone, once per vertex; before the calls below.
+__device__ __forceinline__ void bsdf_prepare(BxDF& b, const Frame& fr, float3 wo_w) {
+    const float3 wo = to_local(fr, wo_w);
+    switch (b.mtype) {
+        case MAT_MICRO_GGX:
+        case MAT_MICRO_BECKMANN:
+        case MAT_GLASS_ROUGH: b.term_o = ndf_lambda(b, wo); break;
+        case MAT_PLASTIC_GGX:
+        case MAT_PLASTIC_BECKMANN: b.term_o = fb_power(fmaxf(0.f, wo.y)); break;
+        default: b.term_o = 0.f;
+    }
 }
 
 // BSDF::DistributionFunction and BSDF::Pdf(flags) of one direction pair in one pass.

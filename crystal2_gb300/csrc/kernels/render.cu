@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                 bx.mtype = MT;  // compile-time material: the BxDF switches fold away
                 bx.flags = material_flags(MT);
                 fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
+                bsdf_prepare(bx, fr, wo);
                 do_nee = true;
             }
         }
@@ -979,6 +980,7 @@ __device__ __noinline__ void finish_shade(const DevScene& S, const WaveArgs& a, 
         bx.flags = material_flags(MT);
         Frame fr;
         fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
+        bsdf_prepare(bx, fr, wo);
         // eligible area lights: one unused 1D sample each
         bool eligible = false, area = false;
         if (sub < S.n_lights) {
