@@ -473,8 +473,8 @@ int c2g_trace_rays(c2g_ctx* ctx, int n, const float* o, const float* d, const fl
     if (rc) return rc;
     std::string err;
     size_t n3 = (size_t)n * 12, n1 = (size_t)n * 4;
-    size_t total = 2 * n3 + 4 * n1;
-    char* buf = (char*)ctx->arena->alloc(total, err);
+    size_t total = 2 * n3 + (t ? 5 : 4) * n1;
+    char* buf = (char*)ctx->arena->borrow(total, err);
     if (!buf) return fail(ctx, C2G_ERR_OOM, err);
     float* d_o = (float*)buf;
     float* d_d = (float*)(buf + n3);
@@ -482,11 +482,10 @@ int c2g_trace_rays(c2g_ctx* ctx, int n, const float* o, const float* d, const fl
     float* d_tmax = (float*)(buf + 2 * n3 + n1);
     int* d_ign = (int*)(buf + 2 * n3 + 2 * n1);
     int* d_obj = (int*)(buf + 2 * n3 + 3 * n1);
-    float* d_t = t ? (float*)ctx->arena->alloc(n1, err) : nullptr;
+    float* d_t = t ? (float*)(buf + 2 * n3 + 4 * n1) : nullptr;
     cudaStream_t st = ctx->stream;
     rc = C2G_OK;
     do {
-        if (t && !d_t) { rc = fail(ctx, C2G_ERR_OOM, err); break; }
         if (cudaMemcpyAsync(d_o, o, n3, cudaMemcpyHostToDevice, st) != cudaSuccess ||
             cudaMemcpyAsync(d_d, d, n3, cudaMemcpyHostToDevice, st) != cudaSuccess) { rc = fail(ctx, C2G_ERR_CUDA, "copy failed"); break; }
         if (tmin && cudaMemcpyAsync(d_tmin, tmin, n1, cudaMemcpyHostToDevice, st) != cudaSuccess) { rc = fail(ctx, C2G_ERR_CUDA, "copy failed"); break; }
@@ -502,8 +501,7 @@ int c2g_trace_rays(c2g_ctx* ctx, int n, const float* o, const float* d, const fl
         if (rc) fail(ctx, rc, err);
     } while (0);
     cudaStreamSynchronize(st);
-    ctx->arena->free(buf);
-    if (d_t) ctx->arena->free(d_t);
+    ctx->arena->give_back(buf);
     return rc;
 }
 

@@ -1103,12 +1103,14 @@ int GuideTrainer::eval(DeviceArena& arena, const float* host_xnw, int n, float* 
     if (!params_) { err = "guide network not initialised"; return C2G_ERR_STATE; }
     if (n <= 0) return C2G_OK;
     // the inputs are already records (9 floats each); the buffer holds whole tiles
-    float* din = (float*)arena.alloc(stage_bytes((size_t)n), err);
-    float* dout = (float*)arena.alloc((size_t)n * kGuideOut * 4, err);
-    int* derr = (int*)arena.alloc(16, err);
+    const size_t in_bytes = (stage_bytes((size_t)n) + 255) & ~size_t(255), out_bytes = ((size_t)n * kGuideOut * 4 + 255) & ~size_t(255);
+    char* buf = (char*)arena.borrow(in_bytes + out_bytes + 16, err);
     int rc = C2G_OK;
-    if (!din || !dout || !derr) rc = C2G_ERR_OOM;
+    if (!buf) rc = C2G_ERR_OOM;
     if (!rc) {
+        float* din = (float*)buf;
+        float* dout = (float*)(buf + in_bytes);
+        int* derr = (int*)(buf + in_bytes + out_bytes);
         cudaMemcpy(din, host_xnw, (size_t)n * 9 * 4, cudaMemcpyHostToDevice);
         cudaMemset(derr, 0, 16);
         prepare_launch();
@@ -1122,9 +1124,7 @@ int GuideTrainer::eval(DeviceArena& arena, const float* host_xnw, int n, float* 
             rc = C2G_ERR_DEVICE;
         } else cudaMemcpy(host_out, dout, (size_t)n * kGuideOut * 4, cudaMemcpyDeviceToHost);
     }
-    if (din) arena.free(din);
-    if (dout) arena.free(dout);
-    if (derr) arena.free(derr);
+    arena.give_back(buf);
     return rc;
 }
 
@@ -1133,7 +1133,7 @@ int GuideTrainer::gradient(DeviceArena& arena, const float* host_samples, int n,
     if (n <= 0) { err = "empty batch"; return C2G_ERR_INVALID; }
     // batch (64 bytes per sample), the samples as given, the error word
     const size_t raw = (size_t)n * 14 * 4, packed = (size_t)n * 64;
-    unsigned char* buf = (unsigned char*)arena.alloc(packed + raw + 16, err);
+    unsigned char* buf = (unsigned char*)arena.borrow(packed + raw + 16, err);
     if (!buf) return C2G_ERR_OOM;
     float4* db = (float4*)buf;
     float* ds = (float*)(buf + packed);
@@ -1161,7 +1161,7 @@ int GuideTrainer::gradient(DeviceArena& arena, const float* host_samples, int n,
             if (loss) *loss = wsum > 0 ? (double)ls / wsum : 0.0;
         }
     }
-    arena.free(buf);
+    arena.give_back(buf);
     return rc;
 }
 

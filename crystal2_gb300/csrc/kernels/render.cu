@@ -36,6 +36,11 @@ void* DeviceArena::alloc(size_t bytes, std::string& err) {
     }
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && kept_.p) {
+        cudaGetLastError();
+        drop_kept();
+        e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         err = std::string("cudaMalloc failed: ") + cudaGetErrorString(e);
@@ -58,7 +63,35 @@ void DeviceArena::free(void* p) {
     }
 }
 
+void* DeviceArena::borrow(size_t bytes, std::string& err) {
+    if (kept_.p && kept_.n >= bytes) {
+        blocks_.push_back(kept_);
+        used_ += kept_.n;
+        kept_ = {nullptr, 0};
+        return blocks_.back().p;
+    }
+    drop_kept();
+    return alloc(bytes, err);
+}
+
+void DeviceArena::give_back(void* p) {
+    if (!p) return;
+    if (!cap_ && !kept_.p && !blocks_.empty() && blocks_.back().p == p && blocks_.back().n <= kKeptBytes) {
+        kept_ = blocks_.back();
+        used_ -= kept_.n;
+        blocks_.pop_back();
+        return;
+    }
+    free(p);
+}
+
+void DeviceArena::drop_kept() {
+    if (kept_.p) cudaFree(kept_.p);
+    kept_ = {nullptr, 0};
+}
+
 void DeviceArena::free_all() {
+    drop_kept();
     for (auto& b : blocks_) cudaFree(b.p);
     blocks_.clear();
     used_ = 0;
@@ -2314,9 +2347,9 @@ int GpuScene::halton(int width, int height, int n, const int* px, const int* py,
     if (n <= 0 || ndim <= 0) return C2G_OK;
     HaltonParams hp = halton_params(width, height);
     size_t bytes_i = (size_t)n * 4, bytes_o = (size_t)n * ndim * 4;
-    int* dpx = (int*)arena.alloc(bytes_i * 3, err);
-    float* dout = (float*)arena.alloc(bytes_o, err);
-    if (!dpx || !dout) { arena.free(dpx); arena.free(dout); return C2G_ERR_OOM; }
+    int* dpx = (int*)arena.borrow(bytes_i * 3 + bytes_o, err);
+    if (!dpx) return C2G_ERR_OOM;
+    float* dout = (float*)(dpx + 3 * (size_t)n);
     int rc = C2G_OK;
     do {
         if (cudaMemcpy(dpx, px, bytes_i, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2326,8 +2359,7 @@ int GpuScene::halton(int width, int height, int n, const int* px, const int* py,
         if (cudaGetLastError() != cudaSuccess || cudaMemcpy(out, dout, bytes_o, cudaMemcpyDeviceToHost) != cudaSuccess) rc = C2G_ERR_CUDA;
     } while (0);
     if (rc) err = "halton query failed";
-    arena.free(dpx);
-    arena.free(dout);
+    arena.give_back(dpx);
     return rc;
 }
 
@@ -2336,9 +2368,9 @@ int GpuScene::sampler_values(int width, int n, const int* px, const int* py, con
     if (!sb_->S.perm) { err = "no scene loaded"; return C2G_ERR_STATE; }
     if (n <= 0) return C2G_OK;
     size_t bytes_i = (size_t)n * 4, bytes_o = (size_t)n * (two_d ? 2 : 1) * 4;
-    int* dpx = (int*)arena.alloc(bytes_i * 3, err);
-    float* dout = (float*)arena.alloc(bytes_o, err);
-    if (!dpx || !dout) { arena.free(dpx); arena.free(dout); return C2G_ERR_OOM; }
+    int* dpx = (int*)arena.borrow(bytes_i * 3 + bytes_o, err);
+    if (!dpx) return C2G_ERR_OOM;
+    float* dout = (float*)(dpx + 3 * (size_t)n);
     int rc = C2G_OK;
     do {
         if (cudaMemcpy(dpx, px, bytes_i, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2348,15 +2380,14 @@ int GpuScene::sampler_values(int width, int n, const int* px, const int* py, con
         if (cudaGetLastError() != cudaSuccess || cudaMemcpy(out, dout, bytes_o, cudaMemcpyDeviceToHost) != cudaSuccess) rc = C2G_ERR_CUDA;
     } while (0);
     if (rc) err = "sampler query failed";
-    arena.free(dpx);
-    arena.free(dout);
+    arena.give_back(dpx);
     return rc;
 }
 
 int GpuScene::camera_rays(int n, const float* pos2, float* o, float* d, DeviceArena& arena, std::string& err) {
     if (!sb_->film) { err = "no scene loaded"; return C2G_ERR_STATE; }
     if (n <= 0) return C2G_OK;
-    float* buf = (float*)arena.alloc((size_t)n * 8 * 4, err);
+    float* buf = (float*)arena.borrow((size_t)n * 8 * 4, err);
     if (!buf) return C2G_ERR_OOM;
     int rc = C2G_OK;
     if (cudaMemcpy(buf, pos2, (size_t)n * 8, cudaMemcpyHostToDevice) != cudaSuccess) rc = C2G_ERR_CUDA;
@@ -2367,7 +2398,7 @@ int GpuScene::camera_rays(int n, const float* pos2, float* o, float* d, DeviceAr
             rc = C2G_ERR_CUDA;
     }
     if (rc) err = "camera query failed";
-    arena.free(buf);
+    arena.give_back(buf);
     return rc;
 }
 
