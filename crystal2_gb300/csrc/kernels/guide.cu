@@ -31,7 +31,7 @@ __device__ __forceinline__ float luminance(float3 c) { return 0.2126f * c.x + 0.
 // records of consecutive work items back to back.  k_guide_mlp_tc streams 128-record tiles into
 // shared memory with the bulk-copy engine; every thread frequency-encodes its own row into the
 // BF16 operand tile, already in the tensor core's shared-memory layout, and the warpgroup runs the
-// four layers: two warpgroups per CTA share the staged weights; per warpgroup and tile one thread
+// four layers: five warpgroups per CTA share the staged weights; per warpgroup and tile one thread
 // issues K/16 tcgen05.mma (M = 128, N = 64 or 48, K = 80 with the bias folded in below, BF16
 // operands from shared-memory descriptors, FP32 accumulator in 64 tensor-memory columns) and
 // commits them to an mbarrier; every thread then reads its row (tcgen05.ld), applies ReLU and
@@ -42,7 +42,11 @@ __device__ __forceinline__ float luminance(float3 c) { return 0.2126f * c.x + 0.
 // K-column operand sits at (r / 8) * 16K + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2 bytes, so one
 // K=16 step spans two core matrices 128 B apart (descriptor LBO), 8-row groups 16K bytes apart (SBO).
 constexpr int kTcRows = 128;
-constexpr int kTcGroups = 2;                            // warpgroups per CTA
+// Warpgroups per CTA, one CTA an SM: a tile is a chain of encoding, four MMAs and their epilogues, so warps
+// in flight bound the kernel.  Five share one copy of the weights in 164 KB and have 96 registers each
+// without spills: 0.99 -> 0.92 ms for the guided slit frame, against two CTAs of two; six and seven
+// (80 and 72 registers, spills) take 0.95 and 0.94.
+constexpr int kTcGroups = 5;
 constexpr int kTcThreads = kTcRows * kTcGroups;
 constexpr int kTcRecFloats = 9;                         // network input record: x, n, wo
 constexpr int kTcRecBytes = kTcRows * kTcRecFloats * 4;   // one tile of records: 4608 B
@@ -68,8 +72,9 @@ constexpr int kTcBar = tc_wi_off(4) + kTcGroups * kTcGroupBytes;  // per warpgro
 constexpr int kTcTmemSlot = kTcBar + 16 * kTcGroups;
 constexpr size_t kTcSmem = (size_t)kTcTmemSlot + 8;
 constexpr uint32_t kTcColsPerGroup = 64;
-constexpr uint32_t kTcCols = kTcColsPerGroup * kTcGroups;  // tensor-memory columns per CTA (power of 2)
+constexpr uint32_t kTcCols = 512;  // tensor-memory columns per CTA: a power of 2, and the CTA is alone on its SM
 constexpr uint32_t kTcWaitPolls = 1u << 22;
+static_assert(kTcGroups * kTcColsPerGroup <= kTcCols && 2 * kTcSmem > (227u << 10), "one CTA holds the tensor memory");
 static_assert(tc_in(0) % 128 == 0 && tc_rec(0) % 16 == 0 && kTcGroupBytes % 128 == 0 && kTcBar % 8 == 0,
               "operand, bulk-copy and barrier alignment");
 static_assert(kTcRecBytes % 16 == 0 && (32 * kTcRecFloats * 4) % 16 == 0, "record tiles and warp chunks are 16-byte multiples");
@@ -177,7 +182,7 @@ __global__ void __launch_bounds__(256) k_guide_record(DevScene S, const float4* 
 // are not read).  MODE 0: the guided buckets' vertices, packed mixtures per work item (field-major,
 // out_stride float4 per field); MODE 1: n_in explicit inputs, raw outputs (kGuideOut floats each).
 template <int MODE>
-__global__ void __launch_bounds__(kTcThreads, 2) k_guide_mlp_tc(GuideNet net, const unsigned char* __restrict__ stage,
+__global__ void __launch_bounds__(kTcThreads, 1) k_guide_mlp_tc(GuideNet net, const unsigned char* __restrict__ stage,
                                                                const int* bucket_cnt, int mask, int n_in, float* out,
                                                                int out_stride, int* err) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1014,7 +1019,7 @@ void GuideTrainer::prepare_launch() {
     int smem_sm = 0;
     cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     const int per_smem = smem_sm / (int)(kTcSmem + 1024);
-    per = std::max(per, std::min(2, per_smem));
+    per = std::max(per, std::min(1, per_smem));
     g_infer_grid = std::max(1, sms * std::max(1, per));
     g_train_grid = std::max(1, sms);
     int per_enc = 0;
