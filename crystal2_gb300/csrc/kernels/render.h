@@ -171,6 +171,12 @@ private:
     // Third stream of a wave: the next bounce level's extension starts on it as soon as this level's
     // shading has filled the next queue, beside this level's shadow and MIS rays and accumulation.
     cudaStream_t ahead_ = nullptr;
+    // More streams for the shading of scenes of more than three material buckets: a level of few paths is
+    // the latency of its bucket kernels one after another.
+    static constexpr int kMore = 4;
+    cudaStream_t more_[kMore] = {};
+    cudaEvent_t more_join_[kMore] = {};
+    int more_n_ = 0;             // of them there
     cudaEvent_t fork_ev_[4] = {nullptr, nullptr, nullptr, nullptr}, join_ev_[4] = {nullptr, nullptr, nullptr, nullptr};
     // Paths entering each bounce level, written by the look-ahead extension (page-locked host memory and
     // its device address): the host stops enqueuing levels when a queue is empty or small.
