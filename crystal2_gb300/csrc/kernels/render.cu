@@ -288,7 +288,7 @@ __global__ void k_raygen(DevScene S, WaveArgs a, PathRefs out, float4* out_L, in
     }
 }
 
-// Minimum resident 256-thread blocks per SM of the persistent traversal kernels: a budget of 64
+// Minimum resident 256-thread blocks per SM of the persistent traversal kernels: a cap of 64
 // registers per thread.  The traversal waits on dependent node loads, so more resident warps hide more
 // of that latency, until spills to local memory cost more: 1080p many-material step 45.5 ms at four
 // blocks, 49.5 at five (48 registers, spills), 50.4 at three.
