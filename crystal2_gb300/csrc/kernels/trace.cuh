@@ -31,15 +31,14 @@ __device__ __forceinline__ RayQ make_rayq(float3 o, float3 d) {
     return r;
 }
 
-// Ray of the four-wide traversal with quantised planes: iv is the reciprocal direction clamped to a
-// finite value, m the amount by which its slab distances are widened (see node4_slabs).
-constexpr float kInvMax = 0x1p100f;
+// Ray of the four-wide traversal with quantised planes: iv is the reciprocal direction clamped to
+// +-S.inv_max, m the amount by which its slab distances are widened (see node4_slabs).
 constexpr float kSlabMargin = 20.f * 0x1p-24f;
 struct Ray4 {
     float3 o, d, iv, m;
 };
 
-__device__ __forceinline__ float inv_clamped(float d) { return fminf(fmaxf(__frcp_rn(d), -kInvMax), kInvMax); }
+__device__ __forceinline__ float inv_clamped(const DevScene& S, float d) { return fminf(fmaxf(__frcp_rn(d), -S.inv_max), S.inv_max); }
 
 // R: Ray4 (quantised planes) or RayQ (exact planes)
 template <class R>
@@ -51,7 +50,7 @@ __device__ __forceinline__ Ray4 make_ray<Ray4>(const DevScene& S, float3 o, floa
     Ray4 r;
     r.o = o;
     r.d = d;
-    r.iv = f3(inv_clamped(d.x), inv_clamped(d.y), inv_clamped(d.z));
+    r.iv = f3(inv_clamped(S, d.x), inv_clamped(S, d.y), inv_clamped(S, d.z));
     r.m = f3((S.extent[0] + fabsf(o.x)) * kSlabMargin * fabsf(r.iv.x), (S.extent[1] + fabsf(o.y)) * kSlabMargin * fabsf(r.iv.y),
              (S.extent[2] + fabsf(o.z)) * kSlabMargin * fabsf(r.iv.z));
     return r;
@@ -66,15 +65,15 @@ template <> struct QueueTuning<RayQ> { static constexpr int kWalkers = 0, kLeave
 __device__ __forceinline__ constexpr bool loose_boxes(const RayQ&) { return false; }
 __device__ __forceinline__ constexpr bool loose_boxes(const Ray4&) { return true; }
 // The exact ray of the primitive tests.
-__device__ __forceinline__ const RayQ& exact_ray(const RayQ& r) { return r; }
-__device__ __forceinline__ RayQ exact_ray(const Ray4& r) {
+__device__ __forceinline__ const RayQ& exact_ray(const DevScene&, const RayQ& r) { return r; }
+__device__ __forceinline__ RayQ exact_ray(const DevScene& S, const Ray4& r) {
     RayQ q;
     q.o = r.o;
     q.d = r.d;
     q.inv = r.iv;
-    if (fabsf(r.iv.x) == kInvMax) q.inv.x = __frcp_rn(r.d.x);
-    if (fabsf(r.iv.y) == kInvMax) q.inv.y = __frcp_rn(r.d.y);
-    if (fabsf(r.iv.z) == kInvMax) q.inv.z = __frcp_rn(r.d.z);
+    if (fabsf(r.iv.x) == S.inv_max) q.inv.x = __frcp_rn(r.d.x);
+    if (fabsf(r.iv.y) == S.inv_max) q.inv.y = __frcp_rn(r.d.y);
+    if (fabsf(r.iv.z) == S.inv_max) q.inv.z = __frcp_rn(r.d.z);
     q.neg[0] = q.inv.x < 0.f;
     q.neg[1] = q.inv.y < 0.f;
     q.neg[2] = q.inv.z < 0.f;
@@ -231,7 +230,7 @@ __device__ __forceinline__ bool leaf_box_hit(const DevScene& S, int first, int c
 #pragma unroll
         for (int k = 0; k < 3; k++) { mn[k] = fminf(mn[k], lo[k]); mx[k] = fmaxf(mx[k], hi[k]); }
     }
-    return box_test(exact_ray(r), mn, mx, t0, t1);
+    return box_test(exact_ray(S, r), mn, mx, t0, t1);
 }
 
 // Closest-hit test of one prim (the leaf body of BVH::Intersect, BVH.cpp:73-90).
@@ -245,7 +244,7 @@ __device__ __forceinline__ void closest_prim(const DevScene& S, int pi, const R&
         float mn[3], mx[3];
         prim_box(a, b, c, type, mn, mx);
         float t0 = 0.f, t1 = smin(tmax, h.t);
-        if (!box_test(exact_ray(r), mn, mx, t0, t1)) return;
+        if (!box_test(exact_ray(S, r), mn, mx, t0, t1)) return;
     }
     float dis;
     float u = 0.f, v = 0.f;
@@ -280,7 +279,7 @@ __device__ __forceinline__ bool anyhit_prim(const DevScene& S, int pi, const R& 
     if (S.anyhit_clip) {
         float mn[3], mx[3];
         prim_box(a, b, c, type, mn, mx);
-        if (!box_test(exact_ray(r), mn, mx, t0, t1)) return false;
+        if (!box_test(exact_ray(S, r), mn, mx, t0, t1)) return false;
     }
     if (type == SHAPE_TRI) {
         if (t0 > t1) return false;
@@ -517,8 +516,11 @@ __device__ __forceinline__ bool trace_any_sah(const DevScene& S, const RayQ& r, 
 // the largest coordinate of the scene on the axis, |scale| <= 1.35 E and v < 2, the roundings of t
 // (product, org - o, offset, final FMA) come to at most u (7.1 E + 3 |o|) |iv|, those of the exact
 // test to 2 u (E + |o|) |iv|, and a plane may lie inside its box by 2^-21 E = 8 u E (quantise_axis):
-// together below m = 20 u (E + |o|) |iv|.  iv is finite (a zero direction component gives 2^100): the
-// slab of a parallel axis then accepts exactly when the origin lies within it, up to the margin.
+// together below m = 20 u (E + |o|) |iv|.  A zero direction component gives iv = S.inv_max: the slab of a
+// parallel axis then accepts exactly when the origin lies within it, up to the margin.  S.inv_max is
+// 2^100, and less in scenes beyond 2^20 units, so that scale * iv and the offset of an origin among the
+// scene's coordinates stay finite (at 2^100 the product overflowed from 4e8 units on, and a near plane at
+// infinity hid the whole node).
 constexpr int kStack4 = 128;
 
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {

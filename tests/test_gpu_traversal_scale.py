@@ -1,0 +1,76 @@
+"""Four-wide traversal with quantised planes in scenes and along rays of extreme scale, against the binary SAH
+traversal: the same bits of every closest hit's distance, the same any-hit answers.
+
+The scene is a soup of small triangles in the unit cube (over a thousand nodes) and one triangle far away, so
+that the nodes near the root span the distance and the others do not."""
+import os
+
+import numpy as np
+import pytest
+
+from crystal2_gb300 import Context, scenes
+from crystal2_gb300 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+TRIS = 4096
+
+
+def _soup(d, far, spp=1, size=64):
+    tris = scenes.tri_soup_arrays(TRIS, 3).astype(np.float64)
+    tris = tris + (tris - tris.mean(axis=1, keepdims=True)) * 4  # edges of some 0.03
+    if far:
+        tris = np.concatenate([tris, (np.float64([[0, 0, 0], [1, 0, 0], [0, 1, 0]]) * 0.1 + 1.0)[None] * far])
+    tris = tris.astype(np.float32)
+    n = np.cross((tris[:, 1] - tris[:, 0]).astype(np.float64), (tris[:, 2] - tris[:, 0]).astype(np.float64))
+    n /= np.linalg.norm(n, axis=1, keepdims=True)
+    path = os.path.join(d, "soup.obj")
+    scenes.write_obj(path, tris.reshape(-1, 3), n.astype(np.float32), np.arange(3 * len(tris)).reshape(-1, 3),
+                     np.repeat(np.arange(len(tris))[:, None], 3, axis=1))
+    cfg = scenes.config_json(size, size, spp, 4)
+    return scenes.write_scene(d, cfg, scenes.camera((0.5, 0.5, -1.5), (0.5, 0.5, 0.5), 45), [scenes.mesh(path, scenes.diffuse((0.5, 0.5, 0.5)))], "soup"), tris
+
+
+def _axis_rays(tris, seed, zero):
+    """Axis-parallel rays at the soup's triangles; the other components are `zero`."""
+    rng = np.random.default_rng(seed)
+    c = tris[:TRIS].mean(axis=1)
+    k = rng.integers(0, 3, TRIS)
+    s = rng.choice([-1.0, 1.0], TRIS)
+    d = np.full((TRIS, 3), zero, np.float32)
+    d[np.arange(TRIS), k] = s
+    o = c.copy()
+    o[np.arange(TRIS), k] -= np.float32(1.5) * s.astype(np.float32)
+    return o.astype(np.float32), d
+
+
+def _free_rays(seed, n=4096):
+    rng = np.random.default_rng(seed)
+    d = rng.normal(size=(n, 3))
+    return rng.random((n, 3)).astype(np.float32), (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+
+
+def _compare(ctx, o, d, tmax):
+    got = {}
+    for width in (2, 4):
+        ctx.set_traversal(width)
+        got[width] = ctx.trace_rays(o, d) + (ctx.trace_rays(o, d, any_hit=True, tmax=tmax),)
+    (obj2, t2, any2), (obj4, t4, any4) = got[2], got[4]
+    assert np.array_equal(t2.view(np.uint32), t4.view(np.uint32))
+    assert np.array_equal(any2, any4)
+    return obj2, any2
+
+
+# scale * 2^100 is infinite from 4.0e8 units on, the offset from 8e8
+@pytest.mark.parametrize("far", [0, 1e2, 1e6, 3e8, 4.1e8, 7e8, 9e8, 1e10, 1e18])
+def test_axis_parallel_rays_with_a_far_triangle(tmp_path, far):
+    (cp, sp), tris = _soup(str(tmp_path), far)
+    with Context(0) as ctx:
+        ctx.load(cp, sp, tree=N.TREE_SAH)
+        for zero in (0.0, -0.0):
+            o, d = _axis_rays(tris, 5, zero)
+            obj, occluded = _compare(ctx, o, d, np.full(len(o), 1.5, np.float32))
+            assert np.mean(obj >= 0) > 0.9 and np.mean(occluded) > 0.3
+        o, d = _free_rays(7)
+        obj, _ = _compare(ctx, o, d, np.full(len(o), 0.5, np.float32))
+        assert np.mean(obj >= 0) > 0.2
