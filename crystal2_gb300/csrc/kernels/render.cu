@@ -1605,9 +1605,9 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
         for (int k = 0; k < 3; k++) { box_lo_[k] = std::min(box_lo_[k], b[k]); box_hi_[k] = std::max(box_hi_[k], b[3 + k]); }
     }
     for (int k = 0; k < 3; k++) S.extent[k] = std::max(std::fabs(box_lo_[k]), std::fabs(box_hi_[k]));
+    S.reach = std::max({S.extent[0], S.extent[1], S.extent[2]});
     // scale <= 1.35 reach and an offset of at most 2.7 reach keep their products below 2^122
-    const float reach = std::max({S.extent[0], S.extent[1], S.extent[2], 1.f});
-    S.inv_max = std::min(0x1p100f, 0x1p120f / reach);
+    S.inv_max = 0x1p120f / std::max(S.reach, 1.f);
     guide_steps_ = 0;
     wave_counter_ = nullptr;  // freed with the previous scene's buffers
     guide_.release(arena);  // a new scene trains a new network

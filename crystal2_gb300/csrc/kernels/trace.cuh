@@ -53,6 +53,13 @@ __device__ __forceinline__ Ray4 make_ray<Ray4>(const DevScene& S, float3 o, floa
     r.iv = f3(inv_clamped(S, d.x), inv_clamped(S, d.y), inv_clamped(S, d.z));
     r.m = f3((S.extent[0] + fabsf(o.x)) * kSlabMargin * fabsf(r.iv.x), (S.extent[1] + fabsf(o.y)) * kSlabMargin * fabsf(r.iv.y),
              (S.extent[2] + fabsf(o.z)) * kSlabMargin * fabsf(r.iv.z));
+    // clamped components: no distance at which the ray can meet the scene may lie outside their slabs
+    const float longest = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+    const float far = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), S.reach));
+    const float whole = longest > 0.f ? 8.f * far * __frcp_rn(longest) : 0.f;
+    if (fabsf(r.iv.x) == S.inv_max) r.m.x += whole;
+    if (fabsf(r.iv.y) == S.inv_max) r.m.y += whole;
+    if (fabsf(r.iv.z) == S.inv_max) r.m.z += whole;
     return r;
 }
 
@@ -516,11 +523,14 @@ __device__ __forceinline__ bool trace_any_sah(const DevScene& S, const RayQ& r, 
 // the largest coordinate of the scene on the axis, |scale| <= 1.35 E and v < 2, the roundings of t
 // (product, org - o, offset, final FMA) come to at most u (7.1 E + 3 |o|) |iv|, those of the exact
 // test to 2 u (E + |o|) |iv|, and a plane may lie inside its box by 2^-21 E = 8 u E (quantise_axis):
-// together below m = 20 u (E + |o|) |iv|.  A zero direction component gives iv = S.inv_max: the slab of a
-// parallel axis then accepts exactly when the origin lies within it, up to the margin.  S.inv_max is
-// 2^100, and less in scenes beyond 2^20 units, so that scale * iv and the offset of an origin among the
-// scene's coordinates stay finite (at 2^100 the product overflowed from 4e8 units on, and a near plane at
-// infinity hid the whole node).
+// together below m = 20 u (E + |o|) |iv|.  A direction component that is zero, or so small that the
+// ray crosses the whole scene without moving along the axis, gives iv = S.inv_max, and m then adds the
+// largest distance at which the ray can meet the scene: the slab accepts when the origin lies within it, up
+// to 2^-116 reach^2 for unit directions, whatever the length of the direction.  (Without this term
+// directions of 1e-28 and shorter, whose hits lie beyond 2^100 times their slab, lost them.)  S.inv_max is
+// 2^120 over the scene's reach, so that scale * iv and the offset of an origin among the scene's
+// coordinates stay finite (with 2^100 for every scene the product overflowed from 4e8 units on, and a near
+// plane at infinity hid the whole node).
 constexpr int kStack4 = 128;
 
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {

@@ -74,3 +74,19 @@ def test_axis_parallel_rays_with_a_far_triangle(tmp_path, far):
         o, d = _free_rays(7)
         obj, _ = _compare(ctx, o, d, np.full(len(o), 0.5, np.float32))
         assert np.mean(obj >= 0) > 0.2
+
+
+# a hit's distance is 1.5 / |d|, up to 2^125 here, against a slab distance of 2^100 or more along the other axes
+@pytest.mark.parametrize("far", [0, 1e6])
+@pytest.mark.parametrize("length", [-125, -115, -105, -98, -96, -90, -60, 40, 100])
+def test_directions_of_any_length(tmp_path, length, far):
+    (cp, sp), tris = _soup(str(tmp_path), far)
+    with Context(0) as ctx:
+        ctx.load(cp, sp, tree=N.TREE_SAH)
+        for (o, d), hit in ((_axis_rays(tris, 5, 0.0), 0.5), (_free_rays(7), 0.1)):
+            obj, _ = _compare(ctx, o, np.ldexp(d, length), np.ldexp(np.full(len(o), 1.5, np.float32), -length))
+            assert length < -100 or np.mean(obj >= 0) > hit  # below, the primitives' own determinants are denormal
+        # one component far shorter than the others
+        o, d = _free_rays(8)
+        d[np.arange(len(d)), np.arange(len(d)) % 3] *= np.float32(2.0 ** -length if length > 0 else 2.0 ** length)
+        _compare(ctx, o, d, np.full(len(o), 0.5, np.float32))
