@@ -334,8 +334,9 @@ inline int plane_byte(double v) {
 
 // One axis of a Node4: org, scale and the plane bytes of the used children.  Byte 0 stands for the
 // node's lowest plane and byte 255 for its highest, so the outermost planes (flat walls and floors
-// among them) stay exact to float rounding; planes between are rounded outwards.  `tol` (2^-22 of the
-// coordinates) absorbs the rounding of org and scale; the traversal's margin covers it.  An axis
+// among them) stay exact to float rounding; planes between are rounded outwards.  `tol` is what the
+// rounding of org and scale moves the outermost planes by, at most 2^-24 (|org| + 1.5 scale): a plane at the
+// end of the node keeps byte 0 or 255, and the traversal's margin covers it.  An axis
 // with a non-finite plane gets a NaN org: its slab distances are NaN, which the slab test ignores.
 void quantise_axis(const Slot* c, const int* child, int k, float& org, float& scale, uint32_t& qlo, uint32_t& qhi) {
     double lo = std::numeric_limits<double>::infinity(), hi = -lo;
@@ -349,8 +350,8 @@ void quantise_axis(const Slot* c, const int* child, int k, float& org, float& sc
         scale = 0.f;
         return;
     }
-    const double tol = std::ldexp(std::max({std::fabs(lo), std::fabs(hi), hi - lo}), -22);
     auto plane = [&](int q) { return (double)org + (double)scale * plane_value(q); };
+    const double tol = std::max(std::fabs(plane(0) - lo), std::fabs(plane(255) - hi));
     for (int i = 0; i < 4; i++) {
         int l = 255, h = 0;  // empty slot: an inverted box
         if (child[i] != INT_MIN) {
@@ -419,6 +420,21 @@ void collapse_bvh4(SahTree& t) {
     t.nodes4x.clear();
     emit4(t.nodes, 0, t.nodes4, t.nodes4x);
     if (t.nodes4.size() > kExactNodes) t.nodes4x.clear();
+}
+
+bool has_narrow_leaves(const SahTree& t, float width) {
+    size_t leaves = 0, narrow = 0;
+    auto add = [&](const float* lo, const float* hi) {
+        float side = 0.f;
+        for (int k = 0; k < 3; k++) side = std::max(side, hi[k] - lo[k]);
+        leaves++;
+        narrow += side < width;
+    };
+    for (const WideNode& n : t.nodes) {
+        if (n.n0 > 0) add(n.lo0, n.hi0);
+        if (n.n1 > 0) add(n.lo1, n.hi1);
+    }
+    return narrow * 16 > leaves;
 }
 
 void make_prims(const HostScene& s, const std::vector<int>& order, std::vector<Prim>& prims) {

@@ -25,8 +25,9 @@ struct DevScene {
     const WideNode* wide_nodes;   // tree == SAH: root 0
     const Node4* nodes4;          // tree == SAH: the same tree four-wide, root 0
     const Node4x* nodes4x;        // those nodes with exact planes, or null (SahTree::nodes4x)
-    float extent[3];              // largest absolute coordinate of the scene box per axis (slab margin of Node4)
+    float extent[3];              // largest finite absolute coordinate of the objects' boxes per axis (slab margin of Node4)
     float reach;                  // largest of them
+    int near_margin;              // 1: leaves are small against the reach (Ray4n)
     float inv_max;                // largest reciprocal direction component of the Node4 slabs
     int sah_width;                // SAH traversal variant: 2 (WideNode) or 4 (Node4)
     int anyhit_clip;              // 1: BVH semantics (object-box-clipped shadow interval)

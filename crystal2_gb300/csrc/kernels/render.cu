@@ -1598,16 +1598,18 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
     C2G_CUDA(cudaMemset(sb_->film, 0, npx * sizeof(float4)));
     C2G_CUDA(cudaMemset(sb_->film_m2, 0, npx * sizeof(float4)));
     sb_->n_lights = S.n_lights;
-    for (int k = 0; k < 3; k++) { box_lo_[k] = INFINITY; box_hi_[k] = -INFINITY; }
+    for (int k = 0; k < 3; k++) { box_lo_[k] = INFINITY; box_hi_[k] = -INFINITY; S.extent[k] = 0.f; }
     for (size_t o = 0; o < s.objs.size(); o++) {
         float b[6];
         s.object_box((int)o, b);
         for (int k = 0; k < 3; k++) { box_lo_[k] = std::min(box_lo_[k], b[k]); box_hi_[k] = std::max(box_hi_[k], b[3 + k]); }
+        for (int k = 0; k < 6; k++)
+            if (std::isfinite(b[k])) S.extent[k % 3] = std::max(S.extent[k % 3], std::fabs(b[k]));
     }
-    for (int k = 0; k < 3; k++) S.extent[k] = std::max(std::fabs(box_lo_[k]), std::fabs(box_hi_[k]));
     S.reach = std::max({S.extent[0], S.extent[1], S.extent[2]});
     // scale <= 1.35 reach and an offset of at most 2.7 reach keep their products below 2^122
     S.inv_max = 0x1p120f / std::max(S.reach, 1.f);
+    S.near_margin = sah && has_narrow_leaves(*sah, std::ldexp(S.reach, -14));
     guide_steps_ = 0;
     wave_counter_ = nullptr;  // freed with the previous scene's buffers
     guide_.release(arena);  // a new scene trains a new network
@@ -1672,14 +1674,26 @@ namespace {
 // paths and 1.35 ms without).  Measured limits: 640 x 360 many-material step 1.99 ms without, 1.50 at
 // 4096 paths, 1.44 at 8192, 1.43 at 16384; the 1080p step 44.07, 44.03, 44.08, 44.97.
 constexpr int kFinishPaths = 8192, kFinishMaterials = 5;
-int g_raygen = 0, g_shade = 0, g_acc = 0, g_film = 0, g_finish[2] = {0, 0};
 // Traversal kernels: one ray per thread (reference tree, binary nodes), four-wide nodes with quantised
-// or with exact planes.
-enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_KINDS = 3 };
+// planes (margin of the whole scene, or of each node) or with exact ones.
+enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_NEAR4 = 3, TRACE_KINDS = 4 };
 int trace_kind(const DevScene& S) {
     if (S.tree != C2G_TREE_SAH || S.sah_width != 4) return TRACE_PLAIN;
-    return S.nodes4x ? TRACE_EXACT4 : TRACE_QUANT4;
+    return S.nodes4x ? TRACE_EXACT4 : S.near_margin ? TRACE_NEAR4 : TRACE_QUANT4;
 }
+// Calls f with the ray type of a four-wide kind.
+template <class R>
+struct RayTag {
+    using type = R;
+};
+template <class F>
+void by_ray(int kind, F f) {
+    if (kind == TRACE_QUANT4) f(RayTag<Ray4>{});
+    else if (kind == TRACE_NEAR4) f(RayTag<Ray4n>{});
+    else f(RayTag<RayQ>{});
+}
+#define C2G_RAY(tag) typename decltype(tag)::type
+int g_raygen = 0, g_shade = 0, g_acc = 0, g_film = 0, g_finish[TRACE_KINDS] = {};
 // Persistent grids of the traversal kernels for one block size (64, 128 or 256 threads), per kind and
 // without / with counters.
 struct TraceGrids {
@@ -1693,21 +1707,22 @@ void ensure_grids() {
     g_shade = grid_for((const void*)k_shade<MAT_DIFFUSE, false>, 128);
     g_acc = grid_for((const void*)k_accumulate, 256);
     g_film = grid_for((const void*)k_film, 256);
-    g_finish[0] = grid_for((const void*)k_finish<Ray4>, 128);
-    g_finish[1] = grid_for((const void*)k_finish<RayQ>, 128);
+    for (int k = 1; k < TRACE_KINDS; k++)
+        by_ray(k, [&](auto tag) { g_finish[k] = grid_for((const void*)k_finish<C2G_RAY(tag)>, 128); });
     for (int i = 0; i < 3; i++) {
         const int tb = 64 << i;
         TraceGrids& g = g_trace[i];
         for (int c = 0; c < 2; c++) {
             g.ext[0][c] = grid_for(c ? (const void*)k_extend<true> : (const void*)k_extend<false>, tb);
-            g.ext[1][c] = grid_for(c ? (const void*)k_extend_fetch<true, Ray4> : (const void*)k_extend_fetch<false, Ray4>, tb);
-            g.ext[2][c] = grid_for(c ? (const void*)k_extend_fetch<true, RayQ> : (const void*)k_extend_fetch<false, RayQ>, tb);
             g.sh[0][c] = grid_for(c ? (const void*)k_shadow<true> : (const void*)k_shadow<false>, tb);
-            g.sh[1][c] = grid_for(c ? (const void*)k_shadow_fetch<true, Ray4> : (const void*)k_shadow_fetch<false, Ray4>, tb);
-            g.sh[2][c] = grid_for(c ? (const void*)k_shadow_fetch<true, RayQ> : (const void*)k_shadow_fetch<false, RayQ>, tb);
             g.mis[0][c] = grid_for(c ? (const void*)k_mis<true> : (const void*)k_mis<false>, tb);
-            g.mis[1][c] = grid_for(c ? (const void*)k_mis_fetch<true, Ray4> : (const void*)k_mis_fetch<false, Ray4>, tb);
-            g.mis[2][c] = grid_for(c ? (const void*)k_mis_fetch<true, RayQ> : (const void*)k_mis_fetch<false, RayQ>, tb);
+            for (int k = 1; k < TRACE_KINDS; k++)
+                by_ray(k, [&](auto tag) {
+                    using R = C2G_RAY(tag);
+                    g.ext[k][c] = grid_for(c ? (const void*)k_extend_fetch<true, R> : (const void*)k_extend_fetch<false, R>, tb);
+                    g.sh[k][c] = grid_for(c ? (const void*)k_shadow_fetch<true, R> : (const void*)k_shadow_fetch<false, R>, tb);
+                    g.mis[k][c] = grid_for(c ? (const void*)k_mis_fetch<true, R> : (const void*)k_mis_fetch<false, R>, tb);
+                });
         }
     }
 }
@@ -1721,12 +1736,12 @@ void launch_extend(const DevScene& S, int tb, const WaveBuffers& w, int q, int* 
     if (k == TRACE_PLAIN) {
         if (count) k_extend<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_extend<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
-    } else if (k == TRACE_QUANT4) {
-        if (count) k_extend_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
-        else k_extend_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
     } else {
-        if (count) k_extend_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
-        else k_extend_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
+        by_ray(k, [&](auto tag) {
+            using R = C2G_RAY(tag);
+            if (count) k_extend_fetch<true, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
+            else k_extend_fetch<false, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntExtendFetch, cnt);
+        });
     }
 #undef C2G_ARGS
 }
@@ -1737,12 +1752,12 @@ void launch_shadow(const DevScene& S, int tb, const WaveBuffers& w, bool count, 
     if (k == TRACE_PLAIN) {
         if (count) k_shadow<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_shadow<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
-    } else if (k == TRACE_QUANT4) {
-        if (count) k_shadow_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
-        else k_shadow_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
     } else {
-        if (count) k_shadow_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
-        else k_shadow_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
+        by_ray(k, [&](auto tag) {
+            using R = C2G_RAY(tag);
+            if (count) k_shadow_fetch<true, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
+            else k_shadow_fetch<false, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntShadowFetch, cnt);
+        });
     }
 #undef C2G_ARGS
 }
@@ -1753,12 +1768,12 @@ void launch_mis(const DevScene& S, int tb, const WaveBuffers& w, bool count, uns
     if (k == TRACE_PLAIN) {
         if (count) k_mis<true><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
         else k_mis<false><<<g, tb, 0, st>>>(C2G_ARGS, cnt);
-    } else if (k == TRACE_QUANT4) {
-        if (count) k_mis_fetch<true, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
-        else k_mis_fetch<false, Ray4><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
     } else {
-        if (count) k_mis_fetch<true, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
-        else k_mis_fetch<false, RayQ><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+        by_ray(k, [&](auto tag) {
+            using R = C2G_RAY(tag);
+            if (count) k_mis_fetch<true, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+            else k_mis_fetch<false, R><<<g, tb, 0, st>>>(C2G_ARGS, C + kCntMisFetch, cnt);
+        });
     }
 #undef C2G_ARGS
 }
@@ -1766,12 +1781,13 @@ void launch_mis(const DevScene& S, int tb, const WaveBuffers& w, bool count, uns
 // Lanes per path of k_finish: two more than the lights, as a power of two from 8 on.
 int finish_log2g(int K) { return K <= 6 ? 3 : (K <= 14 ? 4 : 5); }
 void launch_finish(const DevScene& S, const WaveArgs& a, const WaveBuffers& w, int q, bool have_hits, cudaStream_t st) {
-    const bool exact = trace_kind(S) == TRACE_EXACT4;
+    const int kind = trace_kind(S);
     const PathRefs cur{w.o[q], w.d[q], w.beta[q], w.L[q]};
     const float4* hits = have_hits ? w.hit : nullptr;
     int* C = w.counters;
-    if (exact) k_finish<RayQ><<<g_finish[1], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q * kLine, C + kCntFinish, finish_log2g(a.K));
-    else k_finish<Ray4><<<g_finish[0], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q * kLine, C + kCntFinish, finish_log2g(a.K));
+    by_ray(kind, [&](auto tag) {
+        k_finish<C2G_RAY(tag)><<<g_finish[kind], 128, 0, st>>>(S, a, cur, hits, w.out_L, C + q * kLine, C + kCntFinish, finish_log2g(a.K));
+    });
 }
 
 __global__ void k_advance(int* sample0, int by) { *sample0 += by; }
@@ -2347,23 +2363,19 @@ int GpuScene::trace_rays_dev(int n, const float* o, const float* d, const float*
     const DevScene& S = sb_->S;
     const int kind = trace_kind(S);
     if (kind != TRACE_PLAIN) {
-        static int grids[2][2] = {};
-        if (!grids[0][0]) {
-            grids[0][0] = grid_for((const void*)k_closest_rays_fetch<Ray4>, 128);
-            grids[0][1] = grid_for((const void*)k_any_rays_fetch<Ray4>, 128);
-            grids[1][0] = grid_for((const void*)k_closest_rays_fetch<RayQ>, 128);
-            grids[1][1] = grid_for((const void*)k_any_rays_fetch<RayQ>, 128);
-        }
-        const bool exact = kind == TRACE_EXACT4;
-        const int g = grids[exact][any_hit ? 1 : 0];
+        static int grids[TRACE_KINDS][2] = {};
+        if (!grids[kind][0])
+            by_ray(kind, [&](auto tag) {
+                grids[kind][1] = grid_for((const void*)k_any_rays_fetch<C2G_RAY(tag)>, 128);
+                grids[kind][0] = grid_for((const void*)k_closest_rays_fetch<C2G_RAY(tag)>, 128);
+            });
+        const int g = grids[kind][any_hit ? 1 : 0];
         C2G_CUDA(cudaMemsetAsync(sb_->fetch, 0, sizeof(int), st));
-        if (any_hit) {
-            if (exact) k_any_rays_fetch<RayQ><<<g, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, obj, sb_->fetch);
-            else k_any_rays_fetch<Ray4><<<g, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, obj, sb_->fetch);
-        } else {
-            if (exact) k_closest_rays_fetch<RayQ><<<g, 128, 0, st>>>(S, n, o, d, obj, t, sb_->fetch);
-            else k_closest_rays_fetch<Ray4><<<g, 128, 0, st>>>(S, n, o, d, obj, t, sb_->fetch);
-        }
+        by_ray(kind, [&](auto tag) {
+            using R = C2G_RAY(tag);
+            if (any_hit) k_any_rays_fetch<R><<<g, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, obj, sb_->fetch);
+            else k_closest_rays_fetch<R><<<g, 128, 0, st>>>(S, n, o, d, obj, t, sb_->fetch);
+        });
     } else {
         k_trace_rays<<<(n + 127) / 128, 128, 0, st>>>(S, n, o, d, tmin, tmax, ignore, any_hit, obj, t);
     }

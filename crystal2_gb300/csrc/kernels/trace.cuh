@@ -32,48 +32,59 @@ __device__ __forceinline__ RayQ make_rayq(float3 o, float3 d) {
 }
 
 // Ray of the four-wide traversal with quantised planes: iv is the reciprocal direction clamped to
-// +-S.inv_max, m the amount by which its slab distances are widened (see node4_slabs).
-constexpr float kSlabMargin = 20.f * 0x1p-24f;
-struct Ray4 {
+// +-S.inv_max, m the amount by which its slab distances are widened (see slab_axis).  NEAR: m holds the
+// ray's own part, and every node adds what its numbers need; else m covers the whole scene.
+template <bool NEAR>
+struct QuantRay {
     float3 o, d, iv, m;
 };
+using Ray4 = QuantRay<false>;
+using Ray4n = QuantRay<true>;
+constexpr float kUlp = 0x1p-24f;
 
 __device__ __forceinline__ float inv_clamped(const DevScene& S, float d) { return fminf(fmaxf(__frcp_rn(d), -S.inv_max), S.inv_max); }
+__device__ __forceinline__ float max_abs(float3 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
 
-// R: Ray4 (quantised planes) or RayQ (exact planes)
+// R: Ray4 or Ray4n (quantised planes), or RayQ (exact planes)
 template <class R>
-__device__ __forceinline__ R make_ray(const DevScene& S, float3 o, float3 d);
+struct RayMaker;
 template <>
-__device__ __forceinline__ RayQ make_ray<RayQ>(const DevScene&, float3 o, float3 d) { return make_rayq(o, d); }
-template <>
-__device__ __forceinline__ Ray4 make_ray<Ray4>(const DevScene& S, float3 o, float3 d) {
-    Ray4 r;
-    r.o = o;
-    r.d = d;
-    r.iv = f3(inv_clamped(S, d.x), inv_clamped(S, d.y), inv_clamped(S, d.z));
-    r.m = f3((S.extent[0] + fabsf(o.x)) * kSlabMargin * fabsf(r.iv.x), (S.extent[1] + fabsf(o.y)) * kSlabMargin * fabsf(r.iv.y),
-             (S.extent[2] + fabsf(o.z)) * kSlabMargin * fabsf(r.iv.z));
-    // clamped components: no distance at which the ray can meet the scene may lie outside their slabs
-    const float longest = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
-    const float far = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), S.reach));
-    const float whole = longest > 0.f ? 8.f * far * __frcp_rn(longest) : 0.f;
-    if (fabsf(r.iv.x) == S.inv_max) r.m.x += whole;
-    if (fabsf(r.iv.y) == S.inv_max) r.m.y += whole;
-    if (fabsf(r.iv.z) == S.inv_max) r.m.z += whole;
-    return r;
-}
+struct RayMaker<RayQ> {
+    static __device__ __forceinline__ RayQ make(const DevScene&, float3 o, float3 d) { return make_rayq(o, d); }
+};
+template <bool NEAR>
+struct RayMaker<QuantRay<NEAR>> {
+    static __device__ __forceinline__ QuantRay<NEAR> make(const DevScene& S, float3 o, float3 d) {
+        QuantRay<NEAR> r;
+        r.o = o;
+        r.d = d;
+        r.iv = f3(inv_clamped(S, d.x), inv_clamped(S, d.y), inv_clamped(S, d.z));
+        // clamped components: no distance at which the ray can meet the scene may lie outside their slabs
+        const float ix = fabsf(r.iv.x), iy = fabsf(r.iv.y), iz = fabsf(r.iv.z);
+        const float whole = max_abs(d) > 0.f ? 8.f * fmaxf(max_abs(o), S.reach) * fminf(fminf(ix, iy), iz) : 0.f;
+        r.m = f3(margin(S.extent[0], o.x) * ix + (ix == S.inv_max ? whole : 0.f), margin(S.extent[1], o.y) * iy + (iy == S.inv_max ? whole : 0.f),
+                 margin(S.extent[2], o.z) * iz + (iz == S.inv_max ? whole : 0.f));
+        return r;
+    }
+    static __device__ __forceinline__ float margin(float extent, float o) {
+        return NEAR ? 2.f * kUlp * fabsf(o) : __fmaf_rn(fabsf(o), 7.f * kUlp, extent * (16.f * kUlp));
+    }
+};
+template <class R>
+__device__ __forceinline__ R make_ray(const DevScene& S, float3 o, float3 d) { return RayMaker<R>::make(S, o, d); }
 
 // Thresholds of trace_queue.
-template <class R> struct QueueTuning;
-template <> struct QueueTuning<Ray4> { static constexpr int kWalkers = 10, kLeaves = 8; };
+template <class R> struct QueueTuning { static constexpr int kWalkers = 10, kLeaves = 8; };
 template <> struct QueueTuning<RayQ> { static constexpr int kWalkers = 0, kLeaves = 1; };
 
 // Whether the boxes above a leaf may be larger than exact.
 __device__ __forceinline__ constexpr bool loose_boxes(const RayQ&) { return false; }
-__device__ __forceinline__ constexpr bool loose_boxes(const Ray4&) { return true; }
+template <bool NEAR>
+__device__ __forceinline__ constexpr bool loose_boxes(const QuantRay<NEAR>&) { return true; }
 // The exact ray of the primitive tests.
 __device__ __forceinline__ const RayQ& exact_ray(const DevScene&, const RayQ& r) { return r; }
-__device__ __forceinline__ RayQ exact_ray(const DevScene& S, const Ray4& r) {
+template <bool NEAR>
+__device__ __forceinline__ RayQ exact_ray(const DevScene& S, const QuantRay<NEAR>& r) {
     RayQ q;
     q.o = r.o;
     q.d = r.d;
@@ -519,18 +530,28 @@ __device__ __forceinline__ bool trace_any_sah(const DevScene& S, const RayQ& r, 
 // rays 21.4 -> 17.4 ms, extension 12.6 -> 11.2 ms; 2M closest-hit rays of a 65k-triangle soup
 // 1.38 -> 0.93 ms, any hit 0.82 -> 0.54 ms.  15-bit planes (96 bytes) measured 18.8 / 12.3 ms.
 //
-// Slab distances: t = v(q) * (scale * iv) + (org - o) * iv, widened by m per ray.  With u = 2^-24 and E
-// the largest coordinate of the scene on the axis, |scale| <= 1.35 E and v < 2, the roundings of t
-// (product, org - o, offset, final FMA) come to at most u (7.1 E + 3 |o|) |iv|, those of the exact
-// test to 2 u (E + |o|) |iv|, and a plane may lie inside its box by 2^-21 E = 8 u E (quantise_axis):
-// together below m = 20 u (E + |o|) |iv|.  A direction component that is zero, or so small that the
-// ray crosses the whole scene without moving along the axis, gives iv = S.inv_max, and m then adds the
-// largest distance at which the ray can meet the scene: the slab accepts when the origin lies within it, up
-// to 2^-116 reach^2 for unit directions, whatever the length of the direction.  (Without this term
-// directions of 1e-28 and shorter, whose hits lie beyond 2^100 times their slab, lost them.)  S.inv_max is
-// 2^120 over the scene's reach, so that scale * iv and the offset of an origin among the scene's
-// coordinates stay finite (with 2^100 for every scene the product overflowed from 4e8 units on, and a near
-// plane at infinity hid the whole node).
+// Slab distances: t = v(q) * a + p with a = scale * iv and p = (org - o) * iv, widened by m.  With
+// u = 2^-24 and v < 2 the roundings of t (a, org - o, the offset and the final FMA) come to at most
+// u (4 |a| + 3 |p|), those of the exact test of a plane, at most 2 scale from org, to u (4 |a| + 2 |p|),
+// and a plane may lie inside its box by u (1.5 scale + |org|) (quantise_axis), where
+// |org| <= |org - o| + |o|: together u (9.5 |a| + 6 |p| + |o iv|).
+//   Ray4n: m = u (12 |a| + 8 |p| + 2 |o iv|), from the node's own numbers.
+//   Ray4: with E the scene's largest coordinate on the axis, planes and o at most E + |o| apart,
+//   scale <= 1.35 E and |org| <= 1.7 E, the same sum is below u (13 E + 5 |o|) |iv|; m = u (16 E + 7 |o|) |iv|
+//   is the ray's for all nodes, and saves two FMAs per axis.
+// One object far from all others makes E large against most boxes: 1e5 units from a soup of triangles of
+// 0.05 in the unit cube a ray tested 280 of them instead of 11, and every one at 1e6.  So scenes with more
+// than a few leaves narrower than 2^-14 of their reach, 64 times m, take Ray4n: 11 there, as without the far
+// object.  For every scene it would cost the 1080p many-material frame 0.4%, and 2M closest-hit rays of a
+// 65k-triangle soup 5%.
+//
+// A direction component that is zero, or so small that the ray crosses the whole scene without moving along
+// the axis, gives iv = S.inv_max, and m then adds the largest distance at which the ray can meet the scene:
+// the slab accepts when the origin lies within it, up to 2^-116 reach^2 for unit directions, whatever the
+// length of the direction.  (Without this term directions of 1e-28 and shorter, whose hits lie beyond 2^100
+// times their slab, lost them.)  S.inv_max is 2^120 over the scene's reach, so that scale * iv and the
+// offset of an origin among the scene's coordinates stay finite (with 2^100 for every scene the product
+// overflowed from 4e8 units on, and a near plane at infinity hid the whole node).
 constexpr int kStack4 = 128;
 
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
@@ -549,9 +570,11 @@ template <int K>
 __device__ __forceinline__ float plane_byte(uint32_t w) {
     return __uint_as_float(__byte_perm(w, 0x3f000000u, 0x7044u | (K << 8)));
 }
+template <bool NEAR>
 __device__ __forceinline__ void slab_axis(uint32_t qlo, uint32_t qhi, float org, float scale, float o, float iv, float m,
                                           float tn[4], float tf[4]) {
     const float dx = org - o, a = scale * iv;
+    if (NEAR) m = __fmaf_rn(__fmaf_rn(scale, 1.5f, fabsf(dx)), 8.f * kUlp * fabsf(iv), m);
     const float bn = __fmaf_rn(dx, iv, -m), bf = __fmaf_rn(dx, iv, m);
     const uint32_t wn = iv < 0.f ? qhi : qlo, wf = iv < 0.f ? qlo : qhi;
     fma2(plane_byte<0>(wn), plane_byte<1>(wn), a, bn, tn[0], tn[1]);
@@ -565,15 +588,16 @@ __device__ __forceinline__ void ld256(const void* p, uint32_t v[8]) {
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p));
 }
 // Entry and exit distances of a node's four child boxes, and its children.
-__device__ __forceinline__ int4 node4_slabs(const DevScene& S, int ref, const Ray4& r, float t0, float t1, float tn[4], float tf[4]) {
+template <bool NEAR>
+__device__ __forceinline__ int4 node4_slabs(const DevScene& S, int ref, const QuantRay<NEAR>& r, float t0, float t1, float tn[4], float tf[4]) {
     const Node4* nodes = S.nodes4;
     uint32_t u[8], v[8];
     ld256(nodes + ref, u);
     ld256(reinterpret_cast<const char*>(nodes + ref) + 32, v);
     float xn[4], xf[4], yn[4], yf[4], zn[4], zf[4];
-    slab_axis(u[6], u[7], __uint_as_float(u[0]), __uint_as_float(u[3]), r.o.x, r.iv.x, r.m.x, xn, xf);
-    slab_axis(v[0], v[1], __uint_as_float(u[1]), __uint_as_float(u[4]), r.o.y, r.iv.y, r.m.y, yn, yf);
-    slab_axis(v[2], v[3], __uint_as_float(u[2]), __uint_as_float(u[5]), r.o.z, r.iv.z, r.m.z, zn, zf);
+    slab_axis<NEAR>(u[6], u[7], __uint_as_float(u[0]), __uint_as_float(u[3]), r.o.x, r.iv.x, r.m.x, xn, xf);
+    slab_axis<NEAR>(v[0], v[1], __uint_as_float(u[1]), __uint_as_float(u[4]), r.o.y, r.iv.y, r.m.y, yn, yf);
+    slab_axis<NEAR>(v[2], v[3], __uint_as_float(u[2]), __uint_as_float(u[5]), r.o.z, r.iv.z, r.m.z, zn, zf);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         tn[k] = fmaxf(fmaxf(xn[k], yn[k]), fmaxf(zn[k], t0));

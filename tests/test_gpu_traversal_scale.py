@@ -90,3 +90,25 @@ def test_directions_of_any_length(tmp_path, length, far):
         o, d = _free_rays(8)
         d[np.arange(len(d)), np.arange(len(d)) % 3] *= np.float32(2.0 ** -length if length > 0 else 2.0 ** length)
         _compare(ctx, o, d, np.full(len(o), 0.5, np.float32))
+
+
+# The boxes below the root are as tight as without the far triangle.  The children of the root (and of the few
+# nodes that still span the distance) may all be entered, and the tree's levels pair up differently: four nodes
+# and a quarter more.
+@pytest.mark.parametrize("far", [1e2, 1e4, 1e5, 1e6, 1e9, 1e18])
+def test_a_far_triangle_costs_no_culling(tmp_path, far):
+    per_ray = []
+    for k, dist in enumerate((0, far)):
+        d = tmp_path / str(k)
+        d.mkdir()
+        (cp, sp), _ = _soup(str(d), dist)
+        with Context(0) as ctx:
+            ctx.load(cp, sp, tree=N.TREE_SAH)
+            ctx.set_counting(N.COUNT_TRAVERSAL)
+            ctx.render(ctx.render_params())
+            s = ctx.stats()
+            assert s.rays[N.K_EXTEND] > 4096
+            per_ray.append((s.nodes[N.K_EXTEND] / s.rays[N.K_EXTEND], s.prims[N.K_EXTEND] / s.rays[N.K_EXTEND]))
+    (nodes0, prims0), (nodes1, prims1) = per_ray
+    assert nodes1 <= 1.25 * nodes0 + 4
+    assert prims1 <= 1.25 * prims0 + 1
