@@ -112,32 +112,32 @@ __device__ __forceinline__ float2 cos_sin_phi(float3 w, float sinT) {
     return make_float2(fminf(fmaxf(w.x / sinT, -1.f), 1.f), fminf(fmaxf(-w.z / sinT, -1.f), 1.f));
 }
 
-__device__ __forceinline__ float ndf_D(const BxDF& b, float3 wh) {
+__device__ __forceinline__ float ndf_D(const BxDF& b, float3 wh, Rounding r) {
     if (!is_beckmann(b.mtype)) {
         float cos2 = wh.y * wh.y;
-        float sin2 = fmaxf(0.f, 1.f - cos2);
+        float sin2 = fmaxf(0.f, r == Rounding::FREE ? 1.f - cos2 : r == Rounding::SAMPLED ? one_minus_rounded_sq(wh.y) : one_minus_sq(wh.y));
         float2 p = cos_sin_phi(wh, sqrtf(sin2));
         float A = sq(p.x) / sq(b.ax) + sq(p.y) / sq(b.ay);
-        return 1.f / (kPiF * b.ax * b.ay * sq(A - cos2 * (A - 1)));
+        return 1.f / (kPiF * b.ax * b.ay * sq(r == Rounding::FREE ? A - cos2 * (A - 1) : __fmaf_rn(-cos2, A - 1, A)));
     }
     float cos2 = wh.y * wh.y;
-    float sin2 = 1.f - cos2;
+    float sin2 = r == Rounding::FREE ? 1.f - cos2 : one_minus_rounded_sq(wh.y);
     float tan2 = sin2 / cos2;
     if (isinf(tan2)) return 0.f;
     float cos4 = cos2 * cos2;
-    float2 v = cos_sin_phi(wh, sqrtf(sin2));
+    float2 v = cos_sin_phi(wh, sqrtf(r == Rounding::LIGHT ? one_minus_sq(wh.y) : sin2));
     float bot = kPiF * b.ax * b.ay * cos4;
     float top = expf(-tan2 * (sq(v.x) / sq(b.ax) + sq(v.y) / sq(b.ay)));
     return top / bot;
 }
 
-__device__ __forceinline__ float ndf_lambda(const BxDF& b, float3 w) {
+__device__ __forceinline__ float ndf_lambda(const BxDF& b, float3 w, Rounding r) {
     if (!is_beckmann(b.mtype)) {
         float cos2 = w.y * w.y;
-        float sin2 = 1.f - cos2;
+        float sin2 = r == Rounding::FREE ? 1.f - cos2 : one_minus_rounded_sq(w.y);
         float tan2 = sin2 / cos2;
         if (isinf(tan2)) return 0.f;
-        float2 p = cos_sin_phi(w, sqrtf(sin2));
+        float2 p = cos_sin_phi(w, sqrtf(r == Rounding::LIGHT ? one_minus_sq(w.y) : sin2));
         float a2 = sq(p.x) * sq(b.ax) + sq(p.y) * sq(b.ay);
         return (-1 + sqrtf(1 + a2 * tan2)) / 2;
     }
@@ -153,7 +153,7 @@ __device__ __forceinline__ float ndf_lambda(const BxDF& b, float3 w) {
 }
 
 // Smith's G of the prepared wo (b.term_o is its Lambda) and wi.
-__device__ __forceinline__ float ndf_G(const BxDF& b, float3 wi) { return 1.f / (1.f + b.term_o + ndf_lambda(b, wi)); }
+__device__ __forceinline__ float ndf_G(const BxDF& b, float3 wi, Rounding r) { return 1.f / (1.f + b.term_o + ndf_lambda(b, wi, r)); }
 
 // GetUnitVectorUsingCos (Utils.h:79-83)
 __device__ __forceinline__ float3 unit_from_cos(float cosT, float phi) {
@@ -217,10 +217,10 @@ __device__ __forceinline__ bool refract(float3 wo, float3 wh, float eta, float3&
 // (bsdf_prepare), and a sampled direction uses its H and D twice, unless the clamp that follows the
 // density changed it.  Shading of the slit room (most of it GGX): 4.65 -> 4.30 ms, of the many-material frame 12.7 -> 11.3.
 __device__ __forceinline__ float mf_refl_pdf(float3 wo, float3 H, float D) { return D * fabsf(H.y) / (4 * dot(wo, H)); }
-__device__ __forceinline__ float3 mf_refl_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
+__device__ __forceinline__ float3 mf_refl_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D, Rounding r) {
     if (wo.y * wi.y < 0) return f3(0.f, 0.f, 0.f);
     float F = bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wi);
+    float G = ndf_G(b, wi, r);
     return b.R * D * G * F / (4 * fmaxf(0.f, wi.y) * fmaxf(0.f, wo.y));
 }
 __device__ __forceinline__ float mf_trans_pdf(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
@@ -229,14 +229,14 @@ __device__ __forceinline__ float mf_trans_pdf(const BxDF& b, float3 wo, float3 w
     float s = dot(wo, H) + eta * dot(wi, H);
     return D * fabsf(H.y) * (eta * eta * fabsf(dot(H, wi)) / sq(s));
 }
-__device__ __forceinline__ float3 mf_trans_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D) {
+__device__ __forceinline__ float3 mf_trans_f(const BxDF& b, float3 wo, float3 wi, float3 H, float D, Rounding r) {
     if (wi.y * wo.y > 0) return f3(0.f, 0.f, 0.f);
     if (wo.y == 0.f) return f3(0.f, 0.f, 0.f);
     float eta = b.eta_ba;
     if (H.y < 0) H = -H;  // D is even in H
     float bot = sq(dot(wo, H) + eta * dot(wi, H));
     float F = 1.f - bxdf_fresnel(b, fmaxf(0.f, dot(wo, H)));
-    float G = ndf_G(b, wi);
+    float G = ndf_G(b, wi, r);
     return b.R * D * G * F * fabsf(dot(H, wo)) * fabsf(dot(H, wi)) / (bot * fmaxf(0.f, -wi.y) * fmaxf(0.f, wo.y));
 }
 // Half vector of a reflection, or of a transmission.
@@ -244,41 +244,44 @@ __device__ __forceinline__ float3 mf_half(const BxDF& b, bool trans, float3 wo, 
     return normalize(wo + wi * (trans ? b.eta_ba : 1.f));
 }
 // f and pdf of one (wo, wi) pair.
-__device__ __forceinline__ float3 mf_f_pdf(const BxDF& b, bool trans, float3 wo, float3 wi, float& pdf) {
+__device__ __forceinline__ float3 mf_f_pdf(const BxDF& b, bool trans, float3 wo, float3 wi, float& pdf, Rounding r) {
     const float3 H = mf_half(b, trans, wo, wi);
-    const float D = ndf_D(b, H);
+    const float D = ndf_D(b, H, r);
     pdf = trans ? mf_trans_pdf(b, wo, wi, H, D) : mf_refl_pdf(wo, H, D);
-    return trans ? mf_trans_f(b, wo, wi, H, D) : mf_refl_f(b, wo, wi, H, D);
+    return trans ? mf_trans_f(b, wo, wi, H, D, r) : mf_refl_f(b, wo, wi, H, D, r);
 }
 // f and pdf of a sampled direction: the density of wi as drawn, then f of wi clamped to [-1, 1].  The
 // density takes the technique from wi's side (glass), f from the technique that drew it.
-__device__ __forceinline__ float3 mf_sampled(const BxDF& b, bool trans, float3 wo, float3& wi, float& pdf) {
+__device__ __forceinline__ float3 mf_sampled(const BxDF& b, bool trans, float3 wo, float3& wi, float& pdf, Rounding r) {
     const bool across = b.mtype == MAT_GLASS_ROUGH && wo.y * wi.y < 0;
     float3 H = mf_half(b, across, wo, wi);
-    float D = ndf_D(b, H);
+    float D = ndf_D(b, H, r);
     pdf = across ? mf_trans_pdf(b, wo, wi, H, D) : mf_refl_pdf(wo, H, D);
     const float3 c = clamp1(wi);
     if (c.x != wi.x || c.y != wi.y || c.z != wi.z || trans != across) {
         H = mf_half(b, trans, wo, c);
-        D = ndf_D(b, H);
+        D = ndf_D(b, H, r);
     }
     wi = c;
-    return trans ? mf_trans_f(b, wo, wi, H, D) : mf_refl_f(b, wo, wi, H, D);
+    return trans ? mf_trans_f(b, wo, wi, H, D, r) : mf_refl_f(b, wo, wi, H, D, r);
 }
 
 // ---- FresnelBlend (BSDFs/FresnelBlend.cpp) ----------------------------------------------
 __device__ __forceinline__ float fb_power(float cosT) { return 1.f - powf(1.f - 0.5f * cosT, 5.f); }
-__device__ __forceinline__ float3 fb_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
+__device__ __forceinline__ float3 fb_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf, Rounding r) {
     float3 H = normalize(wo + wi);
-    float D = ndf_D(b, H);
+    float D = ndf_D(b, H, r);
     pdf = 0.5f * (over_pi(fmaxf(0.f, wi.y)) + D * fabsf(H.y) / (4 * dot(wo, H)));
     float cosI = fmaxf(0.f, wi.y), cosO = fmaxf(0.f, wo.y);
     float k = (28.f / (23.f * kPiF));
-    float3 diffuse = k * b.R * (f3(1.f, 1.f, 1.f) - b.S) * b.term_o * fb_power(cosI);
+    float3 diffuse = k * b.R * (f3(1.f, 1.f, 1.f) - b.S) * b.term_o;  // times fb_power(cosI)
     float cwh = dot(wi, H);
     float sp = D / (4 * cwh * fmaxf(cosI, cosO));
     float3 schlick = b.S + (f3(1.f, 1.f, 1.f) - b.S) * powf(1.f - cwh, 5.f);
-    return diffuse + sp * schlick;
+    const float pw = fb_power(cosI);
+    if (r == Rounding::FREE) return diffuse * pw + sp * schlick;
+    return f3(__fmaf_rn(diffuse.x, pw, __fmul_rn(sp, schlick.x)), __fmaf_rn(diffuse.y, pw, __fmul_rn(sp, schlick.y)),
+              __fmaf_rn(diffuse.z, pw, __fmul_rn(sp, schlick.z)));
 }
 
 // ---- Oren-Nayar (BSDFs/Reflections.cpp:7-66); A, B in ax, ay -----------------------------
@@ -321,14 +324,14 @@ __device__ __forceinline__ float2 phong_redraw(float2 u, int attempt) {
 
 // ---- per-BxDF dispatch (local frame) ------------------------------------------------------
 // f and pdf of the BxDF at one (wo, wi) pair.
-__device__ __forceinline__ float3 bxdf_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf) {
+__device__ __forceinline__ float3 bxdf_f_pdf(const BxDF& b, float3 wo, float3 wi, float& pdf, Rounding r) {
     switch (b.mtype) {
         case MAT_DIFFUSE: pdf = over_pi(fmaxf(0.f, wi.y)); return b.R_pi;
         case MAT_MICRO_GGX:
-        case MAT_MICRO_BECKMANN: return mf_f_pdf(b, false, wo, wi, pdf);
-        case MAT_GLASS_ROUGH: return mf_f_pdf(b, wo.y * wi.y < 0, wo, wi, pdf);
+        case MAT_MICRO_BECKMANN: return mf_f_pdf(b, false, wo, wi, pdf, r);
+        case MAT_GLASS_ROUGH: return mf_f_pdf(b, wo.y * wi.y < 0, wo, wi, pdf, r);
         case MAT_PLASTIC_GGX:
-        case MAT_PLASTIC_BECKMANN: return fb_f_pdf(b, wo, wi, pdf);
+        case MAT_PLASTIC_BECKMANN: return fb_f_pdf(b, wo, wi, pdf, r);
         case MAT_ORENNAYAR: pdf = over_pi(fmaxf(0.f, wi.y)); return on_f(b, wo, wi);
         case MAT_BLINNPHONG: pdf = bp_pdf(b, wo, wi); return bp_f(b, wo, wi);
     }
@@ -350,7 +353,7 @@ __device__ __forceinline__ float3 cosine_hemisphere(float2 u, float& pdf) {
 
 // BxDF::SampleDirection.  Returns f; writes wi (local), pdf and the sampled type.  A zero return
 // leaves pdf as it was, like the reference.
-__device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo, float3& wi, float& pdf, int& stype) {
+__device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo, float3& wi, float& pdf, int& stype, Rounding r) {
     const float3 zero = f3(0.f, 0.f, 0.f);
     switch (b.mtype) {
         case MAT_DIFFUSE: {
@@ -380,7 +383,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
             float3 wh = ndf_sample(b, u);
             if (dot(wo, wh) <= 0) return zero;
             wi = reflect(-wo, wh);
-            return mf_sampled(b, false, wo, wi, pdf);
+            return mf_sampled(b, false, wo, wi, pdf, r);
         }
         case MAT_GLASS_ROUGH: {  // MicrofacetBlend (Microfacet.cpp:164-199)
             float3 wh = ndf_sample(b, u);
@@ -391,7 +394,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
             const bool trans = !refl && refract(wo, wh, b.eta_ab, t);  // else total reflection
             stype = (trans ? BXDF_TRANSMISSION : BXDF_REFLECTION) | BXDF_GLOSSY;
             wi = trans ? t : reflect(-wo, wh);
-            const float3 f = mf_sampled(b, trans, wo, wi, pdf);
+            const float3 f = mf_sampled(b, trans, wo, wi, pdf, r);
             pdf = pdf * (refl ? fr : 1 - fr);
             return f;
         }
@@ -408,7 +411,7 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
                 if (L.y * wo.y <= 0) return zero;
                 wi = clamp1(L);
             }
-            return fb_f_pdf(b, wo, wi, pdf);
+            return fb_f_pdf(b, wo, wi, pdf, r);
         }
         case MAT_ORENNAYAR: {
             wi = cosine_hemisphere(u, pdf);
@@ -437,12 +440,12 @@ __device__ __forceinline__ float3 bxdf_sample(const BxDF& b, float2 u, float3 wo
 __device__ __forceinline__ bool matches(int bxdf_flags, int flags) { return (bxdf_flags & flags) == bxdf_flags; }
 
 // The terms of f that depend on wo alone, once per vertex; before the calls below.
-__device__ __forceinline__ void bsdf_prepare(BxDF& b, const Frame& fr, float3 wo_w) {
+__device__ __forceinline__ void bsdf_prepare(BxDF& b, const Frame& fr, float3 wo_w, bool guided) {
     const float3 wo = to_local(fr, wo_w);
     switch (b.mtype) {
         case MAT_MICRO_GGX:
         case MAT_MICRO_BECKMANN:
-        case MAT_GLASS_ROUGH: b.term_o = ndf_lambda(b, wo); break;
+        case MAT_GLASS_ROUGH: b.term_o = ndf_lambda(b, wo, guided ? Rounding::FREE : Rounding::SAMPLED); break;
         case MAT_PLASTIC_GGX:
         case MAT_PLASTIC_BECKMANN: b.term_o = fb_power(fmaxf(0.f, wo.y)); break;
         default: b.term_o = 0.f;
@@ -450,7 +453,7 @@ __device__ __forceinline__ void bsdf_prepare(BxDF& b, const Frame& fr, float3 wo
 }
 
 // BSDF::DistributionFunction and BSDF::Pdf(flags) of one direction pair in one pass.
-__device__ __forceinline__ float3 bsdf_f_pdf(const BxDF& b, const Frame& fr, float3 wo_w, float3 wi_w, int flags, float& pdf) {
+__device__ __forceinline__ float3 bsdf_f_pdf(const BxDF& b, const Frame& fr, float3 wo_w, float3 wi_w, int flags, float& pdf, bool guided) {
     float3 wo = to_local(fr, wo_w), wi = to_local(fr, wi_w);
     bool refl = wi.y * wo.y > 0;
     bool fcond = (refl && (b.flags & BXDF_REFLECTION)) || (!refl && (b.flags & BXDF_TRANSMISSION));
@@ -459,7 +462,7 @@ __device__ __forceinline__ float3 bsdf_f_pdf(const BxDF& b, const Frame& fr, flo
     float3 f = f3(0.f, 0.f, 0.f);
     if (fcond || pcond) {
         float p;
-        float3 v = bxdf_f_pdf(b, wo, wi, p);
+        float3 v = bxdf_f_pdf(b, wo, wi, p, guided ? Rounding::FREE : Rounding::LIGHT);
         if (fcond) f = v;
         if (pcond) pdf = p;
     }
@@ -469,7 +472,7 @@ __device__ __forceinline__ float3 bsdf_f_pdf(const BxDF& b, const Frame& fr, flo
 // Returns f; wi_w, pdf, stype written when the BxDF matches `flags`.  ok = false when the BSDF
 // returned zero (no matching BxDF, or the sampled value/pdf is zero).
 __device__ __forceinline__ float3 bsdf_sample(const BxDF& b, const Frame& fr, float u1, float2 u2, float3 wo_w,
-                                              float3& wi_w, float& pdf, int flags, int& stype, bool& ok) {
+                                              float3& wi_w, float& pdf, int flags, int& stype, bool& ok, bool guided) {
     ok = false;
     const float3 zero = f3(0.f, 0.f, 0.f);
     if (!matches(b.flags, flags)) return zero;
@@ -477,7 +480,7 @@ __device__ __forceinline__ float3 bsdf_sample(const BxDF& b, const Frame& fr, fl
     stype = b.flags;
     float3 wo = to_local(fr, wo_w);
     float3 wi = zero;
-    float3 L = bxdf_sample(b, u2, wo, wi, pdf, stype);
+    float3 L = bxdf_sample(b, u2, wo, wi, pdf, stype, guided ? Rounding::FREE : Rounding::SAMPLED);
     if (is_zero(L) || pdf == 0.f) return zero;
     wi_w = to_world(fr, wi);
     ok = true;

@@ -25,6 +25,22 @@ __device__ __forceinline__ float3 operator*(float s, float3 a) { return f3(a.x *
 __device__ __forceinline__ float3 operator*(float3 a, float3 b) { return f3(a.x * b.x, a.y * b.y, a.z * b.z); }
 __device__ __forceinline__ float3 operator/(float3 a, float s) { return f3(a.x / s, a.y / s, a.z / s); }
 __device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// Roundings of the sums in direct light and BxDFs.  Which product of a sum the compiler fuses depends on the
+// code around it, and the level kernels and the finishing kernel must give a path the same bits: where they
+// came out differently, the form that the level kernels had is spelled out, for the direction to a light
+// (LIGHT) and for a sampled one (SAMPLED).  Guided vertices are shaded by one kernel alone: FREE leaves it
+// to the compiler (with these forms the guided bucket spills more, and takes 0.8% longer).
+enum class Rounding { FREE, LIGHT, SAMPLED };
+__device__ __forceinline__ float dot_xfirst(float3 a, float3 b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y))); }
+__device__ __forceinline__ float dot_yfirst(float3 a, float3 b) { return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x))); }
+__device__ __forceinline__ float dot_xfirst(float3 a, float3 b, Rounding r) {
+    return r == Rounding::FREE ? a.x * b.x + a.y * b.y + a.z * b.z : dot_xfirst(a, b);
+}
+__device__ __forceinline__ float dot_yfirst(float3 a, float3 b, Rounding r) {
+    return r == Rounding::FREE ? a.x * b.x + a.y * b.y + a.z * b.z : dot_yfirst(a, b);
+}
+__device__ __forceinline__ float one_minus_sq(float x) { return __fmaf_rn(-x, x, 1.f); }                    // one rounding
+__device__ __forceinline__ float one_minus_rounded_sq(float x) { return __fsub_rn(1.f, __fmul_rn(x, x)); }  // two
 __device__ __forceinline__ float3 cross(float3 a, float3 b) {
     return f3(a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y);
 }

@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                 bx.mtype = MT;  // compile-time material: the BxDF switches fold away
                 bx.flags = material_flags(MT);
                 fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
-                bsdf_prepare(bx, fr, wo);
+                bsdf_prepare(bx, fr, wo, G);
                 do_nee = true;
             }
         }
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
             nee_work = (bx.flags & BXDF_SPECULAR) == 0;
             if (nee_work && n_area > 0 && !gvert) {
                 int stype = 0;
-                f2 = bsdf_sample(bx, fr, 0.f, uB, wo, wi2, pdf_b2, nsflags, stype, mis_ok);
+                f2 = bsdf_sample(bx, fr, 0.f, uB, wo, wi2, pdf_b2, nsflags, stype, mis_ok, G);
                 if (mis_ok) f2 = f2 * fmaxf(0.f, dot(s.N, wi2));
             }
         }
@@ -573,11 +573,11 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                     // light-sampling half (EsimateDirect, :195-227)
                     float3 lpos;
                     float pdf_l;
-                    float3 Li = light_sample_li(S, Lg, s.pos, s.N, uL, lpos, pdf_l);
-                    float3 wi = normalize(lpos - s.pos);
+                    float3 Li = light_sample_li(S, Lg, s.pos, s.N, uL, lpos, pdf_l, G ? Rounding::FREE : Rounding::LIGHT);
+                    float3 wi = light_direction(s.pos, lpos, G ? Rounding::FREE : Rounding::LIGHT);
                     if (pdf_l != 0.f && !is_zero(Li)) {
                         float pdf_b;
-                        float3 f = bsdf_f_pdf(bx, fr, wo, wi, nsflags, pdf_b) * fmaxf(0.f, dot(s.N, wi));
+                        float3 f = bsdf_f_pdf(bx, fr, wo, wi, nsflags, pdf_b, G) * fmaxf(0.f, dot(s.N, wi));
                         if (gvert && alpha < 1.f) pdf_b = alpha * pdf_b + (1.f - alpha) * packed_pdf(lobes, wi);
                         if (!is_zero(f)) {
                             bool back = dot(lpos - s.pos, s.N) < 0;
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                     }
                     // BSDF-sampling half (:229-270): weight for this light of the shared sample
                     if (mis_ok && Lg.type != LIGHT_POINT) {
-                        float pdf_l2 = light_pdf(S, Lg, s.pos, s.N, wi2);
+                        float pdf_l2 = light_pdf(S, Lg, s.pos, s.N, wi2, G ? Rounding::FREE : Rounding::SAMPLED);
                         if (pdf_l2 != 0.f) {
                             float3 m = beta * (f2 * power_heuristic(pdf_b2, pdf_l2) / pdf_b2);
                             mis_c4 = make_float4(m.x, m.y, m.z, 0.f);
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
             const bool mix = gvert && alpha < 1.f;
             const bool use_guide = mix && hash_uniform(pixel, sample, 0x4000u + 4u * bounce, S.seed) >= alpha;
             float3 f = f3(0.f, 0.f, 0.f);
-            if (!use_guide) f = bsdf_sample(bx, fr, u1, u2, wo, wi, pdf, BXDF_ALL, stype, ok);
+            if (!use_guide) f = bsdf_sample(bx, fr, u1, u2, wo, wi, pdf, BXDF_ALL, stype, ok, G);
             float pb_rec = pdf;  // BSDF density of the continuation (local measure), for training
             if (mix) {
                 // One-sample MIS over {BSDF, learned mixture}: q = alpha p_bsdf + (1 - alpha) p_guide,
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(128, C2G_SHADE_MIN_BLOCKS) k_shade(DevScene S,
                     const float sgn = dot(fr.T, c0) < 0.f ? -1.f : 1.f;
                     float3 l = normalize(f3(dot(c0, w), dot(c1, w), dot(c2, w)) * sgn);
                     pb_rec = 0.f;
-                    if (l.y * wol.y > 0.f) f = bxdf_f_pdf(bx, wol, l, pb_rec);  // reflection-only BxDFs
+                    if (l.y * wol.y > 0.f) f = bxdf_f_pdf(bx, wol, l, pb_rec, Rounding::FREE);  // reflection-only BxDFs
                     wi = to_world(fr, l);
                     stype = (bx.flags & ~(BXDF_REFLECTION | BXDF_TRANSMISSION)) | BXDF_REFLECTION;
                 }
@@ -867,8 +867,10 @@ __global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_mis_fetch(DevSce
 // step, whether 500 or 20 paths are left).  k_finish instead follows each path to its end: a group of
 // lanes holds one path, lane l of the group takes light l, the last two lanes the MIS ray and the
 // extension, the sampler's dimensions are evaluated one per lane, and the rays of all the warp's
-// groups are traced together.  Arithmetic and order of every sum are those of the level kernels.
-// 64 x 64 Cornell box at 1 spp: 0.36 ms in 58 launches -> 0.19 in 3; the 640 x 360 step 1.99 -> 1.44 ms.
+// groups are traced together.  A path's radiance has the bits that the level kernels give it (the functions
+// they share are compiled for the material, and see Rounding), so a film does not depend on which kernels
+// traced a wave's last levels.
+// 64 x 64 Cornell box at 1 spp: 0.36 ms in 58 launches -> 0.17 in 3; the 640 x 360 step 1.99 -> 1.42 ms.
 // Its bound is latency, then instruction fetch: four groups of one warp at four materials run one after
 // another (a version without the per-material functions was 0.15 ms, but its other contraction of
 // multiplies and adds turned paths behind mirrors and lenses).
@@ -932,44 +934,35 @@ __device__ __noinline__ float finish_sample(const DevScene& S, const FinishPath&
     return path_sample_part(S, P.vidx, dim, part, P.pixel, P.sample);
 }
 
-// What a vertex's direct light needs of it.
-struct NeeVertex {
-    Surface s;
-    BxDF bx;
-    Frame fr;
-    float3 wo, beta;
-    float2 uL, uB;      // the light pair and the BSDF pair
-};
-
 // Direct light of a vertex: this lane's light (sub), and the BSDF sample that all lights share.
-// One function for every material, not inlined: the BSDF switches stay in one place.
-__device__ __noinline__ void finish_nee(const DevScene& S, unsigned group, int sub, bool eligible, bool any_area, const NeeVertex& v, FinishPath& P) {
+__device__ __forceinline__ void finish_nee(const DevScene& S, unsigned group, int sub, bool eligible, bool any_area, const Surface& s,
+                                           const BxDF& bx, const Frame& fr, float3 wo, float3 beta, float2 uL, float2 uB, FinishPath& P) {
     const int nsflags = BXDF_ALL & ~BXDF_SPECULAR;
     bool mis_ok = false, lane_mis = false;
     float3 f2 = f3(0.f, 0.f, 0.f), wi2 = f3(0.f, 0.f, 0.f);
     float pdf_b2 = 0.f;
     if (any_area) {
         int stype = 0;
-        f2 = bsdf_sample(v.bx, v.fr, 0.f, v.uB, v.wo, wi2, pdf_b2, nsflags, stype, mis_ok);
-        if (mis_ok) f2 = f2 * fmaxf(0.f, dot(v.s.N, wi2));
+        f2 = bsdf_sample(bx, fr, 0.f, uB, wo, wi2, pdf_b2, nsflags, stype, mis_ok, false);
+        if (mis_ok) f2 = f2 * fmaxf(0.f, dot(s.N, wi2));
     }
     if (eligible) {
         const Light Lg = S.lights[sub];
         // light-sampling half (EsimateDirect, PathTracingIntegrator.cpp:195-227)
         float3 lpos;
         float pdf_l;
-        float3 Li = light_sample_li(S, Lg, v.s.pos, v.s.N, v.uL, lpos, pdf_l);
-        float3 wi = normalize(lpos - v.s.pos);
+        float3 Li = light_sample_li(S, Lg, s.pos, s.N, uL, lpos, pdf_l, Rounding::LIGHT);
+        float3 wi = light_direction(s.pos, lpos, Rounding::LIGHT);
         if (pdf_l != 0.f && !is_zero(Li)) {
             float pdf_b;
-            float3 f = bsdf_f_pdf(v.bx, v.fr, v.wo, wi, nsflags, pdf_b) * fmaxf(0.f, dot(v.s.N, wi));
+            float3 f = bsdf_f_pdf(bx, fr, wo, wi, nsflags, pdf_b, false) * fmaxf(0.f, dot(s.N, wi));
             if (!is_zero(f)) {
-                bool back = dot(lpos - v.s.pos, v.s.N) < 0;
-                float3 org = v.s.pos + (back ? -v.s.N : v.s.N) * kSpawnEps;
+                bool back = dot(lpos - s.pos, s.N) < 0;
+                float3 org = s.pos + (back ? -s.N : s.N) * kSpawnEps;
                 float3 c;
                 if (Lg.type == LIGHT_POINT) c = f * Li / pdf_l;
                 else c = f * Li * power_heuristic(pdf_l, pdf_b) / pdf_l;
-                P.sh_c = v.beta * c;
+                P.sh_c = beta * c;
                 P.has = true;
                 P.ign = Lg.type == LIGHT_AREA ? Lg.obj : -1;
                 P.o = org;
@@ -978,16 +971,16 @@ __device__ __noinline__ void finish_nee(const DevScene& S, unsigned group, int s
         }
         // BSDF-sampling half (:229-270): weight for this light of the shared sample
         if (mis_ok && Lg.type != LIGHT_POINT) {
-            float pdf_l2 = light_pdf(S, Lg, v.s.pos, v.s.N, wi2);
+            float pdf_l2 = light_pdf(S, Lg, s.pos, s.N, wi2, Rounding::SAMPLED);
             if (pdf_l2 != 0.f) {
-                P.mis_c = v.beta * (f2 * power_heuristic(pdf_b2, pdf_l2) / pdf_b2);
+                P.mis_c = beta * (f2 * power_heuristic(pdf_b2, pdf_l2) / pdf_b2);
                 lane_mis = true;
             }
         }
     }
     if (__any_sync(group, lane_mis)) {
         P.mis_ray = true;
-        P.mis_o = spawn_origin(v.s, wi2);
+        P.mis_o = spawn_origin(s, wi2);
         P.mis_d = wi2;
     }
 }
@@ -1031,7 +1024,7 @@ __device__ __noinline__ void finish_shade(const DevScene& S, const WaveArgs& a, 
         bx.flags = material_flags(MT);
         Frame fr;
         fr.T = s.dpdu; fr.N = s.N; fr.B = s.dpdv;
-        bsdf_prepare(bx, fr, wo);
+        bsdf_prepare(bx, fr, wo, false);
         // eligible area lights: one unused 1D sample each
         bool eligible = false, area = false;
         if (sub < S.n_lights) {
@@ -1051,17 +1044,14 @@ __device__ __noinline__ void finish_shade(const DevScene& S, const WaveArgs& a, 
         const float ur = __shfl_sync(group, u, lead + 6);
         dim = dim2;
         P.nee = true;
-        if ((bx.flags & BXDF_SPECULAR) == 0) {
-            const NeeVertex v{s, bx, fr, wo, beta, uL, uB};
-            finish_nee(S, group, sub, eligible, n_area > 0, v, P);
-        }
+        if ((bx.flags & BXDF_SPECULAR) == 0) finish_nee(S, group, sub, eligible, n_area > 0, s, bx, fr, wo, beta, uL, uB, P);
         if (!direct) {
             dim += 3;
             float3 wi = f3(0.f, 0.f, 0.f);
             float pdf = 0.f;
             int stype = 0;
             bool ok = false;
-            float3 f = bsdf_sample(bx, fr, 0.f, u2, wo, wi, pdf, BXDF_ALL, stype, ok);
+            float3 f = bsdf_sample(bx, fr, 0.f, u2, wo, wi, pdf, BXDF_ALL, stype, ok, false);
             if (ok && fabsf(pdf) != 0.f) {
                 bool specular = (stype & BXDF_SPECULAR) != 0;
                 float cosine = specular ? 1.0f : fmaxf(0.f, (stype & BXDF_TRANSMISSION) ? dot(-s.N, wi) : dot(s.N, wi));
@@ -1159,10 +1149,9 @@ __global__ void __launch_bounds__(128, 4) k_finish(const __grid_constant__ DevSc
         if (active && has && sub == G - 2) mh = mis_emitted(S, o, d, h);
         const int hl = __shfl_sync(0xffffffffu, __float_as_int(mh.w), misl);
         const float3 Le = shfl3(f3(mh), misl);
-        float3 s = has && q.occluded ? f3(0.f, 0.f, 0.f) : sh_c, m = f3(0.f, 0.f, 0.f);
-        if (sub == hl) m = mis_c * Le;
+        float3 sm = has && q.occluded ? f3(0.f, 0.f, 0.f) : sh_c;
+        if (sub == hl) sm = light_sum(sm, mis_c, Le);
         float3 dl = f3(0.f, 0.f, 0.f);
-        const float3 sm = s + m;
         for (int l = 0; l < K; l++) dl = dl + shfl3(sm, lead + l);
         if (active && nee) P.L = P.L + dl;
         P.hit.t = __shfl_sync(0xffffffffu, h.t, ext);
@@ -1248,11 +1237,10 @@ __global__ void k_accumulate(WaveArgs a, PathRefs cur, PathRefs nxt, const int2*
             for (int l = 0; l < a.K; l++) {
                 const uint32_t bit = nee_bit(l);
                 if (bit != 0u && !(fl & bit) && l != hl) continue;  // nothing to add
-                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (bit == 0u || (fl & bit)) s = sc[i * a.K + l];
-                float3 m = f3(0.f, 0.f, 0.f);
-                if (l == hl) m = f3(mc[i * a.K + l]) * f3(mh);
-                direct = direct + (f3(s) + m);
+                float3 s = f3(0.f, 0.f, 0.f);
+                if (bit == 0u || (fl & bit)) s = f3(sc[i * a.K + l]);
+                if (l == hl) s = light_sum(s, f3(mc[i * a.K + l]), f3(mh));
+                direct = direct + s;
             }
         }
         if (gv.record && ac.y) {

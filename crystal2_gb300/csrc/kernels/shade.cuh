@@ -147,7 +147,7 @@ __device__ __forceinline__ float3 area_Le(const Light& L, float3 n_actual, float
 
 // Intersect the light's own shape (Shape::PdfLight, Shape.cpp:4-12) and return the solid-angle
 // pdf, 0 on a miss.  The ray leaves pos + N * 1e-4 along wi (SurfaceInfo::SpawnRay, no side test).
-__device__ __forceinline__ float light_pdf(const DevScene& S, const Light& L, float3 pos, float3 N, float3 wi) {
+__device__ __forceinline__ float light_pdf(const DevScene& S, const Light& L, float3 pos, float3 N, float3 wi, Rounding r) {
     float3 o = pos + N * kSpawnEps;
     float3 hp, Nh;
     if (L.shape_type == SHAPE_TRI) {
@@ -168,7 +168,8 @@ __device__ __forceinline__ float light_pdf(const DevScene& S, const Light& L, fl
         Nh = s.N;
     }
     float3 dv = pos - hp;
-    return dot(dv, dv) / (fmaxf(0.f, dot(-normalize(wi), Nh)) * L.area);
+    const float3 w = wi * (1.0f / sqrtf(r == Rounding::SAMPLED ? dot_yfirst(wi, wi) : dot_xfirst(wi, wi, r)));
+    return dot(dv, dv) / (fmaxf(0.f, dot(-w, Nh)) * L.area);
 }
 
 // Shape::SampleSurface of the light's shape: position and (unflipped) normal.
@@ -206,20 +207,32 @@ __device__ __forceinline__ void light_sample_surface(const DevScene& S, const Li
 
 // Light::Sample_Li (DiffusedAreaLight.cpp:25-34, PointLight.cpp:13-19).
 __device__ __forceinline__ float3 light_sample_li(const DevScene& S, const Light& L, float3 pos, float3 N, float2 u,
-                                                  float3& endpoint, float& pdf) {
+                                                  float3& endpoint, float& pdf, Rounding r) {
     if (L.type == LIGHT_POINT) {
         endpoint = f3(L.pos[0], L.pos[1], L.pos[2]);
         pdf = 1.0f;
         float3 I = f3(L.Le[0], L.Le[1], L.Le[2]) / (4 * kPiF);
         float3 dv = endpoint - pos;
-        return I / dot(dv, dv);
+        return I / dot_xfirst(dv, dv, r);
     }
     float3 lp, ln;
     light_sample_surface(S, L, u, lp, ln);
     endpoint = lp;
     float3 dir = lp - pos;
-    pdf = light_pdf(S, L, pos, N, dir);
+    pdf = light_pdf(S, L, pos, N, dir, r);
     return area_Le(L, ln, -dir);
+}
+
+// Unit vector to a light's point.
+__device__ __forceinline__ float3 light_direction(float3 from, float3 to, Rounding r) {
+    const float3 v = to - from;
+    return v * (1.0f / sqrtf(dot_yfirst(v, v, r)));
+}
+
+// A light's two halves of direct light: the shadow ray's contribution s and the MIS ray's multiplier m times
+// the radiance Le it reached.
+__device__ __forceinline__ float3 light_sum(float3 s, float3 m, float3 Le) {
+    return f3(__fadd_rn(s.x, __fmul_rn(m.x, Le.x)), __fadd_rn(s.y, __fmul_rn(m.y, Le.y)), __fadd_rn(s.z, __fmul_rn(m.z, Le.z)));
 }
 
 // PowerHeuristic(1, f, 1, g) (Utils.h:168-172)
