@@ -1662,6 +1662,11 @@ namespace {
 // paths and 1.35 ms without).  Measured limits: 640 x 360 many-material step 1.99 ms without, 1.50 at
 // 4096 paths, 1.44 at 8192, 1.43 at 16384; the 1080p step 44.07, 44.03, 44.08, 44.97.
 constexpr int kFinishPaths = 8192, kFinishMaterials = 5;
+// Levels of a captured wave before it first looks at its queue (even: the loop's pairs keep the queues'
+// places).  Eight jobs of 256K paths a wave in a room of albedo 0.95, one graph launch / a stream each:
+// 7.2 / 5.9 ms with two, 7.5 / 5.9 with four; handing over after a number of levels guessed from the wave's
+// size took 16.1 / 14.6 (the queue was still large), every level 10.0 / 6.6.
+constexpr int kCapturedLevels = 2;
 // Traversal kernels: one ray per thread (reference tree, binary nodes), four-wide nodes with quantised
 // planes (margin of the whole scene, or of each node) or with exact ones.
 enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_NEAR4 = 3, TRACE_KINDS = 4 };
@@ -1786,6 +1791,8 @@ __global__ void k_advance_loop(int* sample0, int by, int end, cudaGraphCondition
     *sample0 += by;
     cudaGraphSetConditional(h, *sample0 < end ? 1u : 0u);
 }
+// Whether more than `limit` paths are left: the condition of a captured wave's loop over levels.
+__global__ void k_more_than(const int* count, int limit, cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, *count > limit ? 1u : 0u); }
 // statistics: *total += *count (paths entering a bounce level)
 __global__ void k_level_add(int* total, const int* count) { *total += *count; }
 }  // namespace
@@ -1877,6 +1884,39 @@ int GpuScene::prepare(const c2g_render_params& p, DeviceArena& arena, WavePlan& 
     return C2G_OK;
 }
 
+// Append to the graph that st captures: `body`, as long as *count (after the work before) is above limit.
+static int capture_while(cudaStream_t st, const int* count, int limit, const std::function<void(cudaStream_t)>& body, std::string& err) {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t graph = nullptr, inner = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    cudaGraphConditionalHandle h;
+    cudaGraphNode_t node;
+    cudaGraphNodeParams np{};
+    C2G_CUDA(cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &edges, &n));
+    C2G_CUDA(cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
+    k_more_than<<<1, 1, 0, st>>>(count, limit, h);
+    C2G_CUDA(cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &edges, &n));
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    C2G_CUDA(cudaGraphAddNode(&node, graph, deps, edges, n, &np));
+    C2G_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+    cudaStream_t inside;
+    C2G_CUDA(cudaStreamCreateWithFlags(&inside, cudaStreamNonBlocking));
+    cudaError_t e = cudaStreamBeginCaptureToGraph(inside, np.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
+    if (e == cudaSuccess) {
+        body(inside);
+        k_more_than<<<1, 1, 0, inside>>>(count, limit, h);
+        e = cudaStreamEndCapture(inside, &inner);
+    }
+    cudaStreamDestroy(inside);
+    C2G_CUDA(e);
+    return C2G_OK;
+}
+
 // Enqueue one wave (a.wave_samples samples of every pixel slot) on st: raygen, the bounce levels,
 // the film and (guided) a training step.  begin/end bracket every launch (timing hooks).
 int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideView& gv, bool count, cudaStream_t st,
@@ -1921,7 +1961,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
     int cur = 0;
     // k_finish takes over a queue of at most kFinishPaths paths.  An eager render learns the queue's size
     // from the look-ahead extension, which reports it to page-locked host memory; a captured wave
-    // cannot ask, and switches where a wave of its size has usually come down to that.
+    // loops over pairs of levels on the device until it has come down to that.
     const int materials = __builtin_popcount(present_buckets_ & ~(1 << kBucketMiss));
     const bool can_finish = !guided && !count && trace_kind(S) != TRACE_PLAIN && a.K <= 30 && plan.levels > 0 && materials <= kFinishMaterials;
     const bool poll = overlap && report_host_ && !guided && !count;
@@ -1940,18 +1980,27 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         finish(0, false);
         levels = 0;
     }
-    // captured: roulette starts after the fourth bounce; about 6.5% of a closed room's paths enter level 5,
-    // and 0.6 of them each following level
-    int captured_switch = 1 << 30;
-    if (can_finish && a.sample0_dev) {
-        double left = 0.065 * paths;
-        for (captured_switch = 5; left > kFinishPaths; captured_switch++) left *= 0.6;
+    if (can_finish && a.sample0_dev && levels > 0) {
+        auto level = [&](int q, cudaStream_t ls) {
+            const int nxt = q ^ 1;
+            extend(q, C + nxt * kLine, C + kCntShadow, C + kCntMis, nullptr, ls);
+            ShadeOut so{buf[nxt], C + nxt * kLine, w.sh_o, w.sh_d, w.sh_c, w.mis_o, w.mis_d, w.mis_c, w.sh_list, w.mis_list, C + kCntShadow, C + kCntMis, w.acc, w.mis_hit};
+            for (int bk = 0; bk < kBuckets; bk++)
+                if (present_buckets_ & (1 << bk))
+                    launch_shade(bk, g_shade, ls, S, a, buf[q], w.hit, C + kCntBucket, w.bucket_list, (int)w.P, so, gv, false);
+            launch_shadow(S, tb, w, false, nullptr, ls);
+            launch_mis(S, tb, w, false, nullptr, ls);
+            k_accumulate<<<g_acc, 256, 0, ls>>>(a, buf[q], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + q * kLine, gv, C + kCntMisFetch);
+        };
+        for (int b = 0; b < std::min(levels, kCapturedLevels); b++, cur ^= 1) level(cur, st);
+        if (levels > kCapturedLevels) {
+            int rc = capture_while(st, C + cur * kLine, kFinishPaths, [&](cudaStream_t ls) { level(cur, ls); level(cur ^ 1, ls); }, err);
+            if (rc) return rc;
+            finish(cur, false);
+        }
+        levels = 0;
     }
     for (int b = 0; b < levels; b++) {
-        if (b == captured_switch) {
-            finish(cur, false);
-            break;
-        }
         int nxt = cur ^ 1;
         if (b >= a.max_depth && a.integrator == C2G_INTEGRATOR_DIRECT && !poll) {
             // pass-through hops past the depth: stop once the queue is empty
