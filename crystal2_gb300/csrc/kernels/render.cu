@@ -164,12 +164,6 @@ int GpuScene::side_stream(std::string& err) {
         ahead_ = nullptr;
         return C2G_ERR_CUDA;
     }
-    for (more_n_ = 0; more_n_ < kMore; more_n_++)  // does with fewer
-        if (cudaStreamCreateWithFlags(&more_[more_n_], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&more_join_[more_n_], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
     // page-locked counters the device writes to; without them every level is enqueued
     if (cudaHostAlloc((void**)&report_host_, 256 * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void**)&report_dev_, report_host_, 0) != cudaSuccess) {
@@ -184,6 +178,18 @@ int GpuScene::side_stream(std::string& err) {
             return C2G_ERR_CUDA;
         }
     return C2G_OK;
+}
+
+// Streams for the buckets past the third, `n` of them at most: made when a scene first has that many (each
+// costs the first render some ten microseconds).
+int GpuScene::more_streams(int n) {
+    for (; more_n_ < std::min(n, kMore); more_n_++)  // does with fewer
+        if ((!more_[more_n_] && cudaStreamCreateWithFlags(&more_[more_n_], cudaStreamNonBlocking) != cudaSuccess) ||
+            cudaEventCreateWithFlags(&more_join_[more_n_], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
+    return std::max(0, std::min(n, more_n_));
 }
 
 // ---- small device helpers ------------------------------------------------------------------------
@@ -1973,7 +1979,7 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
         end(st);
         launches++;
     };
-    const int more = overlap ? std::max(0, std::min(more_n_, __builtin_popcount(present_buckets_) - 3)) : 0;
+    const int more = overlap ? more_streams(__builtin_popcount(present_buckets_) - 3) : 0;
     int levels = plan.levels;
     const double paths = (double)a.W * a.H * a.wave_samples;
     if (can_finish && paths <= kFinishPaths) {

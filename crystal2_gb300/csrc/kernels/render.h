@@ -184,6 +184,7 @@ private:
     int* report_dev_ = nullptr;
     static int wait_report(const volatile int* p, cudaStream_t st);
     int side_stream(std::string& err);
+    int more_streams(int n);
     float box_lo_[3] = {0, 0, 0}, box_hi_[3] = {1, 1, 1};  // scene bounds (network input range)
     c2g_stats stats_{};
     int film_w_ = 0, film_h_ = 0;
