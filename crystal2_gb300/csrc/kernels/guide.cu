@@ -873,11 +873,11 @@ __global__ void __launch_bounds__(kSumThreads) k_guide_reduce(const float* __res
     }
 }
 
-// Explicit samples of 14 floats (x, n, wo, wi, w, p_bsdf) -> the batch layout; sets the batch size and
+// Explicit samples of 14 floats (x, n, wo, wi, w, p_bsdf; null: the batch is there) -> the batch layout; sets the batch size and
 // the statistics (a weight sum of n makes the mean weight exactly 1) and clears the error word.
 __global__ void k_guide_pack(const float* __restrict__ samples, int n, float4* batch, int* batch_count, float* stats, int* err) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) {
+    if (samples && j < n) {
         const float* v = samples + (size_t)14 * j;
         batch[4 * (size_t)j] = make_float4(v[0], v[1], v[2], v[12]);
         batch[4 * (size_t)j + 1] = make_float4(v[3], v[4], v[5], 0.f);
@@ -1139,13 +1139,29 @@ int GuideTrainer::gradient(DeviceArena& arena, const float* host_samples, int n,
     // batch (64 bytes per sample), the samples as given, the error word
     const size_t raw = (size_t)n * 14 * 4, packed = (size_t)n * 64;
     unsigned char* buf = (unsigned char*)arena.borrow(packed + raw + 16, err);
-    if (!buf) return C2G_ERR_OOM;
+    float* ds = buf ? (float*)(buf + packed) : nullptr;
+    if (!buf) {  // no room for both: the batch alone, packed here
+        err.clear();
+        buf = (unsigned char*)arena.borrow(packed + 16, err);
+        if (!buf) return C2G_ERR_OOM;
+    }
     float4* db = (float4*)buf;
-    float* ds = (float*)(buf + packed);
-    int* derr = (int*)(buf + packed + raw);
-    cudaMemcpy(ds, host_samples, raw, cudaMemcpyHostToDevice);
+    int* derr = (int*)(buf + packed + (ds ? raw : 0));
+    if (ds) {
+        cudaMemcpy(ds, host_samples, raw, cudaMemcpyHostToDevice);
+    } else {
+        std::vector<float4> b((size_t)n * 4);
+        for (size_t j = 0; j < (size_t)n; j++) {
+            const float* v = host_samples + 14 * j;
+            b[4 * j] = make_float4(v[0], v[1], v[2], v[12]);
+            b[4 * j + 1] = make_float4(v[3], v[4], v[5], 0.f);
+            b[4 * j + 2] = make_float4(v[6], v[7], v[8], 0.f);
+            b[4 * j + 3] = make_float4(v[9], v[10], v[11], v[13]);
+        }
+        cudaMemcpy(db, b.data(), packed, cudaMemcpyHostToDevice);
+    }
     prepare_launch();
-    k_guide_pack<<<(n + 255) / 256, 256>>>(ds, n, db, batch_count_, loss_acc_, derr);
+    k_guide_pack<<<ds ? (n + 255) / 256 : 1, 256>>>(ds, n, db, batch_count_, loss_acc_, derr);
     k_guide_train_tc<<<g_train_grid, kTgThreads, kTgSmem>>>(view(false, false).net, db, batch_count_, n, part_, loss_acc_, 1,
                                                            step_dev_, derr);
     k_guide_reduce<<<kSumBlocks, kSumThreads>>>(part_, nparts_, grad_, loss_acc_, derr);

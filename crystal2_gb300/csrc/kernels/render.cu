@@ -1487,6 +1487,9 @@ void launch_shade(int bk, int grid, cudaStream_t st, const DevScene& S, const Wa
     }
 }
 
+// The permutation tables are the same for every scene: one copy per device, outside the contexts' memory.
+static __device__ float g_perm[kPermTotal];
+
 int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const SahTree* sah, DeviceArena& arena, std::string& err) {
     // release previous scene buffers
     for (void* p : sb_->owned) arena.free(p);
@@ -1554,8 +1557,11 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
     std::vector<uint16_t> perm;
     std::vector<int> off;
     halton_perm_tables(perm, off);
-    S.perm = upload_vec(std::vector<float>(perm.begin(), perm.end()), arena, sb_->owned, err, rc);
-    if (rc) return rc;
+    const std::vector<float> digits(perm.begin(), perm.end());
+    C2G_CUDA(cudaMemcpyToSymbol(g_perm, digits.data(), sizeof(float) * digits.size()));
+    void* digits_dev = nullptr;
+    C2G_CUDA(cudaGetSymbolAddress(&digits_dev, g_perm));
+    S.perm = (const float*)digits_dev;
     S.seed = (uint64_t)s.cfg.seed;
     S.sampler = s.cfg.sampler == "Default" ? SAMPLER_DEFAULT : s.cfg.sampler == "Stratified" ? SAMPLER_STRATIFIED : SAMPLER_HALTON;
     S.spp = std::max(1, s.cfg.spp);
