@@ -828,18 +828,6 @@ __device__ __forceinline__ void trace_queue(Lane& L, int* fetch, int n) {
     }
 }
 
-// Brute semantics (Brute.cpp:19-55): every object, no box tests.
-__device__ __forceinline__ Hit trace_closest_brute(const DevScene& S, const RayQ& r) {
-    Hit h{INFINITY, 0.f, 0.f, -1};
-    for (int i = 0; i < S.n_prims; i++) closest_prim(S, i, r, INFINITY, h);
-    return h;
-}
-__device__ __forceinline__ bool trace_any_brute(const DevScene& S, const RayQ& r, float tmin, float tmax, int ignore) {
-    for (int i = 0; i < S.n_prims; i++)
-        if (anyhit_prim(S, i, r, tmin, tmax, ignore)) return true;
-    return false;
-}
-
 // One ray per thread: the reference tree and the binary SAH tree (four-wide nodes: trace_queue).
 template <bool COUNT>
 __device__ __forceinline__ Hit trace_closest(const DevScene& S, float3 o, float3 d, TraceCounters* cnt) {
