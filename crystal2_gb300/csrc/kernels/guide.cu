@@ -11,6 +11,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <vector>
 
@@ -1003,10 +1004,8 @@ int GuideTrainer::init(DeviceArena& arena, size_t paths, int max_depth, const fl
 
 namespace {
 int g_infer_grid = 0, g_train_grid = 0, g_encode_grid = 0;
-}  // namespace
 
-void GuideTrainer::prepare_launch() {
-    if (g_infer_grid) return;
+void find_launch() {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1025,6 +1024,12 @@ void GuideTrainer::prepare_launch() {
     int per_enc = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_enc, k_guide_record, 256, 0);
     g_encode_grid = std::max(1, sms * std::max(1, per_enc));
+}
+}  // namespace
+
+void GuideTrainer::prepare_launch() {
+    static std::once_flag once;
+    std::call_once(once, find_launch);
 }
 
 int GuideTrainer::infer(cudaStream_t st, const void* Sv, const float4* ray_o, const float4* ray_d, const float4* hits,

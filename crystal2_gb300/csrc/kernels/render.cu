@@ -13,6 +13,7 @@
 #include <functional>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "../host/bvh.h"
@@ -1706,8 +1707,7 @@ struct TraceGrids {
 };
 TraceGrids g_trace[3] = {};
 int trace_block_index(int threads) { return threads <= 64 ? 0 : (threads <= 128 ? 1 : 2); }
-void ensure_grids() {
-    if (g_raygen) return;
+void find_grids() {
     g_raygen = grid_for((const void*)k_raygen, 256);
     g_shade = grid_for((const void*)k_shade<MAT_DIFFUSE, false>, 128);
     g_acc = grid_for((const void*)k_accumulate, 256);
@@ -1730,6 +1730,12 @@ void ensure_grids() {
                 });
         }
     }
+}
+
+// Contexts of several threads may render at once: the first one in finds all the sizes, the others wait.
+void ensure_grids() {
+    static std::once_flag once;
+    std::call_once(once, find_grids);
 }
 
 // The traversal kernels' launches; the variant follows from the scene.  C: the wave's counters.
@@ -2412,12 +2418,14 @@ int GpuScene::trace_rays_dev(int n, const float* o, const float* d, const float*
     const DevScene& S = sb_->S;
     const int kind = trace_kind(S);
     if (kind != TRACE_PLAIN) {
-        static int grids[TRACE_KINDS][2] = {};
-        if (!grids[kind][0])
+        static int grids[TRACE_KINDS][2];
+        static std::once_flag once[TRACE_KINDS];
+        std::call_once(once[kind], [&] {
             by_ray(kind, [&](auto tag) {
-                grids[kind][1] = grid_for((const void*)k_any_rays_fetch<C2G_RAY(tag)>, 128);
                 grids[kind][0] = grid_for((const void*)k_closest_rays_fetch<C2G_RAY(tag)>, 128);
+                grids[kind][1] = grid_for((const void*)k_any_rays_fetch<C2G_RAY(tag)>, 128);
             });
+        });
         const int g = grids[kind][any_hit ? 1 : 0];
         C2G_CUDA(cudaMemsetAsync(sb_->fetch, 0, sizeof(int), st));
         by_ray(kind, [&](auto tag) {
