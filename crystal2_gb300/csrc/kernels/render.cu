@@ -1676,10 +1676,22 @@ namespace {
 // 4096 paths, 1.44 at 8192, 1.43 at 16384; the 1080p step 44.07, 44.03, 44.08, 44.97.
 constexpr int kFinishPaths = 8192, kFinishMaterials = 5;
 // Levels of a captured wave before it first looks at its queue (even: the loop's pairs keep the queues'
-// places).  Eight jobs of 256K paths a wave in a room of albedo 0.95, one graph launch / a stream each:
-// 7.2 / 5.9 ms with two, 7.5 / 5.9 with four; handing over after a number of levels guessed from the wave's
-// size took 16.1 / 14.6 (the queue was still large), every level 10.0 / 6.6.
-constexpr int kCapturedLevels = 2;
+// places).  A graph that runs the wave a few times has two, since its launch costs about 2 us a node: twelve
+// jobs of up to 1M paths, one wave each, 9.9 ms, and 10.9 with the levels below.  Where many waves repeat, a
+// turn of the loop costs each some 10 us, so levels at which even an open scene's queue is large come first:
+// of the 1080p many-material frame's paths 3.5% enter level 4, 1% level 5 and 0.7 of them each second level
+// on (64 mixed jobs of 2^23 / 2^21 paths a wave 4.06 / 5.45 s, with two levels 4.14 / 5.56).
+// Eight jobs of 256K paths a wave in a room of albedo 0.95, one graph launch / a stream each: 7.3 / 5.9 ms;
+// handing over at a level guessed from the wave's size took 16.1 / 14.6 (the queue was still large), every
+// level 10.0 / 6.6.
+int captured_levels(double paths, int waves) {
+    int n = 2;
+    if (waves >= 4 && 0.035 * paths > kFinishPaths) {
+        n = 4;
+        for (double left = 0.0104 * paths; left > kFinishPaths; left *= 0.7) n += 2;
+    }
+    return n;
+}
 // Traversal kernels: one ray per thread (reference tree, binary nodes), four-wide nodes with quantised
 // planes (margin of the whole scene, or of each node) or with exact ones.
 enum : int { TRACE_PLAIN = 0, TRACE_QUANT4 = 1, TRACE_EXACT4 = 2, TRACE_NEAR4 = 3, TRACE_KINDS = 4 };
@@ -2010,8 +2022,9 @@ int GpuScene::enqueue_wave(const WavePlan& plan, const WaveArgs& a, const GuideV
             launch_mis(S, tb, w, false, nullptr, ls);
             k_accumulate<<<g_acc, 256, 0, ls>>>(a, buf[q], buf[nxt], w.acc, w.sh_c, w.mis_c, w.mis_hit, w.out_L, C + q * kLine, gv, C + kCntMisFetch);
         };
-        for (int b = 0; b < std::min(levels, kCapturedLevels); b++, cur ^= 1) level(cur, st);
-        if (levels > kCapturedLevels) {
+        const int first = captured_levels(paths, plan.waves);
+        for (int b = 0; b < std::min(levels, first); b++, cur ^= 1) level(cur, st);
+        if (levels > first) {
             int rc = capture_while(st, C + cur * kLine, kFinishPaths, [&](cudaStream_t ls) { level(cur, ls); level(cur ^ 1, ls); }, err);
             if (rc) return rc;
             finish(cur, false);
@@ -2194,6 +2207,7 @@ int GpuScene::capture_plan(const c2g_render_params& p, bool guide_sample, cudaSt
     plan.a.wave_samples = plan.spw;
     plan.a.sample0 = 0;
     plan.a.sample0_dev = wave_counter_;
+    plan.waves = p.sample_count / plan.spw;
     gv = plan.guided ? guide_.view(true, guide_sample) : GuideView{};
     // batched jobs already overlap each other; the side-stream branches inside each graph measured
     // slower there (64-job batch: 770 vs 872 Mpaths/s), so graphs keep one stream

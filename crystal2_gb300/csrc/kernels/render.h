@@ -73,6 +73,7 @@ struct WavePlan {
     WaveArgs a;
     int spw = 1;
     int levels = 0;
+    int waves = 1;       // times a captured wave is run
     bool guided = false;
 };
 

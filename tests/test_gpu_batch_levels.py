@@ -53,6 +53,23 @@ def test_depths(tmp_path, depth, streams):
     b.close()
 
 
+# four waves of 2^18 and 2^20 paths: four and six levels before the loop
+@pytest.mark.parametrize("side,depth", [(512, 3), (512, 4), (512, 5), (512, 16), (1024, 5), (1024, 6), (1024, 7), (1024, 16)])
+@pytest.mark.parametrize("streams", [0, 1])
+def test_repeated_waves(tmp_path, side, depth, streams):
+    [(ctx, p)] = _jobs(tmp_path, 1, 0.9, side, 4, depth)
+    ctx.film_clear()
+    ctx.render(p)
+    want = ctx.film()[0]
+    ctx.film_clear()
+    b = Batch(0)
+    b.add(ctx, p)
+    b.tune(side * side, streams)
+    b.run()
+    assert np.array_equal(ctx.film()[0], want)
+    b.close()
+
+
 def _best(f, n=7):
     f()
     times = []
