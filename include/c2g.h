@@ -93,9 +93,11 @@ typedef struct {
 #define C2G_K_KINDS 10  /* size of the per-kind arrays */
 
 /* Counting / timing switches of c2g_set_counting. */
-#define C2G_COUNT_TRAVERSAL 1  /* rays, nodes visited and prims tested per traversal kernel */
+#define C2G_COUNT_TRAVERSAL 1  /* rays, nodes visited and prims tested per traversal kernel; every level in the
+                                  level kernels (kind C2G_K_TAIL does not count) */
 #define C2G_COUNT_TIMING 2     /* CUDA events around every launch; per-kind device time */
-#define C2G_COUNT_SERIAL 4     /* one stream: no side or look-ahead stream, so per-kind times are exclusive */
+#define C2G_COUNT_SERIAL 4     /* one stream: no side or look-ahead stream, so per-kind times are exclusive; a wave
+                                  that starts larger than C2G_K_TAIL takes keeps every level in the level kernels */
 
 #define C2G_LEVELS 64  /* size of the per-bounce-level arrays (deeper levels add to the last entry) */
 
