@@ -422,19 +422,14 @@ void collapse_bvh4(SahTree& t) {
     if (t.nodes4.size() > kExactNodes) t.nodes4x.clear();
 }
 
-bool has_narrow_leaves(const SahTree& t, float width) {
-    size_t leaves = 0, narrow = 0;
-    auto add = [&](const float* lo, const float* hi) {
-        float side = 0.f;
-        for (int k = 0; k < 3; k++) side = std::max(side, hi[k] - lo[k]);
-        leaves++;
-        narrow += side < width;
-    };
-    for (const WideNode& n : t.nodes) {
-        if (n.n0 > 0) add(n.lo0, n.hi0);
-        if (n.n1 > 0) add(n.lo1, n.hi1);
+size_t narrow_leaves(const SahTree& t, float width) {
+    size_t n = 0;
+    auto narrow = [&](const float* lo, const float* hi) { return std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]}) < width; };
+    for (const WideNode& w : t.nodes) {
+        n += w.n0 > 0 && narrow(w.lo0, w.hi0);
+        n += w.n1 > 0 && narrow(w.lo1, w.hi1);
     }
-    return narrow * 16 > leaves;
+    return n;
 }
 
 void make_prims(const HostScene& s, const std::vector<int>& order, std::vector<Prim>& prims) {

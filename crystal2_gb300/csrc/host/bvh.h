@@ -43,8 +43,8 @@ void build_sah_tree(const HostScene& s, SahTree& out, int max_leaf = 4);
 // Collapse the binary SAH tree into four-wide nodes: every node absorbs the children of its
 // largest-area inner children until it holds four (Node4; boxes and leaves unchanged).
 void collapse_bvh4(SahTree& t);
-// Whether more than one leaf in 16 has a box whose largest side is below `width`.
-bool has_narrow_leaves(const SahTree& t, float width);
+// Leaves whose box is below `width` on every side.
+size_t narrow_leaves(const SahTree& t, float width);
 
 // Prim records for an object order (traversal order).
 void make_prims(const HostScene& s, const std::vector<int>& order, std::vector<Prim>& prims);

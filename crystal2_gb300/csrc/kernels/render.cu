@@ -1488,6 +1488,10 @@ void launch_shade(int bk, int grid, cudaStream_t st, const DevScene& S, const Wa
     }
 }
 
+// Leaves small against the scene from which on its rays take each node's own margin (see slab_axis): a ray
+// that comes near a detail of n such leaves may test them all otherwise.
+constexpr size_t kNarrowLeaves = 64;
+
 // The permutation tables are the same for every scene: one copy per device, outside the contexts' memory.
 static __device__ float g_perm[kPermTotal];
 
@@ -1610,7 +1614,7 @@ int GpuScene::upload(const HostScene& s, int tree, const RefTree* ref, const Sah
     S.reach = std::max({S.extent[0], S.extent[1], S.extent[2]});
     // scale <= 1.35 reach and an offset of at most 2.7 reach keep their products below 2^122
     S.inv_max = 0x1p120f / std::max(S.reach, 1.f);
-    S.near_margin = sah && has_narrow_leaves(*sah, std::ldexp(S.reach, -14));
+    S.near_margin = sah && narrow_leaves(*sah, std::ldexp(S.reach, -14)) > kNarrowLeaves;
     guide_steps_ = 0;
     wave_counter_ = nullptr;  // freed with the previous scene's buffers
     guide_.release(arena);  // a new scene trains a new network

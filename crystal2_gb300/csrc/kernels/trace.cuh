@@ -541,7 +541,7 @@ __device__ __forceinline__ bool trace_any_sah(const DevScene& S, const RayQ& r, 
 //   is the ray's for all nodes, and saves two FMAs per axis.
 // One object far from all others makes E large against most boxes: 1e5 units from a soup of triangles of
 // 0.05 in the unit cube a ray tested 280 of them instead of 11, and every one at 1e6.  So scenes with more
-// than a few leaves narrower than 2^-14 of their reach, 64 times m, take Ray4n: 11 there, as without the far
+// than 64 leaves narrower than 2^-14 of their reach, 64 times m, take Ray4n: 11 there, as without the far
 // object.  For every scene it would cost the 1080p many-material frame 0.4%, and 2M closest-hit rays of a
 // 65k-triangle soup 5%.
 //

@@ -16,11 +16,13 @@ pytestmark = pytest.mark.gpu
 TRIS = 4096
 
 
-def _soup(d, far, spp=1, size=64):
+def _soup(d, far, spp=1, size=64, others=None):
     tris = scenes.tri_soup_arrays(TRIS, 3).astype(np.float64)
     tris = tris + (tris - tris.mean(axis=1, keepdims=True)) * 4  # edges of some 0.03
     if far:
         tris = np.concatenate([tris, (np.float64([[0, 0, 0], [1, 0, 0], [0, 1, 0]]) * 0.1 + 1.0)[None] * far])
+    if others is not None:
+        tris = np.concatenate([tris, others])
     tris = tris.astype(np.float32)
     n = np.cross((tris[:, 1] - tris[:, 0]).astype(np.float64), (tris[:, 2] - tris[:, 0]).astype(np.float64))
     n /= np.linalg.norm(n, axis=1, keepdims=True)
@@ -112,3 +114,23 @@ def test_a_far_triangle_costs_no_culling(tmp_path, far):
     (nodes0, prims0), (nodes1, prims1) = per_ray
     assert nodes1 <= 1.25 * nodes0 + 4
     assert prims1 <= 1.25 * prims0 + 1
+
+
+# The soup as a detail among many more, far larger triangles: no more of them are tested than through the binary
+# nodes' exact boxes, up to the 8-bit planes' looseness (a tenth without far objects; taken as a quarter and one).
+def test_a_detail_among_large_objects(tmp_path):
+    rng = np.random.default_rng(4)
+    c = rng.uniform(-1e5, 1e5, (40 * TRIS, 1, 3))
+    c = c[np.linalg.norm(c[:, 0], axis=1) > 2e4]
+    assert len(c) > 32 * TRIS
+    (cp, sp), _ = _soup(str(tmp_path), 0, others=c + rng.uniform(-300, 300, (len(c), 3, 3)))
+    prims = []
+    with Context(0) as ctx:
+        ctx.load(cp, sp, tree=N.TREE_SAH)
+        ctx.set_counting(N.COUNT_TRAVERSAL)
+        for width in (2, 4):
+            ctx.set_traversal(width)
+            ctx.render(ctx.render_params())
+            s = ctx.stats()
+            prims.append(s.prims[N.K_EXTEND] / s.rays[N.K_EXTEND])
+    assert prims[1] <= 1.25 * prims[0] + 1
