@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(256, C2G_EXTEND_MIN_BLOCKS) k_mis_fetch(DevSce
 // groups are traced together.  A path's radiance has the bits that the level kernels give it (the functions
 // they share are compiled for the material, and see Rounding), so a film does not depend on which kernels
 // traced a wave's last levels.
-// 64 x 64 Cornell box at 1 spp: 0.36 ms in 58 launches -> 0.17 in 3; the 640 x 360 step 1.99 -> 1.42 ms.
+// 64 x 64 Cornell box at 1 spp: 0.36 ms in 58 launches -> 0.16 in 3; the 640 x 360 step 1.99 -> 1.44 ms.
 // Its bound is latency, then instruction fetch: four groups of one warp at four materials run one after
 // another (a version without the per-material functions was 0.15 ms, but its other contraction of
 // multiplies and adds turned paths behind mirrors and lenses).
